@@ -643,7 +643,10 @@ int vk_create(const vk_config* cfg, vk_ctx** out) {
   if ((e = cudaMalloc(&c->etd, (size_t)c->n_etd * vk::ETD_STRIDE * sizeof(double))) != cudaSuccess)
     return bail(e, "cudaMalloc(etd)");
   if ((e = cudaMalloc(&c->dsc, sizeof(vk::DevScalars))) != cudaSuccess) return bail(e, "cudaMalloc(scalars)");
-  if ((e = cudaMemset(c->dsc, 0, sizeof(vk::DevScalars))) != cudaSuccess) return bail(e, "cudaMemset(scalars)");
+  // on the context's stream: it does not wait for the legacy stream, so a memset
+  // there could run after the first state's scalars were uploaded
+  if ((e = cudaMemsetAsync(c->dsc, 0, sizeof(vk::DevScalars), c->stream)) != cudaSuccess)
+    return bail(e, "cudaMemsetAsync(scalars)");
   // spectrum shells: ceil(sqrt(3 (N/2)^2)) + 1 (spectrum.rs:22-26)
   const double kmx = (double)(n / 2);
   c->n_shells = (int)std::ceil(std::sqrt(kmx * kmx + kmx * kmx + kmx * kmx)) + 1;
@@ -655,6 +658,8 @@ int vk_create(const vk_config* cfg, vk_ctx** out) {
   c->dpart_rows = vk::p5_ctas(n, c->fp32);   // rows of k_p5 at this grid
   if ((e = cudaMalloc(&c->dpart, (size_t)c->dpart_rows * (4 + c->n_shells) * sizeof(double))) != cudaSuccess)
     return bail(e, "cudaMalloc(fused diagnostics)");
+  // the twiddle tables' copies (pageable memory, legacy stream)
+  if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return bail(e, "cudaStreamSynchronize");
   *out = c;
   return VK_OK;
 }
@@ -1345,6 +1350,8 @@ int vk_fft_create(int32_t nx, int32_t ny, int32_t nz, int32_t precision, int32_t
   if ((e = upload_twiddles(nx, p->fp32, &p->twx)) != cudaSuccess) return bail("twiddles");
   if ((e = upload_twiddles(ny, p->fp32, &p->twy)) != cudaSuccess) return bail("twiddles");
   if ((e = upload_twiddles(nz, p->fp32, &p->twz)) != cudaSuccess) return bail("twiddles");
+  // the tables' copies (pageable memory, legacy stream)
+  if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return bail("cudaStreamSynchronize");
   *out = p;
   return VK_OK;
 }
