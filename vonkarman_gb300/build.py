@@ -19,7 +19,8 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libvonkarman_gpu.so")
 
-SOURCES = ["vk_engine_f64.cu", "vk_engine_f32.cu", "vk_misc.cu", "vk_api.cu", "vk_noalloc.cu"]
+SOURCES = ["vk_engine_f64_fft.cu", "vk_engine_f64_step.cu", "vk_engine_f64_adj.cu", "vk_engine_f64_diag.cu",
+           "vk_engine_f32.cu", "vk_misc.cu", "vk_api.cu", "vk_noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 

@@ -78,6 +78,7 @@ template <typename R, int GN = 0, int GM = 0> struct OpAdjXInv {
   VK_GRID_DIMS(GN, GM)
   VK_PAD_ZEROS(GN, GM)
   __host__ __device__ __forceinline__ int kind(int f) const { return f < 3 ? 0 : f < 5 ? 1 : 2; }
+  template <int K> __host__ __device__ static constexpr int exp2() { return K == 2 || sizeof(R) == 4 ? 0 : -3 * ilog2(GN); }   // s_in
   // L2 prefetch of row t of the input tile of field f (as OpXInv's)
   __device__ __forceinline__ void prefetch_row(int f, int lam0, int, int t) const {
     const C2<R>* src = f < 5 ? in : cb;
@@ -94,7 +95,7 @@ template <typename R, int GN = 0, int GM = 0> struct OpAdjXInv {
     if constexpr (K == 2) {
       return v;
     } else {
-      v = cscale<R>(v, s_in);
+      if constexpr (sizeof(R) == 4) v = cscale<R>(v, s_in);
       if constexpr (K == 1) {
         const int ix = unpad_pos(p, n_(), m_());
         const R kx = ks * (R)signed_k(ix < 0 ? 0 : ix, n_());
@@ -156,7 +157,7 @@ template <typename R> struct A3Args {
 
 template <typename R, int M, int CP>
 __host__ __device__ constexpr int adj_z_threads() {
-  return cmin(rthreads<R, M, 9 * CP, true>(), 384);
+  return cmin(rthreads<R, M, 9 * CP, true>(), sizeof(R) == 8 ? 512 : 384);
 }
 // Shared memory of k_adj_z: 9 CP inverse lines (exchange, then the physical
 // values in place) and 6 CP forward lines.
@@ -189,7 +190,7 @@ struct AdjZRowUnpack {
 // columns of pair pr.  Forward lines l = t * 2CP + c: (ab_x + i ab_y),
 // (ab_z + i ob_x), (ob_y + i ob_z) of column c.
 template <typename R, int M, int CP, int NT>
-__global__ void __launch_bounds__(NT, M >= 768 ? 1 : cmax(1, (sizeof(R) == 8 ? 768 : 512) / NT))
+__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? fx_min_blocks<M, NT>() : M >= 768 ? 1 : cmax(1, 512 / NT))
 k_adj_z(A3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int N = 2 * M / 3;
   constexpr int H = N / 2 + 1;
@@ -403,6 +404,38 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
     const R ky = a.ks * (R)signed_k(iy, N);
     const R kz = a.ks * (R)z;
     const R wgt = a.s_out * (z == 0 ? R(1) : R(2));
+    if constexpr (sizeof(R) == 8) {
+      // one loop body for the six fields (the FP64 transform's code is large);
+      // wave numbers from shared memory (their conversion is an FP64 operation)
+      __shared__ double kx_s[N];
+      for (int i = threadIdx.x; i < N; i += NT) kx_s[i] = a.ks * (double)signed_k(i, N);   // ordered by the first FFT's barriers
+#pragma unroll 1
+      for (int c = 0; c < 6; ++c) {
+        if (c > 0) __syncthreads();   // xb is reused
+        const double2* src = a.in + (size_t)c * a.fsin + (iy * H + z);
+        // i k x o_bar (spectral_ops.rs:92-104), one o_bar component at a time:
+        // y_p += i kp o, y_q -= i kq o with (p, q) = (y, z), (z, x), (x, y)
+        const int p = c < 3 ? c : (c - 2) % 3, q = c < 3 ? c : (c - 1) % 3;
+        fft_lines<R, L, false, NT, NLINES, MapInterleaved<R, L, NLINES>, false, true>(
+            xb, tw_s, [&](int, int pos) { return src[pos * (N * H)]; }, PrepNone{},
+            [&](int, int pos, double2 v) {
+              const int ix = unpad_pos(pos, N, L);
+              if (ix < 0) return;
+              v = make_double2(v.x * wgt, v.y * wgt);
+              double2* yp = acc + (p * N + ix) * NLINES + l;
+              if (c < 3) {
+                *yp = v;
+              } else {
+                double2* yq = acc + (q * N + ix) * NLINES + l;
+                const double kx = kx_s[ix];
+                const double kp = c == 3 ? kz : c == 4 ? kx : ky, kq = c == 3 ? ky : c == 4 ? kz : kx;
+                const double2 a1 = *yp, a2 = *yq;
+                *yp = make_double2(fma(-kp, v.y, a1.x), fma(kp, v.x, a1.y));
+                *yq = make_double2(fma(kq, v.y, a2.x), fma(-kq, v.x, a2.y));
+              }
+            });
+      }
+    } else {
     sfor<6>([&](auto cc) {
       constexpr int C = decltype(cc)::value;
       if (C > 0) __syncthreads();   // xb is reused
@@ -432,6 +465,7 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
             }
           });
     });
+    }
   }
   __syncthreads();
 #pragma unroll 1

@@ -1,7 +1,7 @@
 // C ABI of the GB300 periodic pseudospectral solver (declared in
 // include/vonkarman_gpu.h).  Host orchestration only: buffers, the per-step
 // launch schedule and readbacks.  All arithmetic runs in the kernels of
-// vk_engine_f64.cu / vk_engine_f32.cu / vk_misc.cu.
+// vk_engine_f64_*.cu / vk_engine_f32.cu / vk_misc.cu.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "vk_host.h"
+#include "vk_fix.cuh"
 #include "vk_schedule.h"
 #include "vonkarman_gpu.h"
 
@@ -39,29 +40,26 @@ bool fft_len_ok(int n) {
   return n % 3 == 0 && is_pow2(n / 3) && n / 3 >= 4;
 }
 
-// W_L^m = exp(-2 pi i m / L), computed in long double and rounded once.
-std::vector<double> twiddle_table(int L) {
-  std::vector<double> t(2 * (size_t)L);
+// W_L^m = exp(-2 pi i m / L), computed in long double: rounded once to floats,
+// or to the fixed-point words of the FP64 form (the units of its second stage).
+cudaError_t upload_twiddles(int L, bool fp32, void** dst) {
   const long double two_pi = 6.283185307179586476925286766559005768L;
+  const int bits = 64 - vk::fx_growth(vk::fx_radix(L, 1));
+  std::vector<float2> f((size_t)(fp32 ? L : 0));
+  std::vector<vk::fxtw> x((size_t)(fp32 ? 0 : L));
   for (int m = 0; m < L; ++m) {
     const long double a = two_pi * (long double)m / (long double)L;
-    t[2 * m] = (double)cosl(a);
-    t[2 * m + 1] = (double)(-sinl(a));
+    if (fp32) {
+      f[m] = make_float2((float)(double)cosl(a), (float)(double)(-sinl(a)));
+    } else {
+      vk::fx_words(cosl(a), bits, x[m].ch, x[m].cl);
+      vk::fx_words(-sinl(a), bits, x[m].dh, x[m].dl);
+    }
   }
-  return t;
-}
-
-cudaError_t upload_twiddles(int L, bool fp32, void** dst) {
-  std::vector<double> t = twiddle_table(L);
-  size_t bytes = (size_t)L * (fp32 ? sizeof(float2) : sizeof(double2));
+  const size_t bytes = (size_t)L * (fp32 ? sizeof(float2) : sizeof(vk::fxtw));
   cudaError_t e = cudaMalloc(dst, bytes);
   if (e != cudaSuccess) return e;
-  if (fp32) {
-    std::vector<float> f(t.size());
-    for (size_t i = 0; i < t.size(); ++i) f[i] = (float)t[i];
-    return cudaMemcpy(*dst, f.data(), bytes, cudaMemcpyHostToDevice);
-  }
-  return cudaMemcpy(*dst, t.data(), bytes, cudaMemcpyHostToDevice);
+  return cudaMemcpy(*dst, fp32 ? (const void*)f.data() : (const void*)x.data(), bytes, cudaMemcpyHostToDevice);
 }
 
 // theta_j = 2 pi (j + 1/2) / 32 evaluated as in etd.rs:22, then the constant
@@ -642,6 +640,8 @@ int vk_create(const vk_config* cfg, vk_ctx** out) {
   c->n_etd = 3 * half * half + 1;
   if ((e = cudaMalloc(&c->etd, (size_t)c->n_etd * vk::ETD_STRIDE * sizeof(double))) != cudaSuccess)
     return bail(e, "cudaMalloc(etd)");
+  if ((e = vk::launch_etd_ik2(c->etd, c->n_etd, c->ks * c->ks, c->stream)) != cudaSuccess)
+    return bail(e, "etd_ik2");
   if ((e = cudaMalloc(&c->dsc, sizeof(vk::DevScalars))) != cudaSuccess) return bail(e, "cudaMalloc(scalars)");
   // on the context's stream: it does not wait for the legacy stream, so a memset
   // there could run after the first state's scalars were uploaded

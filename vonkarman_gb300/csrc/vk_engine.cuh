@@ -1,5 +1,5 @@
 // Host-side launchers: map runtime grid sizes onto the compile-time kernel
-// instances.  Instantiated once per precision (vk_engine_f64.cu,
+// instances.  Instantiated once per precision (vk_engine_f64_*.cu,
 // vk_engine_f32.cu) so the two compile in parallel.
 #pragma once
 
@@ -193,7 +193,7 @@ inline cudaError_t nle_n(const NleParams<R>& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
   } else {
     TimerScope ts(p.timer, PASS_P3, s);
-    constexpr int CP = zpairs<M, 384>();
+    constexpr int CP = zcross_pairs<R, M>();
     constexpr int NT = p3_threads<R, M, CP>();
     const size_t smem = (size_t)p3_smem_lines<R, M, CP>() * zpad_len<R>(M) * sizeof(C2<R>);
     constexpr auto kern = k_p3<R, M, CP, NT>;
@@ -275,7 +275,7 @@ inline cudaError_t nla_n(const NlaParams<R>& p, cudaStream_t s) {
   }
   {
     TimerScope ts(p.timer, PASS_A3, s);
-    constexpr int CP = zpairs<M, 384>();
+    constexpr int CP = zcross_pairs<R, M>();
     constexpr int NT = adj_z_threads<R, M, CP>();
     const size_t smem = (size_t)adj_z_smem_elems<R, M, CP>() * sizeof(C2<R>);
     constexpr auto kern = k_adj_z<R, M, CP, NT>;
@@ -334,7 +334,7 @@ inline cudaError_t ngrid_n(const NgridParams<R>& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
   }
   TimerScope ts(p.timer, PASS_NZ, s);
-  constexpr int CP = zpairs<N, 512>();
+  constexpr int CP = nz_pairs<R, N>();
   NZArgs<R> a{N * N, p.bufB, fs, p.out, p.which};
   const int nb = (N * N + 2 * CP - 1) / (2 * CP);
   if (both) {
@@ -358,8 +358,8 @@ inline cudaError_t ngrid_n(const NgridParams<R>& p, cudaStream_t s) {
 // Standalone backend: one pass per axis with its own length.
 template <typename R, int L>
 inline cudaError_t fz_pass(const FftParams<R>& p, bool inverse, R scale, cudaStream_t s) {
-  constexpr int CP = zpairs<L, 4096>();
-  constexpr int NT = zthreads<R, CP, L>();
+  constexpr int CP = fz_pairs<R, L>();
+  constexpr int NT = rthreads<R, L, CP, true>();
   const size_t smem = (size_t)CP * zpad_len<R>(L) * sizeof(C2<R>);
   const int ncols = p.nx * p.ny;
   const int nb = (ncols + 2 * CP - 1) / (2 * CP);

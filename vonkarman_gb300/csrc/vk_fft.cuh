@@ -1,12 +1,7 @@
-// Shared-memory batched FFT engine for sm_103a.
-//
-// Lines of length L = 2^a or 3*2^a (8 <= L <= 1536) are transformed in shared
-// memory by a mixed-radix Stockham auto-sort (radix 8/4/3/2, natural-order
-// output, no bit reversal).  All threads of a CTA cooperate on NLINES lines:
-// in each stage every thread loads the inputs of its butterflies into
-// registers, the CTA synchronises, then every thread twiddles, runs the radix
-// kernel and stores.  Twiddles W_L^m = exp(-2 pi i m / L) come from a table
-// computed on the host in extended precision (no device trigonometry).
+// Radix kernels of the line transforms (FP32; the FP64 form runs in fixed point,
+// vk_fix.cuh): in-register DFTs with the stage twiddles fused into the first
+// butterfly layer, complex helpers and the padded layout of contiguous lines.
+// The Stockham stages that use them are in vk_lines.cuh.
 //
 // Forward = exp(-i...), unnormalised; inverse = exp(+i...), unnormalised.  The
 // callers fold the 1/N normalisations of the reference's c2r_3d
@@ -49,78 +44,6 @@ template <typename R>
 __device__ __forceinline__ C2<R> czero() { return cmk<R>(R(0), R(0)); }
 // two loaded complex values (raw inputs that a later step combines)
 template <typename R> struct C2x2 { C2<R> a, b; };
-
-// ---------------------------------------------------------------------------
-// Radix plans.  The first stage carries no twiddles, so the largest radix goes
-// first.
-// ---------------------------------------------------------------------------
-__host__ __device__ constexpr int plan_stages(int L) {
-  return L == 8 ? 1 : L == 16 ? 2 : L == 32 ? 2 : L == 64 ? 2 : L == 128 ? 3 : L == 256 ? 3
-       : L == 512 ? 3 : L == 1024 ? 4 : L == 12 ? 2 : L == 24 ? 2 : L == 48 ? 3 : L == 96 ? 3
-       : L == 192 ? 3 : L == 384 ? 4 : L == 768 ? 4 : L == 1536 ? 4 : -1;
-}
-
-__host__ __device__ constexpr int plan_radix(int L, int s) {
-  return L == 8 ? 8
-       : L == 16 ? 4
-       : L == 32 ? (s == 0 ? 8 : 4)
-       : L == 64 ? 8
-       : L == 128 ? (s == 0 ? 8 : 4)
-       : L == 256 ? (s < 2 ? 8 : 4)
-       : L == 512 ? 8
-       : L == 1024 ? (s < 2 ? 8 : 4)
-       : L == 12 ? (s == 0 ? 4 : 3)
-       : L == 24 ? (s == 0 ? 8 : 3)
-       : L == 48 ? (s < 2 ? 4 : 3)
-       : L == 96 ? (s == 0 ? 8 : s == 1 ? 4 : 3)
-       : L == 192 ? (s < 2 ? 8 : 3)
-       : L == 384 ? (s == 0 ? 8 : s < 3 ? 4 : 3)
-       : L == 768 ? (s < 2 ? 8 : s == 2 ? 4 : 3)
-       : L == 1536 ? (s < 3 ? 8 : 3)
-       : 1;
-}
-
-// FP32 plans use in-register radix-16 stages: fewer shared-memory passes for
-// the bandwidth-bound FP32 form.  FP64 keeps radix <= 8 (registers; the FP64
-// form is bound by the FP64 pipe, where radix 16 saves no instructions).
-__host__ __device__ constexpr int plan_stages_f(int L) {
-  return L == 8 ? 1 : L == 16 ? 1 : L == 32 ? 2 : L == 64 ? 2 : L == 128 ? 2 : L == 256 ? 2
-       : L == 512 ? 3 : L == 1024 ? 3 : L == 12 ? 2 : L == 24 ? 2 : L == 48 ? 2 : L == 96 ? 3
-       : L == 192 ? 3 : L == 384 ? 3 : L == 768 ? 3 : L == 1536 ? 4 : -1;
-}
-
-__host__ __device__ constexpr int plan_radix_f(int L, int s) {
-  return L == 8 ? 8
-       : L == 16 ? 16
-       : L == 32 ? (s == 0 ? 16 : 2)
-       : L == 64 ? (s == 0 ? 16 : 4)
-       : L == 128 ? (s == 0 ? 16 : 8)
-       : L == 256 ? 16
-       : L == 512 ? (s < 2 ? 8 : 8)
-       : L == 1024 ? (s < 2 ? 16 : 4)
-       : L == 12 ? (s == 0 ? 4 : 3)
-       : L == 24 ? (s == 0 ? 8 : 3)
-       : L == 48 ? (s == 0 ? 16 : 3)
-       : L == 96 ? (s == 0 ? 16 : s == 1 ? 2 : 3)
-       : L == 192 ? (s == 0 ? 16 : s == 1 ? 4 : 3)
-       : L == 384 ? (s == 0 ? 16 : s == 1 ? 8 : 3)
-       : L == 768 ? (s < 2 ? 16 : 3)
-       : L == 1536 ? (s < 2 ? 16 : s == 2 ? 2 : 3)
-       : 1;
-}
-
-template <typename R> __host__ __device__ constexpr int stages_of(int L) {
-  return sizeof(R) == 4 ? plan_stages_f(L) : plan_stages(L);
-}
-template <typename R> __host__ __device__ constexpr int radix_of(int L, int s) {
-  return sizeof(R) == 4 ? plan_radix_f(L, s) : plan_radix(L, s);
-}
-// widest butterfly of a plan (threads per line = L / widest)
-template <typename R> __host__ __device__ constexpr int max_radix(int L) {
-  return sizeof(R) == 4 ? ((L % 16 == 0 && L >= 16 && L != 512) ? 16 : 8) : 8;
-}
-
-__host__ __device__ constexpr bool fft_len_supported(int L) { return plan_stages(L) > 0; }
 
 // ---------------------------------------------------------------------------
 // Radix kernels (in registers), with the stage twiddles fused into the first
@@ -438,82 +361,10 @@ __device__ __forceinline__ void dft(C2<R>* v, const C2<R>* w) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// Stockham stages.  Element p of line l lives at buf[l*ld_line + p*ld_elem],
-// or, for contiguous lines (ZPAD), at buf[l*ld_line + zi(p)] with one padding
-// element after every 8: the first stage writes at stride RAD, which would
-// otherwise put most lanes of a warp on the same shared-memory banks.
-// LINE_FAST: consecutive threads take consecutive lines (use when lines are
-// interleaved, ld_line == 1); otherwise consecutive butterflies of a line.
-// ---------------------------------------------------------------------------
 // one padding element per 128-byte row of the line: 8 complex doubles or 16
 // complex floats
 template <typename R> __host__ __device__ constexpr int zrow() { return 128 / (2 * (int)sizeof(R)); }
 template <typename R> __host__ __device__ constexpr int zi(int p) { return p + p / zrow<R>(); }
 template <typename R> __host__ __device__ constexpr int zpad_len(int L) { return L + L / zrow<R>(); }
-
-template <typename R, int L, bool INV, int NT, int NLINES, bool LINE_FAST, int S, int NS, bool ZPAD = false>
-struct StockhamStage {
-  __device__ __forceinline__ static void run(C2<R>* buf, int ld_line, int ld_elem,
-                                             const C2<R>* __restrict__ tw) {
-    constexpr int RAD = radix_of<R>(L, S);
-    constexpr int NB = L / RAD;          // butterflies per line
-    constexpr int TOTAL = NB * NLINES;   // butterflies per stage
-    constexpr int Q = (TOTAL + NT - 1) / NT;
-    constexpr int TWS = L / (NS * RAD);  // twiddle table stride
-    const int tid = threadIdx.x;
-    C2<R> v[Q][RAD];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int g = tid + q * NT;
-      if (TOTAL % NT == 0 || g < TOTAL) {
-        const int l = LINE_FAST ? (g % NLINES) : (g / NB);
-        const int j = LINE_FAST ? (g / NLINES) : (g % NB);
-        const C2<R>* src = buf + l * ld_line;
-#pragma unroll
-        for (int r = 0; r < RAD; ++r) v[q][r] = src[ZPAD ? zi<R>(j + r * NB) : (j + r * NB) * ld_elem];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int g = tid + q * NT;
-      if (TOTAL % NT == 0 || g < TOTAL) {
-        const int l = LINE_FAST ? (g % NLINES) : (g / NB);
-        const int j = LINE_FAST ? (g / NLINES) : (g % NB);
-        const int k = j % NS;
-        C2<R> w[RAD];
-        if (S > 0) {
-#pragma unroll
-          for (int r = 1; r < RAD; ++r) w[r] = tw[r * k * TWS];
-        }
-        dft<R, INV, RAD, (S > 0)>(v[q], w);
-        C2<R>* dst = buf + l * ld_line;
-        const int base = (j - k) * RAD + k;
-#pragma unroll
-        for (int r = 0; r < RAD; ++r) dst[ZPAD ? zi<R>(base + r * NS) : (base + r * NS) * ld_elem] = v[q][r];
-      }
-    }
-    __syncthreads();
-    if constexpr (S + 1 < stages_of<R>(L)) {
-      StockhamStage<R, L, INV, NT, NLINES, LINE_FAST, S + 1, NS * RAD, ZPAD>::run(buf, ld_line, ld_elem, tw);
-    }
-  }
-};
-
-// Transform NLINES lines held in shared memory.  Must be called by all NT
-// threads of the CTA; begins and ends with the data synchronised.
-template <typename R, int L, bool INV, int NT, int NLINES, bool LINE_FAST, bool ZPAD = false>
-__device__ __forceinline__ void fft_smem(C2<R>* buf, int ld_line, int ld_elem,
-                                         const C2<R>* __restrict__ tw) {
-  static_assert(stages_of<R>(L) > 0, "unsupported FFT length");
-  StockhamStage<R, L, INV, NT, NLINES, LINE_FAST, 0, 1, ZPAD>::run(buf, ld_line, ld_elem, tw);
-}
-
-// Contiguous padded lines of length L (line stride zpad_len(L)).
-template <typename R, int L, bool INV, int NT, int NLINES>
-__device__ __forceinline__ void fft_zlines(C2<R>* buf, const C2<R>* __restrict__ tw) {
-  fft_smem<R, L, INV, NT, NLINES, false, true>(buf, zpad_len<R>(L), 1, tw);
-}
 
 }  // namespace vk

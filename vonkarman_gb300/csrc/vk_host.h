@@ -52,7 +52,7 @@ enum StageOp : int {
   ST_ETD_CM_1 = 5, ST_ETD_CM_2 = 6, ST_ETD_CM_3 = 7,
   ST_RK4_1 = 8, ST_RK4_2 = 9, ST_RK4_3 = 10, ST_RK4_4 = 11,
 };
-enum EtdSlot : int { E_FULL = 0, E_HALF = 1, E_A21 = 2, E_A41 = 3, E_B1 = 4, E_B23 = 5, E_B4 = 6 };
+enum EtdSlot : int { E_FULL = 0, E_HALF = 1, E_A21 = 2, E_A41 = 3, E_B1 = 4, E_B23 = 5, E_B4 = 6, E_IK2 = 7 };
 constexpr int ETD_STRIDE = 8;
 
 template <typename R> struct StageArgs {
@@ -179,6 +179,8 @@ constexpr int RED_THREADS = 256;
 // Non-template launchers (vk_misc.cu).
 cudaError_t launch_etd_table(double* tab, int nent, double nu, double ks2, const DevScalars* d, int force,
                              const ContourConsts& cc, cudaStream_t s);
+// the table's E_IK2 entries (1 / |k|^2), which do not depend on dt
+cudaError_t launch_etd_ik2(double* tab, int nent, double ks2, cudaStream_t s);
 cudaError_t launch_cfl_update(DevScalars* d, double dx, double nu, double safety, int mode, cudaStream_t s);
 cudaError_t launch_reset_max(DevScalars* d, cudaStream_t s);
 cudaError_t launch_time_advance(DevScalars* d, cudaStream_t s);

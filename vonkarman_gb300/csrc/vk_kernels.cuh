@@ -53,15 +53,19 @@ __device__ __forceinline__ int signed_k(int i, int N) { return i < N / 2 ? i : i
 
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
+__host__ __device__ constexpr int ilog2(int a) { return a <= 1 ? 0 : 1 + ilog2(a / 2); }
 __host__ __device__ constexpr int round32(int a) { return (a + 31) / 32 * 32; }
 
-// z passes: column pairs per CTA so that CP * L == 768 (z-cross) / 512 (N grid)
+// z passes: column pairs per CTA so that CP * L reaches TARGET.  FP64: about a
+// hundred first-stage threads, and one pair on the smallest grids, where the
+// CTA count matters (N = 16: 288 CTAs).
 template <int L, int TARGET> __host__ __device__ constexpr int zpairs() { return cmax(1, TARGET / L); }
-template <typename R, int NLINES, int L>
-__host__ __device__ constexpr int zthreads() { return cmax(64, cmin(1024, round32(NLINES * L / max_radix<R>(L)))); }
-// Minimum resident CTAs per SM requested from the compiler: enough for 24
-// warps per SM, which caps registers near 85 per thread.
-template <int NT> __host__ __device__ constexpr int min_blocks() { return cmax(1, 768 / NT); }
+template <typename R, int M> __host__ __device__ constexpr int zcross_pairs() {
+  return sizeof(R) == 8 ? zpairs<M, (M >= 96 ? 192 : 1)>() : zpairs<M, 384>();
+}
+template <typename R, int N> __host__ __device__ constexpr int nz_pairs() {
+  return sizeof(R) == 8 ? zpairs<N, (N >= 64 ? 256 : 1)>() : zpairs<N, 512>();
+}
 
 // Grid sizes of a strided-pass op: compile-time when the op is instantiated
 // for one grid (GN > 0: N = GN, padded length M = GM, H = GN/2 + 1), so that
@@ -93,6 +97,8 @@ template <typename R, int GN = 0, int GM = 0> struct OpXInv {
   VK_PAD_ZEROS(GN, GM)
   __host__ __device__ __forceinline__ int kind(int f) const { return f < 3 ? 0 : 1; }
   __host__ __device__ __forceinline__ int src_component(int f) const { return f < 3 ? f : f - 2; }
+  // s_in = 1/N^3 is a power of two: the FP64 form applies it to the output exponent
+  template <int K> __host__ __device__ static constexpr int exp2() { return sizeof(R) == 8 ? -3 * ilog2(GN) : 0; }
   // L2 prefetch of row t of the input tile of field f, lines [lam0, lam0 + nl)
   // (the tile's rows are whole 128-byte lines)
   __device__ __forceinline__ void prefetch_row(int f, int lam0, int, int t) const {
@@ -104,7 +110,7 @@ template <typename R, int GN = 0, int GM = 0> struct OpXInv {
     return ix < 0 ? czero<R>() : in[(size_t)c * cs + ((ix * n_() + iy) * h_() + z)];
   }
   template <int K> __device__ __forceinline__ C2<R> prep(int, int, int, int p, C2<R> v) const {
-    v = cscale<R>(v, s_in);
+    if constexpr (sizeof(R) == 4) v = cscale<R>(v, s_in);
     if constexpr (K == 1) {
       const int ix = unpad_pos(p, n_(), m_());
       const R kx = ks * (R)signed_k(ix < 0 ? 0 : ix, n_());
@@ -431,8 +437,152 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
   }
 }
 
+// FP64 form of the stage epilogue, one mode per call.  The FP64 pipe (2 per
+// clock and SM) bounds it, so every product is fused and the factor s_out of
+// the nonlinear term (nl arrives without it) goes into the coefficients; the
+// operations are explicit, so that all instances round alike.  load() issues
+// the mode's global reads, apply() the arithmetic and the stores.
+struct StageF64 {
+  struct Mode {
+    bool ok;
+    int m;
+    size_t idx;
+    double ik2;                       // 1 / |k|^2, 0 at k = 0
+    double c0, c1, c2, c3;            // table entries of the stage
+    double2 u[3], a[3], b[3];
+  };
+  const StageArgs<double>& s;
+  const double so, dt;
+  __device__ __forceinline__ StageF64(const StageArgs<double>& st, double s_out)
+      : s(st), so(s_out), dt(st.op == ST_NL_OUT ? 0.0 : *st.dt) {}
 
-
+  __device__ __forceinline__ void read(const Mode& md, const double2* p, double2* v) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] = p[c * s.cs + md.idx];
+  }
+  __device__ __forceinline__ void load(Mode& md) const {
+    if (!md.ok) return;
+    const double* e = s.etd + (size_t)md.m * ETD_STRIDE;
+    md.ik2 = e[E_IK2];
+    if (s.op == ST_NL_OUT) return;
+    read(md, s.u, md.u);
+    switch (s.op) {
+      case ST_ETD_REF_1: case ST_ETD_CM_1:
+        md.c0 = e[E_HALF]; md.c1 = e[E_A21];
+        break;
+      case ST_ETD_REF_2: case ST_ETD_CM_2:
+        md.c0 = e[E_HALF]; md.c1 = e[E_A21]; md.c2 = e[E_B1]; md.c3 = e[E_B23];
+        read(md, s.n1, md.a);
+        break;
+      case ST_ETD_REF_3: case ST_ETD_CM_3:
+        md.c0 = s.op == ST_ETD_REF_3 ? e[E_FULL] : e[E_HALF];
+        md.c1 = s.op == ST_ETD_REF_3 ? e[E_A41] : e[E_A21];
+        md.c3 = e[E_B23];
+        read(md, s.n1, md.a);
+        read(md, s.acc, md.b);
+        break;
+      case ST_ETD_4:
+        md.c0 = e[E_FULL]; md.c1 = e[E_B4];
+        read(md, s.acc, md.b);
+        break;
+      case ST_RK4_2: case ST_RK4_3: case ST_RK4_4:
+        read(md, s.temp, md.a);
+        read(md, s.acc, md.b);
+        break;
+      default: break;
+    }
+  }
+  // a x + b y, and c + that
+  __device__ __forceinline__ static double2 lin(double a, double2 x, double b, double2 y) {
+    return make_double2(fma(a, x.x, b * y.x), fma(a, x.y, b * y.y));
+  }
+  __device__ __forceinline__ static double2 mac(double a, double2 x, double2 y) {
+    return make_double2(fma(a, x.x, y.x), fma(a, x.y, y.y));
+  }
+  __device__ __forceinline__ void apply(const Mode& md, const double2* nl, double2* un) const {
+    const size_t cs = s.cs;
+    switch (s.op) {
+      case ST_NL_OUT:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s.out[c * cs + md.idx] = make_double2(so * nl[c].x, so * nl[c].y);
+        return;
+      case ST_ETD_REF_1:    // solver.rs:264-281
+      case ST_ETD_CM_1: {   // textbook: a = E2 u + (h/2) phi1(z/2) N1
+        const double q = (s.op == ST_ETD_REF_1 ? dt : 0.5 * dt) * md.c1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double2 n = make_double2(so * nl[c].x, so * nl[c].y);
+          s.n1[c * cs + md.idx] = n;
+          s.temp[c * cs + md.idx] = lin(q, n, md.c0, md.u[c]);
+        }
+        return;
+      }
+      case ST_ETD_REF_2:    // solver.rs:291-308; acc starts the final sum
+      case ST_ETD_CM_2: {   // b = E2 u + (h/2) phi1(z/2) N2
+        const double q = (s.op == ST_ETD_REF_2 ? dt : 0.5 * dt) * md.c1 * so, b23 = md.c3 * so;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          s.acc[c * cs + md.idx] = lin(b23, nl[c], md.c2, md.a[c]);
+          s.temp[c * cs + md.idx] = lin(q, nl[c], md.c0, md.u[c]);
+        }
+        return;
+      }
+      case ST_ETD_REF_3: {  // solver.rs:318-344
+        const double q = dt * md.c1, q2 = 2.0 * q * so, b23 = md.c3 * so;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          s.acc[c * cs + md.idx] = mac(b23, nl[c], md.b[c]);
+          s.temp[c * cs + md.idx] = mac(q2, nl[c], lin(-q, md.a[c], md.c0, md.u[c]));
+        }
+        return;
+      }
+      case ST_ETD_CM_3: {   // c = E2 a + (h/2) phi1(z/2) (2 N3 - N1), a rebuilt from u, N1
+        const double q = 0.5 * dt * md.c1, q2 = 2.0 * q * so, b23 = md.c3 * so;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          s.acc[c * cs + md.idx] = mac(b23, nl[c], md.b[c]);
+          const double2 av = lin(q, md.a[c], md.c0, md.u[c]);
+          s.temp[c * cs + md.idx] = mac(q2, nl[c], lin(-q, md.a[c], md.c0, av));
+        }
+        return;
+      }
+      case ST_ETD_4: {      // solver.rs:354-378
+        const double b4 = dt * md.c1 * so;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double2 v = mac(b4, nl[c], lin(dt, md.b[c], md.c0, md.u[c]));
+          s.u_out[c * cs + md.idx] = v;
+          flag_nonfinite<double>(s, v);
+          un[c] = v;
+        }
+        return;
+      }
+      default: {            // rhs = N + (-nu k^2) state  (rk4.rs:30-45)
+        const double visc = -s.nu * (s.ks * s.ks * (double)md.m);
+        const double half = 0.5 * dt;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const size_t i = c * cs + md.idx;
+          const double2 rhs = lin(so, nl[c], visc, s.op == ST_RK4_1 ? md.u[c] : md.a[c]);
+          if (s.op == ST_RK4_1) {
+            s.acc[i] = rhs;
+            s.temp[i] = mac(half, rhs, md.u[c]);
+          } else if (s.op != ST_RK4_4) {
+            s.acc[i] = mac(2.0, rhs, md.b[c]);
+            s.temp[i] = mac(s.op == ST_RK4_2 ? half : dt, rhs, md.u[c]);
+          } else {
+            const double2 t = make_double2(md.b[c].x + rhs.x, md.b[c].y + rhs.y);
+            const double2 v = mac(dt / 6.0, t, md.u[c]);
+            s.u_out[i] = v;
+            flag_nonfinite<double>(s, v);
+            un[c] = v;
+          }
+        }
+        return;
+      }
+    }
+  }
+};
 
 // ---------------------------------------------------------------------------
 // z-line helpers.  Two real z lines x, y of length L share one complex line
@@ -444,16 +594,6 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 //                                 Y[k] = (Z[k] - conj Z[-k]) / (2i).
 // ---------------------------------------------------------------------------
 // Lines are in the padded shared layout (position p at zi<R>(p)).
-template <typename R>
-__device__ __forceinline__ void zpack(C2<R>* line, int L, int k, C2<R> X, C2<R> Y) {
-  if (k == 0 || 2 * k == L) {
-    line[zi<R>(k)] = cmk<R>(X.x, Y.x);
-  } else {
-    line[zi<R>(k)] = cmk<R>(X.x - Y.y, X.y + Y.x);
-    line[zi<R>(L - k)] = cmk<R>(X.x + Y.y, Y.x - X.y);
-  }
-}
-
 template <typename R>
 __device__ __forceinline__ void zunpack(const C2<R>* line, int L, int k, C2<R>& X, C2<R>& Y) {
   const C2<R> z = line[zi<R>(k)];
@@ -492,69 +632,6 @@ template <typename R> struct NZArgs {
 
 __device__ __forceinline__ void atomic_max_pos(unsigned long long* p, double v) {
   atomicMax(p, (unsigned long long)__double_as_longlong(v));
-}
-
-
-// ---------------------------------------------------------------------------
-// Standalone backend z passes (FftBackend::r2c_3d / c2r_3d z stage,
-// ndrustfft_backend.rs:33-57).  Real lines of length L, pairs of columns per
-// complex line.
-// ---------------------------------------------------------------------------
-template <typename R> struct FZArgs {
-  int ncols;                  // nx*ny
-  R* real; C2<R>* cplx;       // (ncols, L) real, (ncols, L/2+1) complex
-  R scale;                    // c2r: 1/(nx ny nz)
-};
-
-template <typename R, int L, int CP, int NT>
-__global__ void __launch_bounds__(NT, min_blocks<NT>()) k_fz_r2c(FZArgs<R> a, const C2<R>* __restrict__ tw) {
-  constexpr int H = L / 2 + 1;
-  constexpr int LP = zpad_len<R>(L);
-  extern __shared__ __align__(16) unsigned char vk_smem[];
-  C2<R>* lines = reinterpret_cast<C2<R>*>(vk_smem);
-  const int col0 = blockIdx.x * 2 * CP;
-  for (int e = threadIdx.x; e < CP * L; e += NT) {
-    const int pr = e / L, p = e % L;
-    const int c0 = col0 + 2 * pr;
-    const R x = c0 < a.ncols ? a.real[(size_t)c0 * L + p] : R(0);
-    const R y = c0 + 1 < a.ncols ? a.real[(size_t)(c0 + 1) * L + p] : R(0);
-    lines[pr * LP + zi<R>(p)] = cmk<R>(x, y);
-  }
-  __syncthreads();
-  fft_zlines<R, L, false, NT, CP>(lines, tw);
-  for (int e = threadIdx.x; e < CP * H; e += NT) {
-    const int pr = e / H, k = e % H;
-    const int c0 = col0 + 2 * pr;
-    C2<R> X, Y;
-    zunpack<R>(lines + pr * LP, L, k, X, Y);
-    if (c0 < a.ncols) a.cplx[(size_t)c0 * H + k] = X;
-    if (c0 + 1 < a.ncols) a.cplx[(size_t)(c0 + 1) * H + k] = Y;
-  }
-}
-
-template <typename R, int L, int CP, int NT>
-__global__ void __launch_bounds__(NT, min_blocks<NT>()) k_fz_c2r(FZArgs<R> a, const C2<R>* __restrict__ tw) {
-  constexpr int H = L / 2 + 1;
-  constexpr int LP = zpad_len<R>(L);
-  extern __shared__ __align__(16) unsigned char vk_smem[];
-  C2<R>* lines = reinterpret_cast<C2<R>*>(vk_smem);
-  const int col0 = blockIdx.x * 2 * CP;
-  for (int e = threadIdx.x; e < CP * H; e += NT) {
-    const int pr = e / H, k = e % H;
-    const int c0 = col0 + 2 * pr;
-    const C2<R> X = c0 < a.ncols ? a.cplx[(size_t)c0 * H + k] : czero<R>();
-    const C2<R> Y = c0 + 1 < a.ncols ? a.cplx[(size_t)(c0 + 1) * H + k] : czero<R>();
-    zpack<R>(lines + pr * LP, L, k, X, Y);
-  }
-  __syncthreads();
-  fft_zlines<R, L, true, NT, CP>(lines, tw);
-  for (int e = threadIdx.x; e < CP * L; e += NT) {
-    const int pr = e / L, p = e % L;
-    const int c0 = col0 + 2 * pr;
-    const C2<R> z = lines[pr * LP + zi<R>(p)];
-    if (c0 < a.ncols) a.real[(size_t)c0 * L + p] = z.x * a.scale;
-    if (c0 + 1 < a.ncols) a.real[(size_t)(c0 + 1) * L + p] = z.y * a.scale;
-  }
 }
 
 }  // namespace vk

@@ -21,6 +21,7 @@
 
 #include <type_traits>
 
+#include "vk_fix.cuh"
 #include "vk_kernels.cuh"
 #include "vk_reduce.cuh"
 
@@ -32,9 +33,9 @@
 
 namespace vk {
 
-// FP32 plans: at most two stages up to L = 768, composite in-register radices
-// 6/12/24/32; the larger radix goes first, where it carries no twiddles.  FP64 plans: radix <= 8 (register budget), as in the
-// shared-memory engine.
+// At most two stages up to L = 768, with composite in-register radices; the
+// larger radix goes first, where it carries no twiddles (and where padded
+// inputs prune it).
 __host__ __device__ constexpr int rplan_stages_f(int L) {
   return (L == 8 || L == 12 || L == 16 || L == 24) ? 1
        : (L == 32 || L == 48 || L == 64 || L == 96 || L == 128 || L == 192 || L == 256 || L == 384 || L == 512 || L == 768) ? 2
@@ -60,16 +61,22 @@ __host__ __device__ constexpr int rplan_radix_f(int L, int s) {
 __host__ __device__ constexpr int rplan_radix_fc(int L, int s) {
   return L == 384 ? (s == 0 ? 16 : 24) : rplan_radix_f(L, s);
 }
+// FP64 lines run in fixed point with the plans of vk_fix.cuh, the same for both
+// thread maps.
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rstages(int L) {
-  return sizeof(R) == 4 ? rplan_stages_f(L) : plan_stages(L);
+  return sizeof(R) == 4 ? rplan_stages_f(L) : fx_supported(L) ? 2 : -1;
 }
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rradix(int L, int s) {
-  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : plan_radix(L, s);
+  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : fx_radix(L, s);
 }
-// threads of a CTA: one butterfly per thread in the widest stage
+// threads of a CTA: one butterfly per thread in the widest stage (FP64 above 96
+// points: in the first stage, and a line of the second)
 template <typename R, int L, int NLINES, bool CONTIG = false, int S = 0>
 __host__ __device__ constexpr int rthreads() {
-  if constexpr (S >= rstages<R, CONTIG>(L)) {
+  if constexpr (sizeof(R) == 8) {
+    constexpr int nb0 = L / fx_radix(L, 0), nb1 = L / fx_radix(L, 1);
+    return round32(L <= 96 ? cmax(nb0, nb1) * NLINES : cmax(nb0 * NLINES, CONTIG ? nb1 : 0));
+  } else if constexpr (S >= rstages<R, CONTIG>(L)) {
     return 32;
   } else {
     return cmax(round32(L / rradix<R, CONTIG>(L, S) * NLINES), rthreads<R, L, NLINES, CONTIG, S + 1>());
@@ -114,6 +121,12 @@ __device__ __forceinline__ int ridx(int pos, int l) {
   }
 }
 
+// Resident CTAs per SM of the fixed-point kernels: radices 16 to 32 of 64-bit
+// complex integers hold 64 to 128 registers of data, so about 12 warps of up
+// to 168 registers per SM.
+template <int L, int NT>
+__host__ __device__ constexpr int fx_min_blocks() { return L >= 512 ? 1 : cmax(1, 384 / NT); }
+
 // Minimum resident CTAs per SM requested from the compiler (caps registers):
 // 24 warps per SM for the strided passes where the plan allows it; one or two
 // CTAs for the long FP64 / 768-point plans and for the multi-field P5 kernels
@@ -121,7 +134,7 @@ __device__ __forceinline__ int ridx(int pos, int l) {
 template <typename R, int L, int NT, bool EPI = false>
 __host__ __device__ constexpr int lines_min_blocks() {
   if constexpr (sizeof(R) == 8) {
-    return L >= 512 ? 1 : cmax(1, 768 / NT);
+    return fx_min_blocks<L, NT>();
   } else {
     return L >= 768 ? (EPI ? 1 : 2) : EPI ? cmax(1, 512 / NT) : L >= 512 ? 2 : L >= 384 ? (NT >= 384 ? 2 : 3)
          : NT < 128 ? 4 : cmax(1, 768 / NT);
@@ -274,18 +287,225 @@ struct RegStage {
   }
 };
 
+// FP64 lines in fixed point.  The outputs are multiplied by 2^xe.
+//
+// Stage 0: one butterfly per thread.  Its bound of the inputs' magnitudes
+// (fx_bound) is maximised over the line's threads, by shuffles where a line's
+// butterflies share a warp (contiguous lines) and through shared memory
+// otherwise, and gives the line's exponent.  Stage 1 loops over the rest in
+// rounds of NT threads (whole lines per round where the store functor writes
+// back into the exchange buffer, SL), so that a CTA needs no more threads than
+// stage 0 keeps busy.
+//
+// Lines whose bound is outside the comfortable range carry a code: all zero
+// (the transform's rounding compensations would leave a few units), tiny and
+// huge (scaled by 2^+-FX_RANGE on the way in and back on the way out) or with a
+// NaN or Inf among the inputs (every output is NaN).
+constexpr int FX_RANGE = 600;
+enum FxCode : int { FX_PLAIN = 0, FX_ZERO = 1, FX_TINY = 2, FX_HUGE = 3, FX_NAN = 4 };
+__device__ __forceinline__ double fx_code_factor(int code) {
+  return code == FX_ZERO ? 0.0
+       : code == FX_TINY ? __hiloint2double((1023 - FX_RANGE) << 20, 0)
+       : code == FX_HUGE ? __hiloint2double((1023 + FX_RANGE) << 20, 0)
+                         : __longlong_as_double(0x7ff8000000000000ll);
+}
+// v 2^q, q20 = q << 20 (within the normal range)
+__device__ __forceinline__ double fx_to_double(long long v, int q20) {
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double(h != 0 ? h + q20 : 0, __double2loint(d));
+}
+
+template <int L, int NT, int NLINES, class MAP>
+__host__ __device__ constexpr int fx_round_lines() {   // lines per stage-1 round (contiguous lines)
+  return NT / (L / fx_radix(L, 1)) < NLINES ? NT / (L / fx_radix(L, 1)) : NLINES;
+}
+
+template <int L, bool INV, int NT, int NLINES, class MAP, bool SL, int Z0, int Z1>
+struct FxLines {
+  static constexpr int R0 = fx_radix(L, 0), NB0 = L / R0, G0 = NB0 * NLINES;
+  static constexpr int R1 = fx_radix(L, 1), NB1 = L / R1, G1 = NB1 * NLINES;
+  static constexpr int GR = fx_growth(R1);
+  static constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
+  static constexpr int NW0 = (G0 + 31) / 32;
+  static constexpr int CODE_SHIFT = 24;   // stored line state: exponent + (code << 24)
+  static_assert(G0 <= NT, "one first-stage butterfly per thread");
+  static_assert(!MAP::CONTIG || 32 % NB0 == 0, "a contiguous line's first stage shares a warp");
+  static_assert(MAP::CONTIG || (32 % NLINES == 0 && !SL), "interleaved lines tile a warp");
+
+  __device__ __forceinline__ static int line_max(int m, int* part) {
+    if constexpr (MAP::CONTIG) {
+#pragma unroll
+      for (int o = 1; o < NB0; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    } else {
+#pragma unroll
+      for (int o = NLINES; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const int w = threadIdx.x / 32, ln = threadIdx.x % 32;
+      if (w < NW0 && ln < NLINES) part[w * NLINES + ln] = m;
+      __syncthreads();
+      m = part[ln % NLINES];
+#pragma unroll
+      for (int i = 1; i < NW0; ++i) m = max(m, part[i * NLINES + ln % NLINES]);
+    }
+    return m;
+  }
+
+  // the butterfly's outputs as doubles, stored
+  template <int RAD, class STF>
+  __device__ __forceinline__ static void emit(const fx2* v, int l, int base, int ns, int q, int code, const STF& st) {
+    double2 d[RAD];
+    const int q20 = q << 20;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) d[r] = make_double2(fx_to_double(v[r].x, q20), fx_to_double(v[r].y, q20));
+    if (code != FX_PLAIN) {
+      const double f = fx_code_factor(code);
+#pragma unroll
+      for (int r = 0; r < RAD; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
+    }
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) st(l, base + r * ns, d[r]);
+  }
+
+  // fill(l, j, d): the inputs at positions j + r NB0 of line l (those of ZM excepted)
+  template <class FILL, class STF>
+  __device__ __forceinline__ static void run(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, const STF& st,
+                                             int xe) {
+    __shared__ int part[MAP::CONTIG ? 1 : NW0 * NLINES];
+    __shared__ int line_s[MAP::CONTIG ? NLINES : 1];
+    const int g = threadIdx.x;
+    const int l0 = MAP::template line<NB0>(g), j0 = MAP::template bfly<NB0>(g);
+    const bool act = G0 == NT || g < G0;
+    double2 d[R0];
+    int k = 0;
+    if (act) {
+      __builtin_assume(j0 >= 0 && j0 < NB0);
+      __builtin_assume(l0 >= 0 && l0 < NLINES);
+      fill(l0, j0, d);
+      int top = 0;
+#pragma unroll
+      for (int r = 0; r < R0; ++r)
+        if (!((ZM >> r) & 1u))
+          top = max(top, max(__double2hiint(d[r].x) & 0x7fffffff, __double2hiint(d[r].y) & 0x7fffffff));
+      float sum = 0.f;
+#pragma unroll
+      for (int r = 0; r < R0; ++r)
+        if (!((ZM >> r) & 1u))
+          sum += fx_relative(max(__double2hiint(d[r].x) & 0x7fffffff, __double2hiint(d[r].y) & 0x7fffffff), top);
+      k = top == 0 ? 0 : top >= 0x7ff00000 ? 0x7fff : fx_bound(top, sum);
+    }
+    k = line_max(k, part);
+    int code = FX_PLAIN;
+    if (k < 1023 - 900 || k > 1023 + 900) {
+      code = k == 0 ? FX_ZERO : k == 0x7fff ? FX_NAN : k < 1023 ? FX_TINY : FX_HUGE;
+      k = code == FX_TINY ? k + FX_RANGE : code == FX_HUGE ? k - FX_RANGE : 1023;
+      if (act) {
+        const double f = code == FX_TINY ? fx_code_factor(FX_HUGE) : code == FX_HUGE ? fx_code_factor(FX_TINY) : 0.0;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
+      }
+    }
+    int q = fx_quantum(k) + GR + xe;
+    fx2 v[R0];
+    if (act) {
+#pragma unroll
+      for (int r = 0; r < R0; ++r) {
+        if ((ZM >> r) & 1u) {
+          v[r] = fx2{0, 0};
+        } else {
+          v[r].x = fx_from_double(__double2hiint(d[r].x), __double2loint(d[r].x), k);
+          v[r].y = fx_from_double(__double2hiint(d[r].y), __double2loint(d[r].y), k);
+        }
+      }
+      FxDft<R0, INV>::run(v);
+    }
+    if (act) {
+      if (MAP::CONTIG && j0 == 0) line_s[l0] = q + (code << CODE_SHIFT);
+      sfor<R0>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (FxSpecial<R0, R1>::output(r)) v[r] = fx_multiple<GR + 1>(v[r]);
+        xb[MAP::template idx<0>(j0 * R0 + r, l0)] = v[r];
+      });
+    }
+    __syncthreads();
+    // rounds of stage 1: whole lines (contiguous) or butterflies of all lines
+    constexpr int RL = MAP::CONTIG ? fx_round_lines<L, NT, NLINES, MAP>() : NLINES;
+    constexpr int PER = MAP::CONTIG ? RL * NB1 : NT;                 // butterflies per round
+    constexpr int ROUNDS = MAP::CONTIG ? (NLINES + RL - 1) / RL : (G1 + NT - 1) / NT;
+    static_assert(RL >= 1, "a round holds a line");
+#pragma unroll 1
+    for (int i = 0; i < ROUNDS; ++i) {
+      const int gi = i * PER + g;
+      const int l = MAP::template line<NB1>(gi), j = MAP::template bfly<NB1>(gi);
+      const bool act1 = (PER == NT || g < PER) && (G1 % PER == 0 || gi < G1);
+      fx2 u[R1];
+      int qs = q, cs = code;
+      if (act1) {
+        __builtin_assume(j >= 0 && j < NB1);
+        __builtin_assume(l >= 0 && l < NLINES);
+        if (MAP::CONTIG) {
+          const int s = line_s[l];
+          cs = (s + (1 << (CODE_SHIFT - 1))) >> CODE_SHIFT;
+          qs = s - (cs << CODE_SHIFT);
+        }
+#pragma unroll
+        for (int r = 0; r < R1; ++r) u[r] = xb[MAP::template idx<0>(j + r * NB1, l)];
+      }
+      if constexpr (SL) __syncthreads();
+      if (act1) {
+        u[0] = fx_shift<GR>(u[0]);
+        sfor<R1 - 1>([&](auto rc) {
+          constexpr int r = decltype(rc)::value + 1;
+          u[r] = fx_twiddle<INV>(u[r], tw[(r - 1) * R0 + j], FxSpecial<R0, R1>::template round0<r>(j));
+        });
+        FxDft<R1, INV>::run(u);
+        emit<R1>(u, l, j, R0, qs, cs, st);
+      }
+    }
+  }
+};
+
+// fill functor of FxLines from ld / pp: all loads of a chunk are issued before
+// any arithmetic on them (chunks of 256 bytes per thread where the raw inputs
+// are wider than one complex value)
+template <int L, int Z0, int Z1, class LD, class PP> struct FxFill {
+  const LD& ld;
+  const PP& pp;
+  __device__ __forceinline__ void operator()(int l, int j, double2* d) const {
+    constexpr int R0 = fx_radix(L, 0), NB0 = L / R0;
+    constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
+    using Raw = decltype(ld(0, 0));
+    constexpr int CH = sizeof(Raw) > sizeof(double2) ? cmin(R0, (int)(256 / sizeof(Raw))) : R0;
+#pragma unroll
+    for (int r0 = 0; r0 < R0; r0 += CH) {
+      Raw raw[CH];
+#pragma unroll
+      for (int r = 0; r < CH; ++r)
+        if (r0 + r < R0 && !((ZM >> (r0 + r)) & 1u)) raw[r] = ld(l, j + (r0 + r) * NB0);
+#pragma unroll
+      for (int r = 0; r < CH; ++r)
+        if (r0 + r < R0 && !((ZM >> (r0 + r)) & 1u)) d[r0 + r] = pp(l, j + (r0 + r) * NB0, raw[r]);
+    }
+  }
+};
+
 // Transform NLINES lines.  All NT threads must call it; the exchange buffer
 // xb (MAP::elems() elements) must not be in use by any thread.  Returns with
 // no synchronisation after the last stage.
 // SL: the store functor writes into xb itself (in place), so the last stage
-// also waits for all readers before storing.  TT: tw is the per-stage table
-// of load_twtab (shared memory), else the plain W_L^m table.
+// also waits for all readers before storing.  tw is the per-stage table of
+// load_twtab (shared memory).
 template <typename R, int L, bool INV, int NT, int NLINES, class MAP = MapInterleaved<R, L, NLINES>, bool SL = false,
           bool TT = false, int Z0 = 0, int Z1 = 0, class LD, class PP, class ST>
 __device__ __forceinline__ void fft_lines(C2<R>* xb, const C2<R>* __restrict__ tw, const LD& ld, const PP& pp,
                                           const ST& st) {
   static_assert(rstages<R>(L) > 0, "unsupported FFT length");
-  RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
+  if constexpr (sizeof(R) == 8) {
+    static_assert(TT, "per-stage tables");
+    FxLines<L, INV, NT, NLINES, MAP, SL, Z0, Z1>::run(reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw),
+                                                      FxFill<L, Z0, Z1, LD, PP>{ld, pp}, st, 0);
+  } else {
+    RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
+  }
 }
 // pp for inputs that need no arithmetic after the load
 struct PrepNone {
@@ -315,6 +535,12 @@ __device__ __forceinline__ void load_twtab(C2<R>* tab, const C2<R>* __restrict__
 template <class Op, class = void> struct OpZeroRange { static constexpr int lo = 0, hi = 0; };
 template <class Op> struct OpZeroRange<Op, std::void_t<decltype(Op::ZERO_LO)>> {
   static constexpr int lo = Op::ZERO_LO, hi = Op::ZERO_HI;
+};
+
+// Power of two that an op's FP64 outputs carry (Op::exp2<K>(); 0 by default)
+template <class Op, int K, class = void> struct OpExp2 { static constexpr int value = 0; };
+template <class Op, int K> struct OpExp2<Op, K, std::void_t<decltype(Op::template exp2<K>())>> {
+  static constexpr int value = Op::template exp2<K>();
 };
 
 // Ops that supply prefetch_row(f, lam0, nl, t) (an L2 hint for row t of a
@@ -361,6 +587,28 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
     const int i = op.out_index(p);
     if (ok && i >= 0) op.store(f, outer, z, i, v);
   };
+  if constexpr (sizeof(R) == 8) {
+    // one transform for all kinds, whose loads alone differ: the transform's
+    // code is large, and CTAs of several kinds share an SM's instruction cache
+    constexpr int Z0 = OpZeroRange<Op>::lo, Z1 = OpZeroRange<Op>::hi;
+    auto fill = [&](int l, int j, double2* d) {
+      sfor<Op::NKIND>([&](auto kc) {
+        constexpr int K = decltype(kc)::value;
+        if (kd != K) return;   // uniform over the CTA
+        const auto ld = [&](int, int p) { return op.template load<K>(f, outer, z, p); };
+        const auto pp = [&](int, int p, const auto& raw) { return op.template prep<K>(f, outer, z, p, raw); };
+        FxFill<L, Z0, Z1, decltype(ld), decltype(pp)>{ld, pp}(l, j, d);
+      });
+    };
+    int xe = 0;
+    sfor<Op::NKIND>([&](auto kc) {
+      constexpr int K = decltype(kc)::value;
+      if (kd == K) xe = OpExp2<Op, K>::value;
+    });
+    FxLines<L, INV, NT, NLINES, MapInterleaved<R, L, NLINES>, false, Z0, Z1>::run(
+        reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw_s), fill, st, xe);
+    return;
+  } else {
   sfor<Op::NKIND>([&](auto kc) {
     constexpr int K = decltype(kc)::value;
     if (kd != K) return;   // uniform over the CTA
@@ -369,6 +617,7 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
         xb, tw_s, [&](int, int p) { return op.template load<K>(f, outer, z, p); },
         [&](int, int p, const auto& raw) { return op.template prep<K>(f, outer, z, p, raw); }, st);
   });
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -392,14 +641,17 @@ template <typename R, int L> struct P5Lines { static constexpr int value = p5_li
 // Threads of k_p5: one butterfly per thread in the widest FFT stage; FP32 up
 // to 384 points doubles them (measured 4 % faster at 384: the epilogue keeps
 // the same modes in flight per CTA with one mode per thread, and twice the
-// warps hide its arithmetic), two CTAs per SM.
+// warps hide its arithmetic), two CTAs per SM.  FP64 takes at least 128, for
+// its epilogue, and as many CTAs as shared memory allows (three at 384 points).
 template <typename R, int L, int NLINES>
 __host__ __device__ constexpr int p5_threads() {
-  return sizeof(R) == 4 && L <= 384 ? cmin(2 * rthreads<R, L, NLINES>(), 384) : cmin(rthreads<R, L, NLINES>(), 384);
+  return sizeof(R) == 8 ? cmax(128, rthreads<R, L, NLINES>())
+       : L <= 384 ? cmin(2 * rthreads<R, L, NLINES>(), 384) : cmin(rthreads<R, L, NLINES>(), 384);
 }
 template <typename R, int L, int NLINES, int NT>
 __host__ __device__ constexpr int p5_min_blocks() {
-  return NT >= 2 * rthreads<R, L, NLINES>() ? 2 : lines_min_blocks<R, L, NT, true>();
+  return sizeof(R) == 8 ? (L >= 512 ? 1 : 3)
+       : NT >= 2 * rthreads<R, L, NLINES>() ? 2 : lines_min_blocks<R, L, NT, true>();
 }
 
 // DIAG: the instance for final stages whose new state also feeds the fused
@@ -432,6 +684,20 @@ k_p5(P5Args<R> a, const C2<R>* __restrict__ tw) {
     const bool ok = lam < a.nlines;
     const int iy = ok ? lam / H : 0;
     const int z = ok ? lam - iy * H : 0;
+    if constexpr (sizeof(R) == 8) {
+      // (a loop, not unrolled: the FP64 transform's code is large)
+#pragma unroll 1
+      for (int c = 0; c < 3; ++c) {
+        if (c > 0) __syncthreads();   // xb is reused
+        const C2<R>* src = a.in + (size_t)c * a.fsin + (iy * H + z);
+        fft_lines<R, L, false, NT, NLINES, MapInterleaved<R, L, NLINES>, false, true>(
+            xb, tw_s, [&](int, int p) { return src[p * (N * H)]; }, PrepNone{},
+            [&](int, int p, C2<R> v) {
+              const int ix = unpad_pos(p, N, L);
+              if (ix >= 0) keep[(c * N + ix) * NLINES + (int)(threadIdx.x % NLINES)] = v;
+            });
+      }
+    } else {
     sfor<3>([&](auto cc) {
       constexpr int C = decltype(cc)::value;
       if (C > 0) __syncthreads();   // xb is reused
@@ -443,12 +709,65 @@ k_p5(P5Args<R> a, const C2<R>* __restrict__ tw) {
             if (ix >= 0) keep[(C * N + ix) * NLINES + (int)(threadIdx.x % NLINES)] = v;
           });
     });
+    }
   }
   __syncthreads();
+  if constexpr (sizeof(R) == 8) {
+    // two modes per iteration, so that the loads of both are in flight together
+    constexpr int EM = 2;
+    const int l = threadIdx.x % NLINES;
+    const int lam = blockIdx.x * NLINES + l;
+    const bool line_ok = lam < a.nlines;
+    const int iy = line_ok ? lam / H : 0;
+    const int z = line_ok ? lam - iy * H : 0;
+    const int kyi = signed_k(iy, N);
+    const double ky = a.ks * (double)kyi, kz = a.ks * (double)z;
+    const double w = (z == 0 || z == N / 2) ? 1.0 : 2.0;   // R2C weight
+    StageF64 stage(a.st, a.s_out);
+#pragma unroll 1
+    for (int ix0 = threadIdx.x / NLINES; ix0 < N; ix0 += EM * (NT / NLINES)) {
+      StageF64::Mode md[EM];
+#pragma unroll
+      for (int q = 0; q < EM; ++q) {
+        const int ix = ix0 + q * (NT / NLINES);
+        const int kxi = signed_k(ix < N ? ix : 0, N);
+        md[q].ok = line_ok && ix < N;
+        md[q].idx = ((size_t)(ix < N ? ix : 0) * N + iy) * H + z;
+        md[q].m = kxi * kxi + kyi * kyi + z * z;
+        stage.load(md[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < EM; ++q) {
+        if (!md[q].ok) continue;
+        const int ix = ix0 + q * (NT / NLINES);
+        const int e = ix * NLINES + l;
+        const int kxi = signed_k(ix, N);
+        const double kx = a.ks * (double)kxi;
+        const double2 x = keep[e], y = keep[N * NLINES + e], v = keep[2 * N * NLINES + e];
+        const double dr = fma(kz, v.x, fma(ky, y.x, kx * x.x)) * md[q].ik2;
+        const double di = fma(kz, v.y, fma(ky, y.y, kx * x.y)) * md[q].ik2;
+        const double2 nl[3] = {make_double2(fma(-kx, dr, x.x), fma(-kx, di, x.y)),
+                               make_double2(fma(-ky, dr, y.x), fma(-ky, di, y.y)),
+                               make_double2(fma(-kz, dr, v.x), fma(-kz, di, v.y))};
+        double2 un[3];
+        stage.apply(md[q], nl, un);
+        if constexpr (DIAG) {
+          if (d_t1) {
+            double te, en, he, sh;
+            tier1_terms<double>(kx, ky, kz, un, te, en, he, sh);
+            dsum[0] += w * te; dsum[1] += w * en; dsum[2] += w * he; dsum[3] += w * sh;
+          }
+          if (d_sp) {
+            const int shell = shell_of(kxi, kyi, z, a.st.ks, ks_one);
+            if (shell < a.st.nsh) atomicAdd(&hist[shell], w * spectrum_term<double>(un));
+          }
+        }
+      }
+    }
+  } else {
   // FP32 with the FFT's thread count: two modes per iteration, so that the
-  // epilogue's loads of both are in flight together (FP64 keeps one: register
-  // budget, FP64-pipe bound; doubled threads keep one)
-  constexpr int EM = sizeof(R) == 4 && NT < 2 * rthreads<R, L, NLINES>() ? 2 : 1;
+  // epilogue's loads of both are in flight together (doubled threads keep one)
+  constexpr int EM = NT < 2 * rthreads<R, L, NLINES>() ? 2 : 1;
 #pragma unroll 1
   for (int e0 = threadIdx.x; e0 < N * NLINES; e0 += EM * NT) {
     size_t idx[EM];
@@ -506,6 +825,7 @@ k_p5(P5Args<R> a, const C2<R>* __restrict__ tw) {
         }
       }
     }
+  }
   }
   if constexpr (DIAG) {
     // the CTA's row: Tier-1 sums by a fixed shuffle / warp-order tree, then
@@ -624,8 +944,8 @@ __host__ __device__ constexpr bool z_row_unpack() {
 }
 
 template <typename R, int M, int CP, int NT>
-__global__ void __launch_bounds__(NT, M >= 768 ? (sizeof(R) == 4 && p3_inplace<CP>() ? 3 : 1)
-                                              : cmax(1, (sizeof(R) == 8 ? 768 : 512) / NT))
+__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? fx_min_blocks<M, NT>()
+                                      : M >= 768 ? (p3_inplace<CP>() ? 3 : 1) : cmax(1, 512 / NT))
 k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int N = 2 * M / 3;
   constexpr int H = N / 2 + 1;
@@ -736,7 +1056,7 @@ __host__ __device__ constexpr int nz_threads() {
 }
 
 template <typename R, int N, int CP, bool BOTH, int NT>
-__global__ void __launch_bounds__(NT, N >= 512 ? 1 : cmax(1, (sizeof(R) == 8 ? 768 : 512) / NT))
+__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? fx_min_blocks<N, NT>() : N >= 512 ? 1 : cmax(1, 512 / NT))
 k_nz_max(NZArgs<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int H = N / 2 + 1;
   constexpr int LPP = BOTH ? 6 : 3;   // lines per column pair
@@ -839,5 +1159,83 @@ k_nz_max(NZArgs<R> a, const C2<R>* __restrict__ tw, int pf) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Standalone backend z passes (FftBackend::r2c_3d / c2r_3d z stage,
+// ndrustfft_backend.rs:33-57).  Real lines of length L, two columns per complex
+// line, CP lines per CTA: r2c reads the pair into the first stage, leaves the
+// spectrum in shared memory and unpacks it; c2r packs the half spectra (with
+// the Hermitian extension) in the first stage's loads and stores the two real
+// columns from the last stage's registers.
+// ---------------------------------------------------------------------------
+template <typename R> struct FZArgs {
+  int ncols;                  // nx*ny
+  R* real; C2<R>* cplx;       // (ncols, L) real, (ncols, L/2+1) complex
+  R scale;                    // c2r: 1/(nx ny nz)
+};
+// lines per CTA: about 192 threads in the wider stage
+template <typename R, int L> __host__ __device__ constexpr int fz_pairs() {
+  int rad = rradix<R, true>(L, 0);
+  for (int s = 1; s < rstages<R, true>(L); ++s) rad = cmin(rad, rradix<R, true>(L, s));
+  return cmax(1, 192 * rad / L);
+}
+template <typename R, int NT>
+__host__ __device__ constexpr int fz_min_blocks() { return cmax(1, (sizeof(R) == 8 ? 384 : 768) / NT); }
+
+template <typename R, int L, int CP, int NT>
+__global__ void __launch_bounds__(NT, fz_min_blocks<R, NT>()) k_fz_r2c(FZArgs<R> a, const C2<R>* __restrict__ tw) {
+  constexpr int H = L / 2 + 1;
+  constexpr int LP = zpad_len<R>(L);
+  extern __shared__ __align__(16) unsigned char vk_smem[];
+  __shared__ C2<R> tw_s[twtab_elems<R, true>(L)];
+  load_twtab<R, L, true, NT>(tw_s, tw);
+  C2<R>* lines = reinterpret_cast<C2<R>*>(vk_smem);
+  const int col0 = blockIdx.x * 2 * CP;
+  fft_lines<R, L, false, NT, CP, MapContig<R, L, CP>, true, true>(
+      lines, tw_s,
+      [&](int l, int p) -> C2<R> {
+        const int c = col0 + 2 * l;
+        const R* x = a.real + (size_t)c * L + p;
+        return cmk<R>(c < a.ncols ? x[0] : R(0), c + 1 < a.ncols ? x[L] : R(0));
+      },
+      PrepNone{}, [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
+  __syncthreads();
+  for (int e = threadIdx.x; e < 2 * CP * H; e += NT) {
+    const int col = e / H, k = e % H;
+    if (col0 + col >= a.ncols) break;
+    C2<R> X, Y;
+    zunpack<R>(lines + (col / 2) * LP, L, k, X, Y);
+    a.cplx[(size_t)(col0 + col) * H + k] = col % 2 == 0 ? X : Y;
+  }
+}
+
+template <typename R, int L, int CP, int NT>
+__global__ void __launch_bounds__(NT, fz_min_blocks<R, NT>()) k_fz_c2r(FZArgs<R> a, const C2<R>* __restrict__ tw) {
+  constexpr int H = L / 2 + 1;
+  extern __shared__ __align__(16) unsigned char vk_smem[];
+  __shared__ C2<R> tw_s[twtab_elems<R, true>(L)];
+  load_twtab<R, L, true, NT>(tw_s, tw);
+  const int col0 = blockIdx.x * 2 * CP;
+  fft_lines<R, L, true, NT, CP, MapContig<R, L, CP>, false, true>(
+      reinterpret_cast<C2<R>*>(vk_smem), tw_s,
+      [&](int l, int p) -> C2x2<R> {
+        const int c = col0 + 2 * l;
+        const C2<R>* x = a.cplx + (size_t)c * H + (p < H ? p : L - p);
+        C2x2<R> r{};
+        if (c < a.ncols) r.a = x[0];
+        if (c + 1 < a.ncols) r.b = x[H];
+        return r;
+      },
+      [&](int, int p, const C2x2<R>& r) -> C2<R> {   // Z = X + i Y with the Hermitian extension
+        const C2<R> X = r.a, Y = r.b;
+        if (p == 0 || 2 * p == L) return cmk<R>(X.x, Y.x);   // c2r drops these imaginary parts
+        return p < H ? cmk<R>(X.x - Y.y, X.y + Y.x) : cmk<R>(X.x + Y.y, Y.x - X.y);
+      },
+      [&](int l, int p, C2<R> z) {
+        const int c = col0 + 2 * l;
+        R* x = a.real + (size_t)c * L + p;
+        if (c < a.ncols) x[0] = z.x * a.scale;
+        if (c + 1 < a.ncols) x[L] = z.y * a.scale;
+      });
+}
 
 }  // namespace vk

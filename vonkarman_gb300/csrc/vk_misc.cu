@@ -17,6 +17,11 @@ namespace vk {
 #ifndef VK_ETD_SHARED_RCP
 #define VK_ETD_SHARED_RCP 1
 #endif
+__global__ void k_etd_ik2(double* __restrict__ tab, int nent, double ks2) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m < nent) tab[(size_t)m * ETD_STRIDE + E_IK2] = m == 0 ? 0.0 : 1.0 / (ks2 * (double)m);
+}
+
 __global__ void k_etd_table(double* __restrict__ tab, int nent, double nu, double ks2,
                             const DevScalars* __restrict__ d, int force, ContourConsts cc) {
   if (!force && d->etd_recompute == 0) return;
@@ -95,7 +100,6 @@ __global__ void k_etd_table(double* __restrict__ tab, int nent, double nu, doubl
   t[E_B1] = p1 - 3.0 * p2 + 4.0 * p3;
   t[E_B23] = 2.0 * p2 - 4.0 * p3;
   t[E_B4] = -p2 + 4.0 * p3;
-  t[7] = 0.0;
 }
 
 // CFL step size on the N grid (solver.rs:180-218) and the 1% re-tabulation
@@ -208,6 +212,11 @@ cudaError_t launch_etd_table(double* tab, int nent, double nu, double ks2, const
                              const ContourConsts& cc, cudaStream_t s) {
   const int nt = 128;
   k_etd_table<<<(nent + nt - 1) / nt, nt, 0, s>>>(tab, nent, nu, ks2, d, force, cc);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_etd_ik2(double* tab, int nent, double ks2, cudaStream_t s) {
+  k_etd_ik2<<<(nent + 255) / 256, 256, 0, s>>>(tab, nent, ks2);
   return cudaGetLastError();
 }
 
