@@ -6,6 +6,7 @@
 #include <cmath>
 #include <complex>
 #include <cstdio>
+#include <map>
 #include <random>
 #include <vector>
 
@@ -22,45 +23,40 @@ static std::vector<CL> roots(int L) {
   return w;
 }
 
-template <int R0, int R1, bool INV> struct Line {
-  static constexpr int L = R0 * R1, G = fx_growth(R1);
+// one line through the plan of length L
+template <int L, bool CONTIG, bool INV> struct Line {
+  static constexpr int ST = fx_stages(L, CONTIG), SHIFT = fx_total_growth(L, CONTIG);
+  static constexpr int R0 = fx_radix(L, 0, CONTIG), NB0 = L / R0;
   std::vector<fxtw> tw;
   Line() : tw(L) {
-    const auto w = roots(L);
-    for (int m = 0; m < L; ++m) {
-      fx_words(w[m].real(), 64 - G, tw[m].ch, tw[m].cl);
-      fx_words(w[m].imag(), 64 - G, tw[m].dh, tw[m].dl);
-    }
+    for (int m = 0; m < L; ++m) tw[m] = fx_make_twiddle(m, L, cosl(TWO_PI * m / L), sinl(TWO_PI * m / L));
   }
-  template <int R> void twiddle(fx2* t, int j) const {
-    if constexpr (R < R1) {
-      t[R] = fx_twiddle<INV>(t[R], tw[R * j % L], FxSpecial<R0, R1>::template round0<R>(j));
-      twiddle<R + 1>(t, j);
+  template <int S, int NS> void stages(std::vector<fx2>& v) const {
+    constexpr int R = fx_radix(L, S, CONTIG), NB = L / R, G = fx_growth(R);
+    constexpr int GN = S + 1 < ST ? fx_growth(fx_radix(L, S + 1, CONTIG)) : 1;
+    std::vector<fx2> o(L);
+    for (int j = 0; j < NB; ++j) {
+      const int k = j % NS;
+      fx2 t[R];
+      for (int r = 0; r < R; ++r) {
+        t[r] = v[j + r * NB];
+        if (S > 0) t[r] = r == 0 ? fx_shift<G>(t[r]) : fx_twiddle<INV>(t[r], fx_stage_twiddle(tw[r * k * (L / (NS * R))], G));
+      }
+      FxDft<R, INV>::run(t);
+      if (S + 1 < ST) t[0] = fx_multiple<GN>(t[0]);
+      for (int r = 0; r < R; ++r) o[(j - k) * R + k + r * NS] = t[r];
     }
+    v = o;
+    if constexpr (S + 1 < ST) stages<S + 1, NS * R>(v);
   }
-  std::vector<fx2> run(const std::vector<fx2>& v) const {
-    std::vector<fx2> w(L), o(L);
-    for (int j = 0; j < R1; ++j) {
-      fx2 t[R0];
-      for (int r = 0; r < R0; ++r) t[r] = v[j + r * R1];
-      FxDft<R0, INV>::run(t);
-      for (int r = 0; r < R0; ++r)
-        w[j * R0 + r] = FxSpecial<R0, R1>::output(r) ? fx_multiple<G + 1>(t[r]) : t[r];
-    }
-    for (int j = 0; j < R0; ++j) {
-      fx2 t[R1];
-      for (int r = 0; r < R1; ++r) t[r] = w[j + r * R0];
-      t[0] = fx_shift<G>(t[0]);
-      twiddle<1>(t, j);
-      FxDft<R1, INV>::run(t);
-      for (int r = 0; r < R1; ++r) o[j + r * R0] = t[r];
-    }
-    return o;
+  std::vector<fx2> run(std::vector<fx2> v) const {
+    stages<0, 1>(v);
+    return v;
   }
   // the exponent of a line, as the kernels form it
   static int bound(const std::vector<double>& x) {
     int k = 0;
-    for (int j = 0; j < R1; ++j) {
+    for (int j = 0; j < NB0; ++j) {
       int top = 0;
       float sum = 0.f;
       auto hi = [&](int p, int c) {
@@ -68,33 +64,35 @@ template <int R0, int R1, bool INV> struct Line {
         memcpy(&b, &x[2 * p + c], 8);
         return (int)(b >> 32) & 0x7fffffff;
       };
-      for (int r = 0; r < R0; ++r) top = std::max(top, std::max(hi(j + r * R1, 0), hi(j + r * R1, 1)));
-      for (int r = 0; r < R0; ++r) sum += fx_relative(std::max(hi(j + r * R1, 0), hi(j + r * R1, 1)), top);
+      for (int r = 0; r < R0; ++r) top = std::max(top, std::max(hi(j + r * NB0, 0), hi(j + r * NB0, 1)));
+      for (int r = 0; r < R0; ++r) sum += fx_relative(std::max(hi(j + r * NB0, 0), hi(j + r * NB0, 1)), top);
       k = std::max(k, fx_bound(top, sum));
     }
     return k;
   }
 };
 
-static void fft_double(CD* a, int n, int sign) {
+template <typename F> void fft(std::complex<F>* a, int n, int sign) {
   if (n == 1) return;
   const int r = n % 3 == 0 ? 3 : 2, m = n / r;
-  std::vector<CD> b(n);
+  std::vector<std::complex<F>> b(n);
   for (int i = 0; i < n; ++i) b[(i % r) * m + i / r] = a[i];
-  for (int q = 0; q < r; ++q) fft_double(&b[q * m], m, sign);
+  for (int q = 0; q < r; ++q) fft(&b[q * m], m, sign);
+  static std::map<int, std::vector<CL>> tables;
+  std::vector<CL>& w = tables[n];
+  if (w.empty()) w = roots(n);
   for (int k = 0; k < n; ++k) {
-    CD s = b[k % m];
+    std::complex<F> s = b[k % m];
     for (int q = 1; q < r; ++q) {
-      const LD an = sign * TWO_PI * ((long)q * k % n) / n;
-      s += b[q * m + k % m] * CD((double)cosl(an), (double)sinl(an));
+      const CL c = w[(long)q * k % n];
+      s += b[q * m + k % m] * std::complex<F>((F)c.real(), (F)(sign < 0 ? c.imag() : -c.imag()));
     }
     a[k] = s;
   }
 }
 
-template <int R0, int R1, bool INV> void accuracy() {
-  const Line<R0, R1, INV> line;
-  constexpr int L = R0 * R1;
+template <int L, bool CONTIG, bool INV> void accuracy() {
+  const Line<L, CONTIG, INV> line;
   const auto W = roots(L);
   for (int kind = 0; kind < 5; ++kind) {
     std::mt19937_64 g(5 + kind);
@@ -120,7 +118,7 @@ template <int R0, int R1, bool INV> void accuracy() {
       const auto o = line.run(v);
       std::vector<CD> d(L);
       for (int p = 0; p < L; ++p) d[p] = CD(x[2 * p], x[2 * p + 1]);
-      fft_double(d.data(), L, INV ? 1 : -1);
+      fft<double>(d.data(), L, INV ? 1 : -1);
       const LD inv = 1.0L / scale;
       for (int p = 0; p < L; ++p) {
         CL s = 0;
@@ -128,69 +126,57 @@ template <int R0, int R1, bool INV> void accuracy() {
           const CL w = W[(long)p * q % L];
           s += CL(x[2 * q], x[2 * q + 1]) * (INV ? std::conj(w) : w);
         }
-        const int e = fx_quantum(k) + line.G;
+        const int e = fx_quantum(k) + line.SHIFT;
         const CL f((double)std::ldexp((double)o[p].x, e), (double)std::ldexp((double)o[p].y, e));
         fix += std::norm((f - s) * inv);
         dbl += std::norm((CL(d[p].real(), d[p].imag()) - s) * inv);
         ref += std::norm(s * inv);
       }
     }
-    std::printf("accuracy %d %d %d %.4Le %.4Le\n", L, (int)INV, kind, std::sqrt(fix / ref), std::sqrt(dbl / ref));
+    std::printf("accuracy %d %d %d %d %.4Le %.4Le\n", L, (int)CONTIG, (int)INV, kind, std::sqrt(fix / ref), std::sqrt(dbl / ref));
   }
 }
 
 // mean error of each output over many lines, in standard errors of that mean
-template <int R0, int R1, bool INV> void bias() {
-  const Line<R0, R1, INV> line;
-  constexpr int L = R0 * R1, NR = 1500;
-  const auto W = roots(L);
+template <int L, bool CONTIG, bool INV> void bias() {
+  const Line<L, CONTIG, INV> line;
+  constexpr int NR = 1500;
   std::mt19937_64 g(9);
   std::vector<LD> sx(L, 0), sy(L, 0);
   LD var = 0;
   for (int it = 0; it < NR; ++it) {
     std::vector<fx2> v(L);
-    for (auto& q : v) q = fx2{((long long)g() >> 2) / L, ((long long)g() >> 2) / L};
+    for (auto& q : v) q = fx2{((long long)g() >> 2) / line.R0, ((long long)g() >> 2) / line.R0};
     const auto o = line.run(v);
-    std::vector<CL> B(L);
-    for (int j = 0; j < R1; ++j)
-      for (int k = 0; k < R0; ++k) {
-        CL s = 0;
-        for (int r = 0; r < R0; ++r) {
-          const CL w = W[r * k % R0 * (L / R0)];
-          s += CL(v[j + r * R1].x, v[j + r * R1].y) * (INV ? std::conj(w) : w);
-        }
-        const CL w = W[j * k % L];
-        B[j * R0 + k] = s * (INV ? std::conj(w) : w) / (LD)(1 << line.G);
-      }
-    for (int j = 0; j < R0; ++j)
-      for (int k = 0; k < R1; ++k) {
-        CL s = 0;
-        for (int r = 0; r < R1; ++r) {
-          const CL w = W[r * k % R1 * (L / R1)];
-          s += B[j + r * R0] * (INV ? std::conj(w) : w);
-        }
-        const CL e = CL(o[j + k * R0].x, o[j + k * R0].y) - s;
-        sx[j + k * R0] += e.real();
-        sy[j + k * R0] += e.imag();
-        var += std::norm(e) / 2;
-      }
+    std::vector<CL> d(L);
+    for (int p = 0; p < L; ++p) d[p] = CL(v[p].x, v[p].y);
+    fft<LD>(d.data(), L, INV ? 1 : -1);
+    for (int p = 0; p < L; ++p) {
+      const CL e = CL(o[p].x, o[p].y) - d[p] / (LD)(1 << line.SHIFT);
+      sx[p] += e.real();
+      sy[p] += e.imag();
+      var += std::norm(e) / 2;
+    }
   }
-  const LD se = std::sqrt(var / ((LD)NR * L) / NR);
+  const LD sd = std::sqrt(var / ((LD)NR * L)), noise = sd / std::sqrt((LD)NR);
   LD worst = 0;
-  for (int p = 0; p < L; ++p) worst = std::max(worst, std::max(std::fabs(sx[p]), std::fabs(sy[p])) / NR / se);
-  std::printf("bias %d %d %.3Lf\n", L, (int)INV, worst);
+  for (int p = 0; p < L; ++p) worst = std::max(worst, std::max(std::fabs(sx[p]), std::fabs(sy[p])) / NR);
+  std::printf("bias %d %d %d %.4Lf %.4Lf %.4Lf\n", L, (int)CONTIG, (int)INV, worst, noise, sd);
 }
 
-template <int L> void both() {
-  constexpr int R0 = fx_radix(L, 0), R1 = L / R0;
-  accuracy<R0, R1, false>();
-  accuracy<R0, R1, true>();
-  bias<R0, R1, false>();
-  bias<R0, R1, true>();
+template <int L, bool CONTIG> void both() {
+  accuracy<L, CONTIG, false>();
+  accuracy<L, CONTIG, true>();
+  bias<L, CONTIG, false>();
+  bias<L, CONTIG, true>();
+}
+template <int L> void plans() {
+  both<L, true>();
+  if constexpr (fx_stages(L, false) != fx_stages(L, true)) both<L, false>();
 }
 
 int main() {
-  both<8>(); both<12>(); both<16>(); both<24>(); both<32>(); both<48>(); both<64>(); both<96>();
-  both<128>(); both<192>(); both<256>(); both<384>(); both<512>(); both<768>();
+  plans<8>(); plans<12>(); plans<16>(); plans<24>(); plans<32>(); plans<48>(); plans<64>(); plans<96>();
+  plans<128>(); plans<192>(); plans<256>(); plans<384>(); plans<512>(); plans<768>();
   return 0;
 }

@@ -41,10 +41,9 @@ bool fft_len_ok(int n) {
 }
 
 // W_L^m = exp(-2 pi i m / L), computed in long double: rounded once to floats,
-// or to the fixed-point words of the FP64 form (the units of its second stage).
+// or to the fixed-point words of the FP64 form.
 cudaError_t upload_twiddles(int L, bool fp32, void** dst) {
   const long double two_pi = 6.283185307179586476925286766559005768L;
-  const int bits = 64 - vk::fx_growth(vk::fx_radix(L, 1));
   std::vector<float2> f((size_t)(fp32 ? L : 0));
   std::vector<vk::fxtw> x((size_t)(fp32 ? 0 : L));
   for (int m = 0; m < L; ++m) {
@@ -52,8 +51,7 @@ cudaError_t upload_twiddles(int L, bool fp32, void** dst) {
     if (fp32) {
       f[m] = make_float2((float)(double)cosl(a), (float)(double)(-sinl(a)));
     } else {
-      vk::fx_words(cosl(a), bits, x[m].ch, x[m].cl);
-      vk::fx_words(-sinl(a), bits, x[m].dh, x[m].dl);
+      x[m] = vk::fx_make_twiddle(m, L, cosl(a), sinl(a));
     }
   }
   const size_t bytes = (size_t)L * (fp32 ? sizeof(float2) : sizeof(vk::fxtw));

@@ -103,7 +103,7 @@ inline int zpass_prefetch_distance(int nt, size_t smem) {
 template <typename R, int L, bool INV, bool XAXIS = false, class Op>
 inline cudaError_t launch_lines(const Op& op, int nouter, const C2<R>* tw, cudaStream_t s) {
   constexpr int NLINES = NLof<R, L, XAXIS, Op>::value;
-  constexpr int NT = cmin(rthreads<R, L, NLINES>(), 384);
+  constexpr int NT = cmin(rthreads<R, L, NLINES>(), sizeof(R) == 8 ? 512 : 384);
   const size_t smem = (size_t)rsmem_elems<R, L, NLINES>() * sizeof(C2<R>);
   constexpr auto kern = k_lines<R, L, INV, NLINES, NT, Op>;
   cudaError_t e = prepare_kernel<kern>(smem);
@@ -189,6 +189,18 @@ inline cudaError_t nle_n(const NleParams<R>& p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int pf = VK_P3F_PREFETCH ? wave_blocks<kern>(P3F<CP>::NT, smem) : 0;
     kern<<<ntiles, P3F<CP>::NT, smem, s>>>(a, p.twM, pf);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  } else if constexpr (sizeof(R) == 8) {
+    TimerScope ts(p.timer, PASS_P3, s);
+    constexpr int CP = zcross_pairs<R, M>();
+    constexpr int NT = p3x_threads<M, CP>();
+    const size_t smem = P3X<M, CP>::BYTES;
+    constexpr auto kern = k_p3x<M, CP, NT>;
+    e = prepare_kernel<kern>(smem);
+    if (e != cudaSuccess) return e;
+    P3Args<R> a{M * M, p.bufB, fsB2, p.bufA, fsA3};
+    kern<<<(M * M + 2 * CP - 1) / (2 * CP), NT, smem, s>>>(a, reinterpret_cast<const fxtw*>(p.twM));
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   } else {

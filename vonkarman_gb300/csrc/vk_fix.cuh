@@ -7,16 +7,17 @@
 // SM), so a transform made of integer additions and multiplications runs
 // several times faster than one made of DFMAs.
 //
-// A transform of L = R0 R1 points takes two stages of in-register DFTs.  A line
-// of doubles z becomes integers trunc(z 2^-Q), where 2^(Q + 62) bounds the sum
-// of |z| over the R0 inputs of every first-stage butterfly, so that no partial
-// sum overflows; the stage twiddles carry a factor 1/R1 (R1 rounded up to a
-// power of two), which makes room for the second stage's growth.  Rounding
-// then happens at the quantum 2^Q of the inputs (amplified by sqrt(L)) and at
-// R1 2^Q between the stages (amplified by sqrt(R1)); the butterfly sums are at
-// most sqrt(R0) ||z||, so the error is below one unit in the last place of a
-// double relative to the line's norm in the worst case, and a few times
-// smaller for lines whose norm is spread out.  An FFT in doubles has the same
+// A transform of L points takes two or three stages of in-register DFTs.  A
+// line of doubles z becomes integers trunc(z 2^-Q), where 2^(Q + 62) bounds the
+// sum of |z| over the inputs of every first-stage butterfly, so that no partial
+// sum overflows; the twiddles of the later stages carry a factor 1/G (a power
+// of two, at least their radix), which makes room for the stage's growth.
+// Rounding then happens at the quantum 2^Q of the inputs (amplified by sqrt(L))
+// and at G 2^Q, G^2 2^Q before the later stages (amplified by the square root
+// of what follows); the butterfly sums are at most sqrt(R0) ||z||, so the error
+// is below one unit in the last place of a double relative to the line's norm
+// in the worst case, and a few times smaller for lines whose norm is spread
+// out.  An FFT in doubles has the same
 // kind of bound with a larger constant (tests/test_fix_cpu.py measures both).
 //
 // This header holds the arithmetic and the radix kernels (natural-order
@@ -71,15 +72,21 @@ VK_FIX_HD fx2 fx_sub(fx2 a, fx2 b) { return fx2{a.x - b.x, a.y - b.y}; }
 template <bool INV> VK_FIX_HD fx2 fx_rot(fx2 a) { return INV ? fx2{-a.y, a.x} : fx2{a.y, -a.x}; }
 VK_FIX_HD fx2 fx_neg(fx2 a) { return fx2{-a.x, -a.y}; }
 
-// Rounding is to nearest even, or compensated to a mean of zero: a bias of a
-// fraction of the quantum, the same in every line, would add up over the N^2
-// lines of a grid.
+// Rounding is to nearest even, or compensated to a mean of zero (short twiddles:
+// within an eighth of a unit): a bias that is the same in every line would add
+// up over the N^2 lines of a grid.
 // a w / 2^64, or a conj(w) / 2^64 for INV, of an |a| < 2^62 (so that the sum of
-// the four cross terms stays inside a word).  Their floors lose 1/2 each, which
-// r0 = 2 returns; the dropped low x low terms are below half a unit and have
-// mean zero.  Twiddles with components 0, 1/2 and 1 take a smaller r0 (FxSpecial).
-template <bool INV> VK_FIX_HD fx2 fx_twiddle(fx2 a, fxtw w, int r0) {
+// the four cross terms stays inside a word).  The four floors lose 1/2 each,
+// which r0 = 2 returns; the dropped low x low terms are below half a unit and
+// have mean zero.  Quarter turns have one component of zero, whose products
+// lose nothing, and take r0 = 1; w = 1 takes r0 = 0, and its products are exact
+// where a is a multiple of the factor 2^growth in the table's units (the stage
+// before rounds the outputs that meet it so: all inputs of one butterfly of a
+// line do).  The table holds r0 in the lowest two bits of cl, and no other low
+// word of zero.
+template <bool INV> VK_FIX_HD fx2 fx_twiddle(fx2 a, fxtw w) {
   const fxsplit x = fx_split(a.x), y = fx_split(a.y);
+  const int r0 = w.cl & 3;
   const int nh = -w.dh, nl = -w.dl;
   const int ph = INV ? w.dh : nh, pl = INV ? w.dl : nl;   // y's factor in the real part
   const int qh = INV ? nh : w.dh, ql = INV ? nl : w.dl;   // x's factor in the imaginary part
@@ -89,59 +96,78 @@ template <bool INV> VK_FIX_HD fx2 fx_twiddle(fx2 a, fxtw w, int r0) {
   s = fx_madhi(x.l, qh, fx_madhi(x.h, ql, s));
   return fx2{fx_wide(x.h, w.ch) + fx_wide(y.h, ph) + (long long)t, fx_wide(y.h, w.ch) + fx_wide(x.h, qh) + (long long)s};
 }
-// v + a value that makes the following floor to a multiple of 2^B round to nearest even
+// v plus what makes a floor to a multiple of 2^B round to nearest even
 template <int B> VK_FIX_HD long long fx_bump(long long v) {
   return v + (long long)((1 << (B - 1)) - 1 + ((int)((unsigned)v >> B) & 1));
 }
-// a / 2^B (the untwiddled input beside twiddled ones)
-template <int B> VK_FIX_HD fx2 fx_shift(fx2 a) { return fx2{fx_bump<B>(a.x) >> B, fx_bump<B>(a.y) >> B}; }
 // the nearest multiple of 2^B
 template <int B> VK_FIX_HD fx2 fx_multiple(fx2 a) {
   return fx2{fx_bump<B>(a.x) & -(1ll << B), fx_bump<B>(a.y) & -(1ll << B)};
 }
-// Plans: two stages with 2^b butterflies in the first.  Short lines take small
-// radices (a small grid is bound by the latency of one thread's work), long
-// ones the largest that registers hold.
+// a / 2^B (the untwiddled input beside twiddled ones)
+template <int B> VK_FIX_HD fx2 fx_shift(fx2 a) { return fx2{fx_bump<B>(a.x) >> B, fx_bump<B>(a.y) >> B}; }
+// Plans.  Contiguous lines (z passes): two stages with 2^b butterflies in the
+// first, so that a line's threads share a warp; short lines take small radices
+// (a small grid is bound by the latency of one thread's work), long ones the
+// largest that registers hold.  Interleaved lines (x and y passes): three
+// stages of radices up to 8 from 256 to 512 points, which need half the registers
+// and let twice the warps be resident.
 VK_FIX_HD constexpr int fx_radix0(int L) {
   return L == 8 ? 2 : L == 12 ? 3 : L == 16 ? 4 : L == 24 ? 6 : L == 32 ? 4 : L == 48 ? 6 : L == 64 ? 8 : L == 96 ? 12
        : L == 128 ? 16 : L == 192 ? 12 : L == 256 ? 16 : L == 384 ? 24 : L == 512 ? 16 : L == 768 ? 24 : 0;
 }
 VK_FIX_HD constexpr bool fx_supported(int L) { return fx_radix0(L) > 0; }
-VK_FIX_HD constexpr int fx_radix(int L, int s) { return s == 0 ? fx_radix0(L) : L / fx_radix0(L); }
-// log2 of the factor that the twiddles of a second stage of radix r1 divide by;
+VK_FIX_HD constexpr int fx_stages(int L, bool contig) { return !contig && L >= 256 && L <= 512 ? 3 : 2; }
+VK_FIX_HD constexpr int fx_radix(int L, int s, bool contig) {
+  return fx_stages(L, contig) == 2 ? (s == 0 ? fx_radix0(L) : L / fx_radix0(L))
+       : s < 2 ? 8 : L / 64;
+}
+// log2 of the factor that the twiddles of a later stage of radix r divide by;
 // their components are held in units of 2^-(64 - growth), which makes
 // fx_twiddle's a w / 2^64 the scaled product
-VK_FIX_HD constexpr int fx_growth(int r1) { return r1 <= 4 ? 2 : r1 <= 8 ? 3 : r1 <= 16 ? 4 : 5; }
-// Short twiddles of a two-stage plan: input r of second-stage butterfly j (output
-// j of first-stage butterfly r) is multiplied by W_L^(r j).  Components of 0, 1/2
-// and 1 (multiples of a quarter and a twelfth turn) have a low word of zero, so
-// they lose fewer floors; the first stage rounds the outputs that meet one to
-// multiples of 2^(growth + 1), which makes their products exact, and r0 counts
-// the floors that are left.
-template <int R0, int R1> struct FxSpecial {
-  static constexpr int Q4 = R0 * R1 / 4;
-  static constexpr int Q = R0 % 3 == 0 ? R0 * R1 / 12 : Q4;
-  static VK_FIX_HD constexpr bool at(int r, int j) { return (r * j) % Q == 0; }
-  static VK_FIX_HD constexpr bool output(int j) {   // some input r > 0 of butterfly j
-    for (int r = 1; r < R1; ++r)
-      if (at(r, j)) return true;
-    return false;
+VK_FIX_HD constexpr int fx_growth(int r) { return r <= 4 ? 2 : r <= 8 ? 3 : r <= 16 ? 4 : 5; }
+// sum of the growths of a plan's stages: the outputs' exponent above the quantum
+VK_FIX_HD constexpr int fx_total_growth(int L, bool contig) {
+  int g = 0;
+  for (int s = 1; s < fx_stages(L, contig); ++s) g += fx_growth(fx_radix(L, s, contig));
+  return g;
+}
+// W_L^m = c - i s (cosine and sine of 2 pi m / L) in units of 2^-62 (host)
+inline fxtw fx_make_twiddle(int m, int L, long double c, long double s) {
+  const auto words = [](long double v, int& h, int& l) {
+    v *= 4611686018427387904.0L;
+    const long long q = (long long)(v < 0 ? v - 0.5L : v + 0.5L);
+    l = (int)(unsigned)(unsigned long long)q;
+    h = (int)((q - (long long)l) >> 32);
+  };
+  fxtw w;
+  words(c, w.ch, w.cl);
+  words(-s, w.dh, w.dl);
+  if (m % L == 0) {
+    w.cl = w.dl = 0;
+  } else if (4 * (m % L) % L == 0) {   // (-1, 0) or (0, +-1)
+    w.cl = 1;
+    w.dl = 0;
+  } else {
+    w.cl = (w.cl & ~3) | 2;
+    if (w.dl == 0) w.dl = 1;
   }
-  // r0 of fx_twiddle: j is known at run time only
-  template <int R> static VK_FIX_HD int round0(int j) {
-    int v = j == 0 ? 0 : 2;
-#pragma unroll
-    for (int i = 1; i < R0; ++i)
-      if (at(R, i) && j == i) v = (R * i) % Q4 == 0 ? 0 : 1;
-    return v;
-  }
-};
-// the words of a twiddle component v, |v| <= 1, in units of 2^-bits (host)
-inline void fx_words(long double v, int bits, int& h, int& l) {
-  const long double s = v * (long double)(1ull << bits);
-  const long long q = (long long)(s < 0 ? s - 0.5L : s + 0.5L);
-  l = (int)(unsigned)(unsigned long long)q;
-  h = (int)((q - (long long)l) >> 32);
+  return w;
+}
+// the table's twiddle in the units of a stage of growth g
+VK_FIX_HD fxtw fx_stage_twiddle(fxtw w, int g) {
+  const auto shift = [g](int& h, int& l) {
+    const long long v = ((long long)h * 4294967296ll + l) >> (g - 2);
+    l = (int)(unsigned)(unsigned long long)v;
+    h = (int)((v - (long long)l) >> 32);
+  };
+  const int r0 = w.cl & 3;
+  w.cl &= ~3;
+  shift(w.ch, w.cl);
+  shift(w.dh, w.dl);
+  w.cl = (w.cl & ~3) | r0;
+  if (r0 == 2 && w.dl == 0) w.dl = 1;
+  return w;
 }
 
 // Constants k in (0, 1/2) in units of 2^-64: 1 - cos(2 pi m / 32), sin(2 pi m / 32)

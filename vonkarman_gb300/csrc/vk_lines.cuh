@@ -61,21 +61,21 @@ __host__ __device__ constexpr int rplan_radix_f(int L, int s) {
 __host__ __device__ constexpr int rplan_radix_fc(int L, int s) {
   return L == 384 ? (s == 0 ? 16 : 24) : rplan_radix_f(L, s);
 }
-// FP64 lines run in fixed point with the plans of vk_fix.cuh, the same for both
-// thread maps.
+// FP64 lines run in fixed point with the plans of vk_fix.cuh.
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rstages(int L) {
-  return sizeof(R) == 4 ? rplan_stages_f(L) : fx_supported(L) ? 2 : -1;
+  return sizeof(R) == 4 ? rplan_stages_f(L) : fx_supported(L) ? fx_stages(L, CONTIG) : -1;
 }
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rradix(int L, int s) {
-  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : fx_radix(L, s);
+  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : fx_radix(L, s, CONTIG);
 }
-// threads of a CTA: one butterfly per thread in the widest stage (FP64 above 96
-// points: in the first stage, and a line of the second)
+// threads of a CTA: one butterfly per thread in the widest stage (FP64 plans of
+// two stages above 96 points: in the first stage, and a line of the second; of
+// three stages: in all but the last)
 template <typename R, int L, int NLINES, bool CONTIG = false, int S = 0>
 __host__ __device__ constexpr int rthreads() {
   if constexpr (sizeof(R) == 8) {
-    constexpr int nb0 = L / fx_radix(L, 0), nb1 = L / fx_radix(L, 1);
-    return round32(L <= 96 ? cmax(nb0, nb1) * NLINES : cmax(nb0 * NLINES, CONTIG ? nb1 : 0));
+    constexpr int nb0 = L / fx_radix(L, 0, CONTIG), nb1 = L / fx_radix(L, 1, CONTIG);
+    return round32(L <= 96 || fx_stages(L, CONTIG) == 3 ? cmax(nb0, nb1) * NLINES : cmax(nb0 * NLINES, CONTIG ? nb1 : 0));
   } else if constexpr (S >= rstages<R, CONTIG>(L)) {
     return 32;
   } else {
@@ -126,6 +126,13 @@ __device__ __forceinline__ int ridx(int pos, int l) {
 // to 168 registers per SM.
 template <int L, int NT>
 __host__ __device__ constexpr int fx_min_blocks() { return L >= 512 ? 1 : cmax(1, 384 / NT); }
+#ifndef FX3T
+#define FX3T 1152
+#endif
+template <int L, int NT>
+__host__ __device__ constexpr int fx_lines_min_blocks() {
+  return fx_stages(L, false) == 3 ? cmax(1, FX3T / NT) : L <= 192 ? cmax(1, 512 / NT) : fx_min_blocks<L, NT>();
+}
 
 // Minimum resident CTAs per SM requested from the compiler (caps registers):
 // 24 warps per SM for the strided passes where the plan allows it; one or two
@@ -134,7 +141,7 @@ __host__ __device__ constexpr int fx_min_blocks() { return L >= 512 ? 1 : cmax(1
 template <typename R, int L, int NT, bool EPI = false>
 __host__ __device__ constexpr int lines_min_blocks() {
   if constexpr (sizeof(R) == 8) {
-    return fx_min_blocks<L, NT>();
+    return fx_lines_min_blocks<L, NT>();
   } else {
     return L >= 768 ? (EPI ? 1 : 2) : EPI ? cmax(1, 512 / NT) : L >= 512 ? 2 : L >= 384 ? (NT >= 384 ? 2 : 3)
          : NT < 128 ? 4 : cmax(1, 768 / NT);
@@ -316,16 +323,26 @@ __device__ __forceinline__ double fx_to_double(long long v, int q20) {
   return __hiloint2double(h != 0 ? h + q20 : 0, __double2loint(d));
 }
 
+// State of a line between the stages: output exponent and FxCode.
+struct FxState { int q, code; };
+
 template <int L, int NT, int NLINES, class MAP>
 __host__ __device__ constexpr int fx_round_lines() {   // lines per stage-1 round (contiguous lines)
-  return NT / (L / fx_radix(L, 1)) < NLINES ? NT / (L / fx_radix(L, 1)) : NLINES;
+  return cmin(NT / (L / fx_radix(L, 1, true)), NLINES);
 }
 
 template <int L, bool INV, int NT, int NLINES, class MAP, bool SL, int Z0, int Z1>
 struct FxLines {
-  static constexpr int R0 = fx_radix(L, 0), NB0 = L / R0, G0 = NB0 * NLINES;
-  static constexpr int R1 = fx_radix(L, 1), NB1 = L / R1, G1 = NB1 * NLINES;
+  static constexpr bool CT = MAP::CONTIG;
+  static constexpr int ST = fx_stages(L, CT);
+  static constexpr int R0 = fx_radix(L, 0, CT), NB0 = L / R0, G0 = NB0 * NLINES;
+  // the last stage: radix, butterflies, growth, and its twiddles' place in the table
+  static constexpr int R1 = fx_radix(L, ST - 1, CT), NB1 = L / R1, G1 = NB1 * NLINES;
   static constexpr int GR = fx_growth(R1);
+  static constexpr int TW1 = twtab_off<double, CT>(L, ST - 1);
+  static constexpr int TG = fx_total_growth(L, CT);
+  // growth of the stage after the first
+  static constexpr int GN = fx_growth(fx_radix(L, 1, CT));
   static constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
   static constexpr int NW0 = (G0 + 31) / 32;
   static constexpr int CODE_SHIFT = 24;   // stored line state: exponent + (code << 24)
@@ -350,28 +367,18 @@ struct FxLines {
     return m;
   }
 
-  // the butterfly's outputs as doubles, stored
-  template <int RAD, class STF>
-  __device__ __forceinline__ static void emit(const fx2* v, int l, int base, int ns, int q, int code, const STF& st) {
-    double2 d[RAD];
-    const int q20 = q << 20;
-#pragma unroll
-    for (int r = 0; r < RAD; ++r) d[r] = make_double2(fx_to_double(v[r].x, q20), fx_to_double(v[r].y, q20));
-    if (code != FX_PLAIN) {
-      const double f = fx_code_factor(code);
-#pragma unroll
-      for (int r = 0; r < RAD; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
-    }
-#pragma unroll
-    for (int r = 0; r < RAD; ++r) st(l, base + r * ns, d[r]);
+  using State = FxState;
+  __device__ __forceinline__ static int pack_state(int q, int code) { return q + (code << CODE_SHIFT); }
+  __device__ __forceinline__ static State unpack_state(int s) {
+    const int code = (s + (1 << (CODE_SHIFT - 1))) >> CODE_SHIFT;
+    return State{s - (code << CODE_SHIFT), code};
   }
 
-  // fill(l, j, d): the inputs at positions j + r NB0 of line l (those of ZM excepted)
-  template <class FILL, class STF>
-  __device__ __forceinline__ static void run(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, const STF& st,
-                                             int xe) {
-    __shared__ int part[MAP::CONTIG ? 1 : NW0 * NLINES];
-    __shared__ int line_s[MAP::CONTIG ? NLINES : 1];
+  // Stage 0 from doubles.  fill(l, j, d): the inputs at positions j + r NB0 of
+  // line l (those of ZM excepted).  The state of the thread's line is returned
+  // (interleaved: valid in every thread; contiguous: also in line_s[l]).
+  template <class FILL>
+  __device__ __forceinline__ static State front(fx2* xb, const FILL& fill, int* part, int* line_s, int xe) {
     const int g = threadIdx.x;
     const int l0 = MAP::template line<NB0>(g), j0 = MAP::template bfly<NB0>(g);
     const bool act = G0 == NT || g < G0;
@@ -404,9 +411,9 @@ struct FxLines {
         for (int r = 0; r < R0; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
       }
     }
-    int q = fx_quantum(k) + GR + xe;
-    fx2 v[R0];
+    const int q = fx_quantum(k) + TG + xe;
     if (act) {
+      fx2 v[R0];
 #pragma unroll
       for (int r = 0; r < R0; ++r) {
         if ((ZM >> r) & 1u) {
@@ -416,62 +423,149 @@ struct FxLines {
           v[r].y = fx_from_double(__double2hiint(d[r].y), __double2loint(d[r].y), k);
         }
       }
-      FxDft<R0, INV>::run(v);
+      if (MAP::CONTIG && j0 == 0) line_s[l0] = pack_state(q, code);
+      first_dft(v, [&](int p, fx2 z) { xb[MAP::template idx<0>(p, l0)] = z; }, j0);
     }
+    return State{q, code};
+  }
+  // first-stage butterfly j: put(position, value) into the exchange
+  template <class PUT>
+  __device__ __forceinline__ static void first_dft(fx2* v, const PUT& put, int j) {
+    FxDft<R0, INV>::run(v);
+    sfor<R0>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (r == 0) v[r] = fx_multiple<GN>(v[r]);
+      put(j * R0 + r, v[r]);
+    });
+  }
+  // twiddles and DFT of a later stage's butterfly: twiddle index k of ns
+  template <int RAD, int OFF>
+  __device__ __forceinline__ static void later_dft(fx2* u, const fxtw* __restrict__ tw, int k, int ns) {
+    u[0] = fx_shift<fx_growth(RAD)>(u[0]);
+#pragma unroll
+    for (int r = 1; r < RAD; ++r) u[r] = fx_twiddle<INV>(u[r], tw[OFF + (r - 1) * ns + k]);
+    FxDft<RAD, INV>::run(u);
+  }
+  __device__ __forceinline__ static void last_dft(fx2* u, const fxtw* __restrict__ tw, int j) {
+    later_dft<R1, TW1>(u, tw, j, NB1);
+  }
+  // The middle stage of a three-stage plan, in place (begins and ends with the
+  // exchange complete).
+  __device__ __forceinline__ static void middle(fx2* xb, const fxtw* __restrict__ tw) {
+    constexpr int RM = fx_radix(L, 1, CT), NBM = L / RM, GM = NBM * NLINES;
+    static_assert(GM <= NT, "one butterfly per thread");
+    const int g = threadIdx.x;
+    const int l = MAP::template line<NBM>(g), j = MAP::template bfly<NBM>(g);
+    const bool act = GM == NT || g < GM;
+    fx2 u[RM];
     if (act) {
-      if (MAP::CONTIG && j0 == 0) line_s[l0] = q + (code << CODE_SHIFT);
-      sfor<R0>([&](auto rc) {
-        constexpr int r = decltype(rc)::value;
-        if constexpr (FxSpecial<R0, R1>::output(r)) v[r] = fx_multiple<GR + 1>(v[r]);
-        xb[MAP::template idx<0>(j0 * R0 + r, l0)] = v[r];
-      });
+      __builtin_assume(j >= 0 && j < NBM);
+      __builtin_assume(l >= 0 && l < NLINES);
+#pragma unroll
+      for (int r = 0; r < RM; ++r) u[r] = xb[MAP::template idx<0>(j + r * NBM, l)];
     }
     __syncthreads();
-    // rounds of stage 1: whole lines (contiguous) or butterflies of all lines
+    if (act) {
+      const int k = j % R0;
+      later_dft<RM, 0>(u, tw, k, R0);
+      u[0] = fx_multiple<GR>(u[0]);
+#pragma unroll
+      for (int r = 0; r < RM; ++r) xb[MAP::template idx<0>((j - k) * RM + k + r * R0, l)] = u[r];
+    }
+    __syncthreads();
+  }
+
+  // The last stage, in rounds (whole lines, or butterflies of all lines); the
+  // exchange is complete.  em(u, l, j, state) takes a butterfly's outputs
+  // (positions j + r NB1).
+  template <class EM>
+  __device__ __forceinline__ static void back(const fx2* xb, const fxtw* __restrict__ tw, const int* line_s, State st0,
+                                              const EM& em) {
     constexpr int RL = MAP::CONTIG ? fx_round_lines<L, NT, NLINES, MAP>() : NLINES;
     constexpr int PER = MAP::CONTIG ? RL * NB1 : NT;                 // butterflies per round
     constexpr int ROUNDS = MAP::CONTIG ? (NLINES + RL - 1) / RL : (G1 + NT - 1) / NT;
     static_assert(RL >= 1, "a round holds a line");
+    const int g = threadIdx.x;
 #pragma unroll 1
     for (int i = 0; i < ROUNDS; ++i) {
       const int gi = i * PER + g;
       const int l = MAP::template line<NB1>(gi), j = MAP::template bfly<NB1>(gi);
-      const bool act1 = (PER == NT || g < PER) && (G1 % PER == 0 || gi < G1);
+      const bool act = (PER == NT || g < PER) && (G1 % PER == 0 || gi < G1);
       fx2 u[R1];
-      int qs = q, cs = code;
-      if (act1) {
+      State st = st0;
+      if (act) {
         __builtin_assume(j >= 0 && j < NB1);
         __builtin_assume(l >= 0 && l < NLINES);
-        if (MAP::CONTIG) {
-          const int s = line_s[l];
-          cs = (s + (1 << (CODE_SHIFT - 1))) >> CODE_SHIFT;
-          qs = s - (cs << CODE_SHIFT);
-        }
+        if (MAP::CONTIG) st = unpack_state(line_s[l]);
 #pragma unroll
         for (int r = 0; r < R1; ++r) u[r] = xb[MAP::template idx<0>(j + r * NB1, l)];
       }
       if constexpr (SL) __syncthreads();
-      if (act1) {
-        u[0] = fx_shift<GR>(u[0]);
-        sfor<R1 - 1>([&](auto rc) {
-          constexpr int r = decltype(rc)::value + 1;
-          u[r] = fx_twiddle<INV>(u[r], tw[(r - 1) * R0 + j], FxSpecial<R0, R1>::template round0<r>(j));
-        });
-        FxDft<R1, INV>::run(u);
-        emit<R1>(u, l, j, R0, qs, cs, st);
+      if (act) {
+        last_dft(u, tw, j);
+        em(u, l, j, st);
       }
     }
+  }
+
+  // The last stage of nl contiguous lines, line l at xs + l ls, written back in place
+  // or to lines that no thread reads: em(u, l, j).
+  template <class EM>
+  __device__ __forceinline__ static void back_rt(const fx2* xs, int ls, int nl, const fxtw* __restrict__ tw,
+                                                 const EM& em) {
+    constexpr int RL = fx_round_lines<L, NT, NLINES, MAP>();
+    const int lr = threadIdx.x / NB1, j = threadIdx.x % NB1;
+    __builtin_assume(j >= 0 && j < NB1);
+#pragma unroll 1
+    for (int l0 = 0; l0 < nl; l0 += RL) {
+      const int l = l0 + lr;
+      const bool act = lr < RL && l < nl;
+      fx2 u[R1];
+      if (act) {
+#pragma unroll
+        for (int r = 0; r < R1; ++r) u[r] = xs[l * ls + zi<double>(j + r * NB1)];
+      }
+      __syncthreads();
+      if (act) {
+        last_dft(u, tw, j);
+        em(u, l, j);
+      }
+    }
+  }
+
+  // The whole transform from doubles to doubles: st(l, p, v).
+  template <class FILL, class STF>
+  __device__ __forceinline__ static void run(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, const STF& st,
+                                             int xe) {
+    __shared__ int part[MAP::CONTIG ? 1 : NW0 * NLINES];
+    __shared__ int line_s[MAP::CONTIG ? NLINES : 1];
+    const State s0 = front(xb, fill, part, line_s, xe);
+    __syncthreads();
+    if constexpr (ST == 3) middle(xb, tw);
+    back(xb, tw, line_s, s0, [&](const fx2* u, int l, int j, State s) {
+      double2 d[R1];
+      const int q20 = s.q << 20;
+#pragma unroll
+      for (int r = 0; r < R1; ++r) d[r] = make_double2(fx_to_double(u[r].x, q20), fx_to_double(u[r].y, q20));
+      if (s.code != FX_PLAIN) {
+        const double f = fx_code_factor(s.code);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
+      }
+#pragma unroll
+      for (int r = 0; r < R1; ++r) st(l, j + r * NB1, d[r]);
+    });
   }
 };
 
 // fill functor of FxLines from ld / pp: all loads of a chunk are issued before
 // any arithmetic on them (chunks of 256 bytes per thread where the raw inputs
 // are wider than one complex value)
-template <int L, int Z0, int Z1, class LD, class PP> struct FxFill {
+template <int L, bool CONTIG, int Z0, int Z1, class LD, class PP> struct FxFill {
   const LD& ld;
   const PP& pp;
   __device__ __forceinline__ void operator()(int l, int j, double2* d) const {
-    constexpr int R0 = fx_radix(L, 0), NB0 = L / R0;
+    constexpr int R0 = fx_radix(L, 0, CONTIG), NB0 = L / R0;
     constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
     using Raw = decltype(ld(0, 0));
     constexpr int CH = sizeof(Raw) > sizeof(double2) ? cmin(R0, (int)(256 / sizeof(Raw))) : R0;
@@ -502,7 +596,7 @@ __device__ __forceinline__ void fft_lines(C2<R>* xb, const C2<R>* __restrict__ t
   if constexpr (sizeof(R) == 8) {
     static_assert(TT, "per-stage tables");
     FxLines<L, INV, NT, NLINES, MAP, SL, Z0, Z1>::run(reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw),
-                                                      FxFill<L, Z0, Z1, LD, PP>{ld, pp}, st, 0);
+                                                      FxFill<L, MAP::CONTIG, Z0, Z1, LD, PP>{ld, pp}, st, 0);
   } else {
     RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
   }
@@ -525,7 +619,12 @@ __device__ __forceinline__ void load_twtab(C2<R>* tab, const C2<R>* __restrict__
     const int tws = L / (ns * rad), off = twtab_off<R, CONTIG>(L, S);
     for (int i = threadIdx.x; i < (rad - 1) * ns; i += NT) {
       const int r = i / ns + 1, k = i - (r - 1) * ns;
-      tab[off + i] = tw[r * k * tws];
+      if constexpr (sizeof(R) == 8) {   // in the units of the stage
+        reinterpret_cast<fxtw*>(tab)[off + i] =
+            fx_stage_twiddle(reinterpret_cast<const fxtw*>(tw)[r * k * tws], fx_growth(rad));
+      } else {
+        tab[off + i] = tw[r * k * tws];
+      }
     }
   }
 }
@@ -597,7 +696,7 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
         if (kd != K) return;   // uniform over the CTA
         const auto ld = [&](int, int p) { return op.template load<K>(f, outer, z, p); };
         const auto pp = [&](int, int p, const auto& raw) { return op.template prep<K>(f, outer, z, p, raw); };
-        FxFill<L, Z0, Z1, decltype(ld), decltype(pp)>{ld, pp}(l, j, d);
+        FxFill<L, false, Z0, Z1, decltype(ld), decltype(pp)>{ld, pp}(l, j, d);
       });
     };
     int xe = 0;
@@ -713,8 +812,8 @@ k_p5(P5Args<R> a, const C2<R>* __restrict__ tw) {
   }
   __syncthreads();
   if constexpr (sizeof(R) == 8) {
-    // two modes per iteration, so that the loads of both are in flight together
-    constexpr int EM = 2;
+    // two modes per iteration with 128 threads, so that the loads of both are in flight together
+    constexpr int EM = NT > 128 ? 1 : 2;
     const int l = threadIdx.x % NLINES;
     const int lam = blockIdx.x * NLINES + l;
     const bool line_ok = lam < a.nlines;
@@ -944,8 +1043,7 @@ __host__ __device__ constexpr bool z_row_unpack() {
 }
 
 template <typename R, int M, int CP, int NT>
-__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? fx_min_blocks<M, NT>()
-                                      : M >= 768 ? (p3_inplace<CP>() ? 3 : 1) : cmax(1, 512 / NT))
+__global__ void __launch_bounds__(NT, M >= 768 ? (p3_inplace<CP>() ? 3 : 1) : cmax(1, 512 / NT))
 k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int N = 2 * M / 3;
   constexpr int H = N / 2 + 1;
@@ -1024,6 +1122,262 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
     const int pr = e / (3 * H);
     C2<R> X, Y;
     zunpack<R>(A + (t * CP + pr) * LP, M, k, X, Y);
+    const int ca = col0 + 2 * pr, cb = ca + 1;
+    if (t == 0) {
+      if (ca < a.ncols) {
+        a.out[(size_t)ca * H + k] = X;
+        a.out[a.fsout + (size_t)ca * H + k] = Y;
+      }
+    } else if (t == 1) {
+      if (ca < a.ncols) a.out[2 * a.fsout + (size_t)ca * H + k] = X;
+      if (cb < a.ncols) a.out[2 * a.fsout + (size_t)cb * H + k] = Y;
+    } else {
+      if (cb < a.ncols) {
+        a.out[(size_t)cb * H + k] = X;
+        a.out[a.fsout + (size_t)cb * H + k] = Y;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// P3 in the FP64 form: k_p3's lines, with the fields, their cross products and
+// the spectra as integers from the first stage of the inverse to the unpacked
+// modes (doubles in between would cost 12 conversions and FP64 operations per
+// position on the pipe that is scarce).
+//
+// The last inverse stage leaves the fields in place with each line's exponent
+// and, per real field, the OR of the high words' magnitudes.  Those give each
+// column the shifts that bring u to 62 and omega to 61 bits; a product keeps the
+// upper 59 of its 123 bits (two products and their four floors per component,
+// with their mean returned, as in fx_twiddle).  The forward first stage shifts
+// its line right by what its largest butterfly needs (rounded), at most 6 bits.
+//
+// The inverse runs as a forward transform of lines with real and imaginary
+// parts exchanged, so that both directions share the code of the second stage:
+// CTAs of one SM are in different phases, and their instructions have to fit
+// its instruction cache.  Lines l = t 2CP + c (t: packed pair, c: column); the
+// forward lines (t, pair) use line t 2CP + 2 pair and exchange through the next
+// one, both of which belong to that pair.
+// ---------------------------------------------------------------------------
+struct FxColumn {       // per column: left shifts (negative: right) of the lines' fields, exponent of the products
+  int s1, s2u, s2w, s3;
+  int e, code;
+};
+__device__ __forceinline__ long long fx_shl(long long v, int s) {   // v 2^s, rounded for s < 0
+  return s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
+}
+// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split)
+__device__ __forceinline__ long long fx_det(fxsplit a, fxsplit b, fxsplit c, fxsplit d) {
+  const int nh = -d.h, nl = -d.l;
+  int t = fx_madhi(a.l, b.h, fx_madhi(a.h, b.l, 2));
+  t = fx_madhi(c.l, nh, fx_madhi(c.h, nl, t));
+  return fx_wide(a.h, b.h) + fx_wide(c.h, nh) + (long long)t;
+}
+// bits of a field whose high words' magnitudes OR to m, line exponent q
+__device__ __forceinline__ int fx_field_bits(int q, int m) { return q + 64 - __clz(m); }
+
+template <int M, int CP> __host__ __device__ constexpr int p3x_threads() {
+  return rthreads<double, M, 6 * CP, true>();
+}
+
+// Dynamic shared memory of k_p3x (one array, so that the second stage, a
+// function of its own, addresses it as shared memory).
+template <int M, int CP> struct P3X {
+  static constexpr int LP = zpad_len<double>(M);
+  static constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
+  static constexpr int TW = NI * LP;                                 // in units of fx2
+  static constexpr int INTS = TW + twtab_elems<double, true>(M);
+  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn);
+  __device__ __forceinline__ static fx2* lines() {
+    extern __shared__ __align__(16) unsigned char vk_smem[];
+    return reinterpret_cast<fx2*>(vk_smem);
+  }
+  __device__ __forceinline__ static fxtw* twiddles() { return reinterpret_cast<fxtw*>(lines() + TW); }
+  __device__ __forceinline__ static int* line_s() { return reinterpret_cast<int*>(lines() + INTS); }
+  __device__ __forceinline__ static int* field_m() { return line_s() + NI; }
+  __device__ __forceinline__ static FxColumn* cols() { return reinterpret_cast<FxColumn*>(field_m() + 2 * NI); }
+};
+// Second stage of nl lines at stride ls, from xs to ds (element offsets), with
+// the fields' magnitudes where they are wanted.  Not inlined: both directions
+// run this code.
+template <int M, int CP, int NT>
+__device__ __forceinline__ void p3x_second(int xs, int ds, int ls, int nl, bool maxima) {
+  using P = P3X<M, CP>;
+  using Inv = FxLines<M, false, NT, P::NI, MapContig<double, M, P::NI>, true, 0, 0>;
+  Inv::back_rt(P::lines() + xs, ls, nl, P::twiddles(), [&](const fx2* u, int l, int j) {
+    fx2* dst = P::lines() + ds + l * ls;
+    int mx = 0, my = 0;
+#pragma unroll
+    for (int r = 0; r < Inv::R1; ++r) {
+      const int hx = (int)(u[r].x >> 32), hy = (int)(u[r].y >> 32);
+      mx |= hx ^ (hx >> 31);
+      my |= hy ^ (hy >> 31);
+      dst[zi<double>(j + r * Inv::NB1)] = u[r];
+    }
+    if (maxima) {
+      atomicOr(P::field_m() + 2 * l, my);   // (parts exchanged)
+      atomicOr(P::field_m() + 2 * l + 1, mx);
+    }
+  });
+}
+
+template <int M, int CP, int NT>
+__global__ void __launch_bounds__(NT, fx_min_blocks<M, NT>())
+k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
+  constexpr int N = 2 * M / 3;
+  constexpr int H = N / 2 + 1;
+  constexpr int LP = zpad_len<double>(M);
+  constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
+  using Inv = FxLines<M, false, NT, NI, MapContig<double, M, NI>, true, H, M - H + 1>;
+  using Fwd = FxLines<M, false, NT, NF, MapContig<double, M, NF>, true, 0, 0>;
+  using State = FxState;
+  using P = P3X<M, CP>;
+  fx2* A = P::lines();
+  int* line_s = P::line_s();
+  const int* field_m = P::field_m();
+  FxColumn* cols = P::cols();
+  load_twtab<double, M, true, NT>(reinterpret_cast<double2*>(P::twiddles()), reinterpret_cast<const double2*>(tw));
+  const int col0 = blockIdx.x * NC;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < 2 * NI; i += NT) P::field_m()[i] = 0;
+  {
+      // inverse: packed pairs, positions H .. M - H are the z zero-padding
+      const auto ld = [&](int l, int p) -> C2x2<double> {
+        const int t = l / NC;
+        const int col = col0 + l % NC;
+        const bool lo = p < H;
+        C2x2<double> r{};
+        if (col < a.ncols && (lo || p > M - H)) {
+          const double2* src = a.in + (size_t)col * H + (lo ? p : M - p);
+          r.a = src[(size_t)(2 * t) * a.fsin];
+          r.b = src[(size_t)(2 * t + 1) * a.fsin];
+        }
+        return r;
+      };
+      // Z = X + i Y with the Hermitian extension, parts exchanged
+      const auto pp = [&](int, int p, const C2x2<double>& r) -> double2 {
+        if (p == 0) return make_double2(r.b.x, r.a.x);
+        return p < H ? make_double2(r.a.y + r.b.x, r.a.x - r.b.y) : make_double2(r.b.x - r.a.y, r.a.x + r.b.y);
+      };
+      Inv::front(A, FxFill<M, true, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, nullptr, line_s, 0);
+  }
+  __syncthreads();
+  p3x_second<M, CP, NT>(0, 0, LP, NI, true);
+  __syncthreads();
+    if (tid < NC) {   // the column's shifts
+      int q[3], code[3];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const State s = Inv::unpack_state(line_s[t * NC + tid]);
+        code[t] = s.code;
+        q[t] = s.q + (s.code == FX_TINY ? -FX_RANGE : s.code == FX_HUGE ? FX_RANGE : 0);
+      }
+      const int* m1 = field_m + 2 * tid;
+      const int* m2 = m1 + 2 * NC;
+      const int* m3 = m2 + 2 * NC;
+      constexpr int NONE = -(1 << 20);
+      int bu = code[0] == FX_ZERO ? NONE : fx_field_bits(q[0], m1[0] | m1[1]);
+      int bw = code[2] == FX_ZERO ? NONE : fx_field_bits(q[2], m3[0] | m3[1]);
+      if (code[1] != FX_ZERO) {
+        bu = max(bu, fx_field_bits(q[1], m2[0]));
+        bw = max(bw, fx_field_bits(q[1], m2[1]));
+      }
+      FxColumn c;
+      c.s1 = code[0] == FX_ZERO ? -63 : q[0] - (bu - 62);
+      c.s2u = code[1] == FX_ZERO ? -63 : q[1] - (bu - 62);
+      c.s2w = code[1] == FX_ZERO ? -63 : q[1] - (bw - 61);
+      c.s3 = code[2] == FX_ZERO ? -63 : q[2] - (bw - 61);
+      c.code = code[0] == FX_NAN || code[1] == FX_NAN || code[2] == FX_NAN ? FX_NAN
+             : bu == NONE || bw == NONE ? FX_ZERO : FX_PLAIN;
+      c.e = c.code == FX_PLAIN ? (bu - 62) + (bw - 61) + 64 : NONE;
+      cols[tid] = c;
+    }
+    __syncthreads();
+    for (int e = tid; e < CP * M; e += NT) {
+      const int pr = e / M, p = e % M;
+      const int zp = zi<double>(p);
+      const int ez = max(cols[2 * pr].e, cols[2 * pr + 1].e);
+      long long c[2][3];
+#pragma unroll 1
+      for (int cc = 0; cc < 2; ++cc) {
+        const int col = 2 * pr + cc;
+        const FxColumn& fc = cols[col];
+        const fx2 z1 = A[col * LP + zp], z2 = A[(NC + col) * LP + zp], z3 = A[(2 * NC + col) * LP + zp];
+        // (parts exchanged)
+        const fxsplit ux = fx_split(fx_shl(z1.y, fc.s1)), uy = fx_split(fx_shl(z1.x, fc.s1));
+        const fxsplit uz = fx_split(fx_shl(z2.y, fc.s2u)), wx = fx_split(fx_shl(z2.x, fc.s2w));
+        const fxsplit wy = fx_split(fx_shl(z3.y, fc.s3)), wz = fx_split(fx_shl(z3.x, fc.s3));
+        c[0][0] = c[1][0]; c[0][1] = c[1][1]; c[0][2] = c[1][2];
+        c[1][0] = fx_det(uy, wz, uz, wy);
+        c[1][1] = fx_det(uz, wx, ux, wz);
+        c[1][2] = fx_shl(fx_det(ux, wy, uy, wx), fc.e - ez);
+      }
+      A[2 * pr * LP + zp] = fx2{c[0][0], c[0][1]};
+      A[(NC + 2 * pr) * LP + zp] = fx2{c[0][2], c[1][2]};
+      A[(2 * NC + 2 * pr) * LP + zp] = fx2{c[1][0], c[1][1]};
+    }
+    __syncthreads();
+  {
+      // forward lines l = t CP + pr
+      const int l = MapContig<double, M, NF>::template line<Fwd::NB0>(tid);
+      const int j = MapContig<double, M, NF>::template bfly<Fwd::NB0>(tid);
+      const bool act = tid < Fwd::G0;
+      fx2 v[Fwd::R0];
+      int sum = 0;
+      if (act) {
+        __builtin_assume(j >= 0 && j < Fwd::NB0);
+        __builtin_assume(l >= 0 && l < NF);
+#pragma unroll
+        for (int r = 0; r < Fwd::R0; ++r) {
+          v[r] = A[2 * l * LP + zi<double>(j + r * Fwd::NB0)];
+          const int hx = (int)(v[r].x >> 32), hy = (int)(v[r].y >> 32);
+          sum += max(hx ^ (hx >> 31), hy ^ (hy >> 31)) >> 5;
+        }
+        sum += Fwd::R0;                                // the shifted-out bits
+        sum += (sum >> 2) + (sum >> 3) + (sum >> 4) + 3;   // times 1.4375 > sqrt(2), rounded up
+      }
+      // |z| sums below 2^(37 + bits); to 2^62
+      const int sh = max(0, 37 + 32 - __clz(Fwd::line_max(sum, nullptr)) - 62);
+      if (act) {
+        const long long half = (1ll << sh) >> 1;
+#pragma unroll
+        for (int r = 0; r < Fwd::R0; ++r) v[r] = fx2{(v[r].x + half) >> sh, (v[r].y + half) >> sh};
+        Fwd::first_dft(v, [&](int p, fx2 z) { A[(2 * l + 1) * LP + zi<double>(p)] = z; }, j);
+        if (j == 0) {
+          const int t = l / CP, pr = l - t * CP;
+          const FxColumn& ca = cols[2 * pr];
+          const FxColumn& cb = cols[2 * pr + 1];
+          const int e = t == 0 ? ca.e : t == 1 ? max(ca.e, cb.e) : cb.e;
+          int code = t == 0 ? ca.code : t == 2 ? cb.code : ca.code == FX_NAN || cb.code == FX_NAN ? FX_NAN
+                   : ca.code == FX_ZERO && cb.code == FX_ZERO ? FX_ZERO : FX_PLAIN;
+          int q = e + sh + Fwd::GR - 1;   // the modes are halved by the unpacking
+          if (code == FX_PLAIN && (q < -950 || q > 900)) {   // near the ends of the double range, or beyond
+            code = q < -950 - FX_RANGE ? FX_ZERO : q < 0 ? FX_TINY : q <= 900 + FX_RANGE ? FX_HUGE : FX_NAN;
+            q += q < 0 ? FX_RANGE : -FX_RANGE;
+          }
+          line_s[l] = Fwd::pack_state(code == FX_ZERO || code == FX_NAN ? 0 : q, code);
+        }
+      }
+    }
+    __syncthreads();
+  p3x_second<M, CP, NT>(LP, 0, 2 * LP, NF, false);
+  __syncthreads();
+  for (int e = tid; e < CP * 3 * H; e += NT) {
+    const int k = e % H;
+    const int t = (e / H) % 3;
+    const int pr = e / (3 * H);
+    const State s = Fwd::unpack_state(line_s[t * CP + pr]);
+    const fx2* line = A + 2 * (t * CP + pr) * LP;
+    const fx2 z = line[zi<double>(k)], w = line[zi<double>(k == 0 ? 0 : M - k)];
+    const int q20 = s.q << 20;
+    double2 X = make_double2(fx_to_double(z.x + w.x, q20), fx_to_double(z.y - w.y, q20));
+    double2 Y = make_double2(fx_to_double(z.y + w.y, q20), fx_to_double(w.x - z.x, q20));
+    if (s.code != FX_PLAIN) {
+      const double f = fx_code_factor(s.code);
+      X = make_double2(X.x * f, X.y * f);
+      Y = make_double2(Y.x * f, Y.y * f);
+    }
     const int ca = col0 + 2 * pr, cb = ca + 1;
     if (t == 0) {
       if (ca < a.ncols) {
