@@ -24,16 +24,16 @@ static std::vector<CL> roots(int L) {
 }
 
 // one line through the plan of length L
-template <int L, bool CONTIG, bool INV> struct Line {
-  static constexpr int ST = fx_stages(L, CONTIG), SHIFT = fx_total_growth(L, CONTIG);
-  static constexpr int R0 = fx_radix(L, 0, CONTIG), NB0 = L / R0;
+template <int L, bool INV> struct Line {
+  static constexpr int ST = fx_stages(L), SHIFT = fx_total_growth(L);
+  static constexpr int R0 = fx_radix(L, 0), NB0 = L / R0;
   std::vector<fxtw> tw;
   Line() : tw(L) {
     for (int m = 0; m < L; ++m) tw[m] = fx_make_twiddle(m, L, cosl(TWO_PI * m / L), sinl(TWO_PI * m / L));
   }
   template <int S, int NS> void stages(std::vector<fx2>& v) const {
-    constexpr int R = fx_radix(L, S, CONTIG), NB = L / R, G = fx_growth(R);
-    constexpr int GN = S + 1 < ST ? fx_growth(fx_radix(L, S + 1, CONTIG)) : 1;
+    constexpr int R = fx_radix(L, S), NB = L / R, G = fx_growth(R);
+    constexpr int GN = S + 1 < ST ? fx_growth(fx_radix(L, S + 1)) : 1;
     std::vector<fx2> o(L);
     for (int j = 0; j < NB; ++j) {
       const int k = j % NS;
@@ -91,8 +91,8 @@ template <typename F> void fft(std::complex<F>* a, int n, int sign) {
   }
 }
 
-template <int L, bool CONTIG, bool INV> void accuracy() {
-  const Line<L, CONTIG, INV> line;
+template <int L, bool INV> void accuracy() {
+  const Line<L, INV> line;
   const auto W = roots(L);
   for (int kind = 0; kind < 5; ++kind) {
     std::mt19937_64 g(5 + kind);
@@ -133,13 +133,13 @@ template <int L, bool CONTIG, bool INV> void accuracy() {
         ref += std::norm(s * inv);
       }
     }
-    std::printf("accuracy %d %d %d %d %.4Le %.4Le\n", L, (int)CONTIG, (int)INV, kind, std::sqrt(fix / ref), std::sqrt(dbl / ref));
+    std::printf("accuracy %d %d %d %.4Le %.4Le\n", L, (int)INV, kind, std::sqrt(fix / ref), std::sqrt(dbl / ref));
   }
 }
 
 // mean error of each output over many lines, in standard errors of that mean
-template <int L, bool CONTIG, bool INV> void bias() {
-  const Line<L, CONTIG, INV> line;
+template <int L, bool INV> void bias() {
+  const Line<L, INV> line;
   constexpr int NR = 1500;
   std::mt19937_64 g(9);
   std::vector<LD> sx(L, 0), sy(L, 0);
@@ -161,22 +161,18 @@ template <int L, bool CONTIG, bool INV> void bias() {
   const LD sd = std::sqrt(var / ((LD)NR * L)), noise = sd / std::sqrt((LD)NR);
   LD worst = 0;
   for (int p = 0; p < L; ++p) worst = std::max(worst, std::max(std::fabs(sx[p]), std::fabs(sy[p])) / NR);
-  std::printf("bias %d %d %d %.4Lf %.4Lf %.4Lf\n", L, (int)CONTIG, (int)INV, worst, noise, sd);
+  std::printf("bias %d %d %.4Lf %.4Lf\n", L, (int)INV, worst, noise);
 }
 
-template <int L, bool CONTIG> void both() {
-  accuracy<L, CONTIG, false>();
-  accuracy<L, CONTIG, true>();
-  bias<L, CONTIG, false>();
-  bias<L, CONTIG, true>();
-}
-template <int L> void plans() {
-  both<L, true>();
-  if constexpr (fx_stages(L, false) != fx_stages(L, true)) both<L, false>();
+template <int L> void both() {
+  accuracy<L, false>();
+  accuracy<L, true>();
+  bias<L, false>();
+  bias<L, true>();
 }
 
 int main() {
-  plans<8>(); plans<12>(); plans<16>(); plans<24>(); plans<32>(); plans<48>(); plans<64>(); plans<96>();
-  plans<128>(); plans<192>(); plans<256>(); plans<384>(); plans<512>(); plans<768>();
+  both<8>(); both<12>(); both<16>(); both<24>(); both<32>(); both<48>(); both<64>(); both<96>();
+  both<128>(); both<192>(); both<256>(); both<384>(); both<512>(); both<768>();
   return 0;
 }

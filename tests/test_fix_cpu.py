@@ -26,7 +26,7 @@ def report(tmp_path_factory):
         if f[0] == "accuracy":
             acc[(int(f[1]), int(f[2]), int(f[3]))] = (float(f[4]), float(f[5]))
         else:
-            bias[(int(f[1]), int(f[2]))] = float(f[3])
+            bias[(int(f[1]), int(f[2]))] = (float(f[3]), float(f[4]))
     return acc, bias
 
 
@@ -43,7 +43,10 @@ def test_error_below_one_ulp_of_the_norm_and_below_doubles(report, length):
 
 
 @pytest.mark.parametrize("length", LENGTHS)
-def test_rounding_has_no_bias(report, length):
-    # the mean error of every output is within 6 standard errors of zero
+def test_rounding_bias_stays_below_half_a_quantum(report, length):
+    # the mean error of every output over 1500 lines: short twiddles leave up to
+    # 1/8 of a unit each and no output of a line meets more than two in a stage,
+    # plus 5 standard errors of the mean
     for inv in (0, 1):
-        assert report[1][(length, inv)] < 6.0
+        worst, noise = report[1][(length, inv)]
+        assert worst < 0.25 + 5.0 * noise

@@ -157,7 +157,7 @@ template <typename R> struct A3Args {
 
 template <typename R, int M, int CP>
 __host__ __device__ constexpr int adj_z_threads() {
-  return cmin(rthreads<R, M, 9 * CP, true>(), sizeof(R) == 8 ? 512 : 384);
+  return cmin(rthreads<R, M, 9 * CP, true>(), sizeof(R) == 8 ? 1024 : 384);
 }
 // Shared memory of k_adj_z: 9 CP inverse lines (exchange, then the physical
 // values in place) and 6 CP forward lines.

@@ -103,7 +103,7 @@ inline int zpass_prefetch_distance(int nt, size_t smem) {
 template <typename R, int L, bool INV, bool XAXIS = false, class Op>
 inline cudaError_t launch_lines(const Op& op, int nouter, const C2<R>* tw, cudaStream_t s) {
   constexpr int NLINES = NLof<R, L, XAXIS, Op>::value;
-  constexpr int NT = cmin(rthreads<R, L, NLINES>(), sizeof(R) == 8 ? 512 : 384);
+  constexpr int NT = cmin(rthreads<R, L, NLINES>(), sizeof(R) == 8 ? 1024 : 384);
   const size_t smem = (size_t)rsmem_elems<R, L, NLINES>() * sizeof(C2<R>);
   constexpr auto kern = k_lines<R, L, INV, NLINES, NT, Op>;
   cudaError_t e = prepare_kernel<kern>(smem);

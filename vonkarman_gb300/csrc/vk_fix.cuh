@@ -106,30 +106,29 @@ template <int B> VK_FIX_HD fx2 fx_multiple(fx2 a) {
 }
 // a / 2^B (the untwiddled input beside twiddled ones)
 template <int B> VK_FIX_HD fx2 fx_shift(fx2 a) { return fx2{fx_bump<B>(a.x) >> B, fx_bump<B>(a.y) >> B}; }
-// Plans.  Contiguous lines (z passes): two stages with 2^b butterflies in the
-// first, so that a line's threads share a warp; short lines take small radices
-// (a small grid is bound by the latency of one thread's work), long ones the
-// largest that registers hold.  Interleaved lines (x and y passes): three
-// stages of radices up to 8 from 256 to 512 points, which need half the registers
-// and let twice the warps be resident.
+// Plans.  From 256 points on three stages of small radices (up to 12), whose few
+// registers let three times the warps of a two-stage plan be resident: the
+// integer code is bound by latency, not by its instruction count.  Below, two
+// stages, the shortest lines with small radices (a small grid is bound by the
+// latency of one thread's work).  The first stage has 2^b or 16 c butterflies,
+// so that groups of lanes keep one contiguous line.
 VK_FIX_HD constexpr int fx_radix0(int L) {
   return L == 8 ? 2 : L == 12 ? 3 : L == 16 ? 4 : L == 24 ? 6 : L == 32 ? 4 : L == 48 ? 6 : L == 64 ? 8 : L == 96 ? 12
-       : L == 128 ? 16 : L == 192 ? 12 : L == 256 ? 16 : L == 384 ? 24 : L == 512 ? 16 : L == 768 ? 24 : 0;
+       : L == 128 ? 16 : L == 192 ? 12 : L == 256 ? 8 : L == 384 ? 8 : L == 512 ? 8 : L == 768 ? 12 : 0;
 }
 VK_FIX_HD constexpr bool fx_supported(int L) { return fx_radix0(L) > 0; }
-VK_FIX_HD constexpr int fx_stages(int L, bool contig) { return !contig && L >= 256 && L <= 512 ? 3 : 2; }
-VK_FIX_HD constexpr int fx_radix(int L, int s, bool contig) {
-  return fx_stages(L, contig) == 2 ? (s == 0 ? fx_radix0(L) : L / fx_radix0(L))
-       : s < 2 ? 8 : L / 64;
+VK_FIX_HD constexpr int fx_stages(int L) { return L >= 256 ? 3 : 2; }
+VK_FIX_HD constexpr int fx_radix(int L, int s) {
+  return s == 0 ? fx_radix0(L) : fx_stages(L) == 2 ? L / fx_radix0(L) : s == 1 ? 8 : L / fx_radix0(L) / 8;
 }
 // log2 of the factor that the twiddles of a later stage of radix r divide by;
 // their components are held in units of 2^-(64 - growth), which makes
 // fx_twiddle's a w / 2^64 the scaled product
 VK_FIX_HD constexpr int fx_growth(int r) { return r <= 4 ? 2 : r <= 8 ? 3 : r <= 16 ? 4 : 5; }
 // sum of the growths of a plan's stages: the outputs' exponent above the quantum
-VK_FIX_HD constexpr int fx_total_growth(int L, bool contig) {
+VK_FIX_HD constexpr int fx_total_growth(int L) {
   int g = 0;
-  for (int s = 1; s < fx_stages(L, contig); ++s) g += fx_growth(fx_radix(L, s, contig));
+  for (int s = 1; s < fx_stages(L); ++s) g += fx_growth(fx_radix(L, s));
   return g;
 }
 // W_L^m = c - i s (cosine and sine of 2 pi m / L) in units of 2^-62 (host)
@@ -160,6 +159,7 @@ VK_FIX_HD fxtw fx_stage_twiddle(fxtw w, int g) {
     const long long v = ((long long)h * 4294967296ll + l) >> (g - 2);
     l = (int)(unsigned)(unsigned long long)v;
     h = (int)((v - (long long)l) >> 32);
+    if (l == INT32_MIN) ++l;   // fx_twiddle negates it
   };
   const int r0 = w.cl & 3;
   w.cl &= ~3;
@@ -170,14 +170,12 @@ VK_FIX_HD fxtw fx_stage_twiddle(fxtw w, int g) {
   return w;
 }
 
-// Constants k in (0, 1/2) in units of 2^-64: 1 - cos(2 pi m / 32), sin(2 pi m / 32)
-// (m = 3: 1 - sin), 1 - sqrt(3)/2.  Factors above 1/2 are applied as
-// x - x (1 - k), so that the constant's high word stays signed.
+// Constants k in (0, 1/2) in units of 2^-64: 1 - cos(pi/8), sin(pi/8),
+// 1 - sqrt(1/2), 1 - sqrt(3)/2.  Factors above 1/2 are applied as x - x (1 - k),
+// so that the constant's high word stays signed.
 struct FxConst {
-  static constexpr unsigned long long omc[5] = {0ull, 0x04eb4180451a7eaaull, 0x137ca1866b95cebbull, 0x2b24ceb78af2e7e6ull,
-                                                0x4afb0ccc06219b7cull};
-  static constexpr unsigned long long sn[4] = {0ull, 0x31f17078d34c156dull, 0x61f78a9abaa58b47ull, 0x71c626328cb9bc9bull};
-  static constexpr unsigned long long omr3 = 0x224c28bd3d9aac62ull;
+  static constexpr unsigned long long omc = 0x137ca1866b95cebbull, sn = 0x61f78a9abaa58b47ull;
+  static constexpr unsigned long long omr2 = 0x4afb0ccc06219b7cull, omr3 = 0x224c28bd3d9aac62ull;
 };
 template <unsigned long long K, bool NEG> struct FxWords {
   static constexpr long long v = NEG ? -(long long)K : (long long)K;
@@ -190,36 +188,30 @@ template <unsigned long long K> VK_FIX_HD long long fx_mulc(long long v) {
   const fxsplit s = fx_split(v);
   return fx_wide(s.h, W::h) + (long long)fx_madhi(s.l, W::h, fx_madhi(s.h, W::l, 1));
 }
-// a exp(-+ 2 pi i M / 32) (INV: +)
-template <int M, bool INV> VK_FIX_HD fx2 fx_w32(fx2 a) {
-  constexpr int q = ((M + 4) & 31) / 8;          // quarter turns
-  constexpr int m = ((M + 4) & 31) - 4 - 8 * q;  // rest in [-4, 4)
+// a exp(-+ 2 pi i M / 16) (INV: +)
+template <int M, bool INV> VK_FIX_HD fx2 fx_w16(fx2 a) {
+  constexpr int q = ((M + 2) & 15) / 4;          // quarter turns
+  constexpr int m = ((M + 2) & 15) - 2 - 4 * q;  // rest in [-2, 2)
   if constexpr (q == 1) a = fx_rot<INV>(a);
   if constexpr (q == 2) a = fx_neg(a);
   if constexpr (q == 3) a = fx_rot<!INV>(a);
   if constexpr (m == 0) {
     return a;
-  } else if constexpr (m == -4) {   // sqrt(1/2) (1 +- i): forward exp(+i pi/4)
+  } else if constexpr (m == -2) {   // sqrt(1/2) (1 +- i): forward exp(+i pi/4)
     const long long u = INV ? a.x + a.y : a.x - a.y, w = INV ? a.y - a.x : a.y + a.x;
-    return fx2{u - fx_mulc<FxConst::omc[4]>(u), w - fx_mulc<FxConst::omc[4]>(w)};
+    return fx2{u - fx_mulc<FxConst::omr2>(u), w - fx_mulc<FxConst::omr2>(w)};
   } else {
-    constexpr int ma = m < 0 ? -m : m;
     constexpr bool pos = (m > 0) != INV;   // re = c x + s y, im = c y - s x with s > 0; else the other signs
-    using C = FxWords<FxConst::omc[ma], true>;                              // c = 1 + C
-    using S = FxWords<FxConst::sn[ma], (ma == 3) ? pos : !pos>;             // ma == 3: +-(1 - s') enters negated
-    using T = FxWords<FxConst::sn[ma], (ma == 3) ? !pos : pos>;
+    using C = FxWords<FxConst::omc, true>;   // c = 1 + C
+    using S = FxWords<FxConst::sn, !pos>;
+    using T = FxWords<FxConst::sn, pos>;
     const fxsplit x = fx_split(a.x), y = fx_split(a.y);
     int t = fx_madhi(x.l, C::h, fx_madhi(x.h, C::l, 2));
     t = fx_madhi(y.l, S::h, fx_madhi(y.h, S::l, t));
     int s = fx_madhi(y.l, C::h, fx_madhi(y.h, C::l, 2));
     s = fx_madhi(x.l, T::h, fx_madhi(x.h, T::l, s));
-    fx2 r{fx_wide(x.h, C::h) + fx_wide(y.h, S::h) + (long long)t + a.x,
-          fx_wide(y.h, C::h) + fx_wide(x.h, T::h) + (long long)s + a.y};
-    if constexpr (ma == 3) {
-      r.x = pos ? r.x + a.y : r.x - a.y;
-      r.y = pos ? r.y - a.x : r.y + a.x;
-    }
-    return r;
+    return fx2{fx_wide(x.h, C::h) + fx_wide(y.h, S::h) + (long long)t + a.x,
+               fx_wide(y.h, C::h) + fx_wide(x.h, T::h) + (long long)s + a.y};
   }
 }
 
@@ -263,51 +255,38 @@ template <bool INV> struct FxDft<8, INV> {
     fx2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
     FxDft<4, INV>::run(e);
     FxDft<4, INV>::run(o);
-    o[1] = fx_w32<4, INV>(o[1]);
+    o[1] = fx_w16<2, INV>(o[1]);
     o[2] = fx_rot<INV>(o[2]);
-    o[3] = fx_w32<12, INV>(o[3]);
+    o[3] = fx_w16<6, INV>(o[3]);
     for (int k = 0; k < 4; ++k) {
       v[k] = fx_add(e[k], o[k]);
       v[k + 4] = fx_sub(e[k], o[k]);
     }
   }
 };
-// A x 4 (Cooley-Tukey, A = 4, 8): A-point DFTs over x[b + 4 a], constant
-// twiddles W^(b k), 4-point DFTs over b; output k + A j.
-template <int A, bool INV> struct FxDftBy4 {
-  template <int K> static VK_FIX_HD void column(fx2 (*y)[A], fx2* v) {
-    fx2 t[4] = {y[0][K], fx_w32<K * (8 / A), INV>(y[1][K]), fx_w32<2 * K * (8 / A), INV>(y[2][K]),
-                fx_w32<3 * K * (8 / A), INV>(y[3][K])};
+// 4 x 4 (Cooley-Tukey): 4-point DFTs over x[b + 4 a], constant twiddles W16^(b k),
+// 4-point DFTs over b; output k + 4 j.
+template <bool INV> struct FxDft<16, INV> {
+  template <int K> static VK_FIX_HD void column(fx2 (*y)[4], fx2* v) {
+    fx2 t[4] = {y[0][K], fx_w16<K, INV>(y[1][K]), fx_w16<2 * K, INV>(y[2][K]), fx_w16<3 * K, INV>(y[3][K])};
     FxDft<4, INV>::run(t);
-    for (int j = 0; j < 4; ++j) v[K + A * j] = t[j];
+    for (int j = 0; j < 4; ++j) v[K + 4 * j] = t[j];
   }
   static VK_FIX_HD void run(fx2* v) {
-    fx2 y[4][A];
+    fx2 y[4][4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
 #pragma unroll
-      for (int a = 0; a < A; ++a) y[b][a] = v[b + 4 * a];
-      FxDft<A, INV>::run(y[b]);
+      for (int a = 0; a < 4; ++a) y[b][a] = v[b + 4 * a];
+      FxDft<4, INV>::run(y[b]);
     }
     column<0>(y, v);
     column<1>(y, v);
     column<2>(y, v);
     column<3>(y, v);
-    if constexpr (A == 8) {
-      column<4>(y, v);
-      column<5>(y, v);
-      column<6>(y, v);
-      column<7>(y, v);
-    }
   }
 };
-template <bool INV> struct FxDft<16, INV> {
-  static VK_FIX_HD void run(fx2* v) { FxDftBy4<4, INV>::run(v); }
-};
-template <bool INV> struct FxDft<32, INV> {
-  static VK_FIX_HD void run(fx2* v) { FxDftBy4<8, INV>::run(v); }
-};
-// 3 x B with B = 2, 4, 8 (coprime: no twiddles): n = B n1 + 3 n2 mod 3B, and
+// 3 x B with B = 2, 4 (coprime: no twiddles): n = B n1 + 3 n2 mod 3B, and
 // k = k1 mod 3 = k2 mod B.
 template <int B, bool INV> struct FxDft3 {
   static VK_FIX_HD void run(fx2* v) {
@@ -337,10 +316,6 @@ template <bool INV> struct FxDft<6, INV> {
 template <bool INV> struct FxDft<12, INV> {
   static VK_FIX_HD void run(fx2* v) { FxDft3<4, INV>::run(v); }
 };
-template <bool INV> struct FxDft<24, INV> {
-  static VK_FIX_HD void run(fx2* v) { FxDft3<8, INV>::run(v); }
-};
-
 // ---------------------------------------------------------------------------
 // Doubles <-> fixed point
 // ---------------------------------------------------------------------------

@@ -63,10 +63,10 @@ __host__ __device__ constexpr int rplan_radix_fc(int L, int s) {
 }
 // FP64 lines run in fixed point with the plans of vk_fix.cuh.
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rstages(int L) {
-  return sizeof(R) == 4 ? rplan_stages_f(L) : fx_supported(L) ? fx_stages(L, CONTIG) : -1;
+  return sizeof(R) == 4 ? rplan_stages_f(L) : fx_supported(L) ? fx_stages(L) : -1;
 }
 template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rradix(int L, int s) {
-  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : fx_radix(L, s, CONTIG);
+  return sizeof(R) == 4 ? (CONTIG ? rplan_radix_fc(L, s) : rplan_radix_f(L, s)) : fx_radix(L, s);
 }
 // threads of a CTA: one butterfly per thread in the widest stage (FP64 plans of
 // two stages above 96 points: in the first stage, and a line of the second; of
@@ -74,8 +74,8 @@ template <typename R, bool CONTIG = false> __host__ __device__ constexpr int rra
 template <typename R, int L, int NLINES, bool CONTIG = false, int S = 0>
 __host__ __device__ constexpr int rthreads() {
   if constexpr (sizeof(R) == 8) {
-    constexpr int nb0 = L / fx_radix(L, 0, CONTIG), nb1 = L / fx_radix(L, 1, CONTIG);
-    return round32(L <= 96 || fx_stages(L, CONTIG) == 3 ? cmax(nb0, nb1) * NLINES : cmax(nb0 * NLINES, CONTIG ? nb1 : 0));
+    constexpr int nb0 = L / fx_radix(L, 0), nb1 = L / fx_radix(L, 1);
+    return round32(L <= 96 || fx_stages(L) == 3 ? cmax(nb0, nb1) * NLINES : cmax(nb0 * NLINES, CONTIG ? nb1 : 0));
   } else if constexpr (S >= rstages<R, CONTIG>(L)) {
     return 32;
   } else {
@@ -121,18 +121,14 @@ __device__ __forceinline__ int ridx(int pos, int l) {
   }
 }
 
-// Resident CTAs per SM of the fixed-point kernels: radices 16 to 32 of 64-bit
-// complex integers hold 64 to 128 registers of data, so about 12 warps of up
-// to 168 registers per SM.
+// Resident CTAs per SM of the fixed-point kernels, through the registers they
+// may take: three-stage plans (radices up to 8: 32 registers of data) run best
+// with 1152 threads of 56 registers per SM, two-stage plans (up to radix 16: 64
+// of data) with 512 of 128 (N = 256 P2: 1.35 ms with two stages and 384
+// threads, 1.39 with three and 768, 1.22 with three and 1152; N = 128 P2: 0.168
+// ms with 384 threads, 0.150 with 512).
 template <int L, int NT>
-__host__ __device__ constexpr int fx_min_blocks() { return L >= 512 ? 1 : cmax(1, 384 / NT); }
-#ifndef FX3T
-#define FX3T 1152
-#endif
-template <int L, int NT>
-__host__ __device__ constexpr int fx_lines_min_blocks() {
-  return fx_stages(L, false) == 3 ? cmax(1, FX3T / NT) : L <= 192 ? cmax(1, 512 / NT) : fx_min_blocks<L, NT>();
-}
+__host__ __device__ constexpr int fx_min_blocks() { return cmax(1, (fx_stages(L) == 3 ? 1152 : 512) / NT); }
 
 // Minimum resident CTAs per SM requested from the compiler (caps registers):
 // 24 warps per SM for the strided passes where the plan allows it; one or two
@@ -141,7 +137,7 @@ __host__ __device__ constexpr int fx_lines_min_blocks() {
 template <typename R, int L, int NT, bool EPI = false>
 __host__ __device__ constexpr int lines_min_blocks() {
   if constexpr (sizeof(R) == 8) {
-    return fx_lines_min_blocks<L, NT>();
+    return fx_min_blocks<L, NT>();
   } else {
     return L >= 768 ? (EPI ? 1 : 2) : EPI ? cmax(1, 512 / NT) : L >= 512 ? 2 : L >= 384 ? (NT >= 384 ? 2 : 3)
          : NT < 128 ? 4 : cmax(1, 768 / NT);
@@ -328,32 +324,43 @@ struct FxState { int q, code; };
 
 template <int L, int NT, int NLINES, class MAP>
 __host__ __device__ constexpr int fx_round_lines() {   // lines per stage-1 round (contiguous lines)
-  return cmin(NT / (L / fx_radix(L, 1, true)), NLINES);
+  return cmin(NT / (L / fx_radix(L, fx_stages(L) - 1)), NLINES);
 }
 
 template <int L, bool INV, int NT, int NLINES, class MAP, bool SL, int Z0, int Z1>
 struct FxLines {
-  static constexpr bool CT = MAP::CONTIG;
-  static constexpr int ST = fx_stages(L, CT);
-  static constexpr int R0 = fx_radix(L, 0, CT), NB0 = L / R0, G0 = NB0 * NLINES;
+  static constexpr int ST = fx_stages(L);
+  static constexpr int R0 = fx_radix(L, 0), NB0 = L / R0, G0 = NB0 * NLINES;
   // the last stage: radix, butterflies, growth, and its twiddles' place in the table
-  static constexpr int R1 = fx_radix(L, ST - 1, CT), NB1 = L / R1, G1 = NB1 * NLINES;
+  static constexpr int R1 = fx_radix(L, ST - 1), NB1 = L / R1, G1 = NB1 * NLINES;
   static constexpr int GR = fx_growth(R1);
-  static constexpr int TW1 = twtab_off<double, CT>(L, ST - 1);
-  static constexpr int TG = fx_total_growth(L, CT);
+  static constexpr int TW1 = twtab_off<double, MAP::CONTIG>(L, ST - 1);
+  static constexpr int TG = fx_total_growth(L);
   // growth of the stage after the first
-  static constexpr int GN = fx_growth(fx_radix(L, 1, CT));
+  static constexpr int GN = fx_growth(fx_radix(L, 1));
   static constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
   static constexpr int NW0 = (G0 + 31) / 32;
   static constexpr int CODE_SHIFT = 24;   // stored line state: exponent + (code << 24)
   static_assert(G0 <= NT, "one first-stage butterfly per thread");
-  static_assert(!MAP::CONTIG || 32 % NB0 == 0, "a contiguous line's first stage shares a warp");
+  static_assert(!MAP::CONTIG || 32 % NB0 == 0 || NB0 % 16 == 0, "groups of lanes keep one contiguous line");
+  // words of the part array of front and line_max
+  static constexpr int PARTS = !MAP::CONTIG ? NW0 * NLINES : 32 % NB0 == 0 ? 1 : G0 / 16;
   static_assert(MAP::CONTIG || (32 % NLINES == 0 && !SL), "interleaved lines tile a warp");
 
   __device__ __forceinline__ static int line_max(int m, int* part) {
-    if constexpr (MAP::CONTIG) {
+    if constexpr (MAP::CONTIG && 32 % NB0 == 0) {
 #pragma unroll
       for (int o = 1; o < NB0; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    } else if constexpr (MAP::CONTIG) {   // a line's threads are whole groups of 16 lanes
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const int g = threadIdx.x;
+      if (g < G0 && g % 16 == 0) part[g / 16] = m;
+      __syncthreads();
+      const int l = g < G0 ? g / NB0 : 0;
+      m = part[l * (NB0 / 16)];
+#pragma unroll
+      for (int i = 1; i < NB0 / 16; ++i) m = max(m, part[l * (NB0 / 16) + i]);
     } else {
 #pragma unroll
       for (int o = NLINES; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -452,7 +459,7 @@ struct FxLines {
   // The middle stage of a three-stage plan, in place (begins and ends with the
   // exchange complete).
   __device__ __forceinline__ static void middle(fx2* xb, const fxtw* __restrict__ tw) {
-    constexpr int RM = fx_radix(L, 1, CT), NBM = L / RM, GM = NBM * NLINES;
+    constexpr int RM = fx_radix(L, 1), NBM = L / RM, GM = NBM * NLINES;
     static_assert(GM <= NT, "one butterfly per thread");
     const int g = threadIdx.x;
     const int l = MAP::template line<NBM>(g), j = MAP::template bfly<NBM>(g);
@@ -471,6 +478,29 @@ struct FxLines {
       u[0] = fx_multiple<GR>(u[0]);
 #pragma unroll
       for (int r = 0; r < RM; ++r) xb[MAP::template idx<0>((j - k) * RM + k + r * R0, l)] = u[r];
+    }
+    __syncthreads();
+  }
+
+  // the same for nl contiguous lines, line l at xs + l ls
+  __device__ __forceinline__ static void middle_rt(fx2* xs, int ls, int nl, const fxtw* __restrict__ tw) {
+    constexpr int RM = fx_radix(L, 1), NBM = L / RM;
+    static_assert(NBM * NLINES <= NT, "one butterfly per thread");
+    const int l = threadIdx.x / NBM, j = threadIdx.x % NBM;
+    __builtin_assume(j >= 0 && j < NBM);
+    const bool act = l < nl;
+    fx2 u[RM];
+    if (act) {
+#pragma unroll
+      for (int r = 0; r < RM; ++r) u[r] = xs[l * ls + zi<double>(j + r * NBM)];
+    }
+    __syncthreads();
+    if (act) {
+      const int k = j % R0;
+      later_dft<RM, 0>(u, tw, k, R0);
+      u[0] = fx_multiple<GR>(u[0]);
+#pragma unroll
+      for (int r = 0; r < RM; ++r) xs[l * ls + zi<double>((j - k) * RM + k + r * R0)] = u[r];
     }
     __syncthreads();
   }
@@ -537,7 +567,7 @@ struct FxLines {
   template <class FILL, class STF>
   __device__ __forceinline__ static void run(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, const STF& st,
                                              int xe) {
-    __shared__ int part[MAP::CONTIG ? 1 : NW0 * NLINES];
+    __shared__ int part[PARTS];
     __shared__ int line_s[MAP::CONTIG ? NLINES : 1];
     const State s0 = front(xb, fill, part, line_s, xe);
     __syncthreads();
@@ -561,11 +591,11 @@ struct FxLines {
 // fill functor of FxLines from ld / pp: all loads of a chunk are issued before
 // any arithmetic on them (chunks of 256 bytes per thread where the raw inputs
 // are wider than one complex value)
-template <int L, bool CONTIG, int Z0, int Z1, class LD, class PP> struct FxFill {
+template <int L, int Z0, int Z1, class LD, class PP> struct FxFill {
   const LD& ld;
   const PP& pp;
   __device__ __forceinline__ void operator()(int l, int j, double2* d) const {
-    constexpr int R0 = fx_radix(L, 0, CONTIG), NB0 = L / R0;
+    constexpr int R0 = fx_radix(L, 0), NB0 = L / R0;
     constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
     using Raw = decltype(ld(0, 0));
     constexpr int CH = sizeof(Raw) > sizeof(double2) ? cmin(R0, (int)(256 / sizeof(Raw))) : R0;
@@ -596,7 +626,7 @@ __device__ __forceinline__ void fft_lines(C2<R>* xb, const C2<R>* __restrict__ t
   if constexpr (sizeof(R) == 8) {
     static_assert(TT, "per-stage tables");
     FxLines<L, INV, NT, NLINES, MAP, SL, Z0, Z1>::run(reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw),
-                                                      FxFill<L, MAP::CONTIG, Z0, Z1, LD, PP>{ld, pp}, st, 0);
+                                                      FxFill<L, Z0, Z1, LD, PP>{ld, pp}, st, 0);
   } else {
     RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
   }
@@ -696,7 +726,7 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
         if (kd != K) return;   // uniform over the CTA
         const auto ld = [&](int, int p) { return op.template load<K>(f, outer, z, p); };
         const auto pp = [&](int, int p, const auto& raw) { return op.template prep<K>(f, outer, z, p, raw); };
-        FxFill<L, false, Z0, Z1, decltype(ld), decltype(pp)>{ld, pp}(l, j, d);
+        FxFill<L, Z0, Z1, decltype(ld), decltype(pp)>{ld, pp}(l, j, d);
       });
     };
     int xe = 0;
@@ -749,7 +779,7 @@ __host__ __device__ constexpr int p5_threads() {
 }
 template <typename R, int L, int NLINES, int NT>
 __host__ __device__ constexpr int p5_min_blocks() {
-  return sizeof(R) == 8 ? (L >= 512 ? 1 : 3)
+  return sizeof(R) == 8 ? (L >= 768 ? 1 : 3)
        : NT >= 2 * rthreads<R, L, NLINES>() ? 2 : lines_min_blocks<R, L, NT, true>();
 }
 
@@ -1149,8 +1179,7 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
 // The last inverse stage leaves the fields in place with each line's exponent
 // and, per real field, the OR of the high words' magnitudes.  Those give each
 // column the shifts that bring u to 62 and omega to 61 bits; a product keeps the
-// upper 59 of its 123 bits (two products and their four floors per component,
-// with their mean returned, as in fx_twiddle).  The forward first stage shifts
+// upper 59 of its 123 bits.  The forward first stage shifts
 // its line right by what its largest butterfly needs (rounded), at most 6 bits.
 //
 // The inverse runs as a forward transform of lines with real and imaginary
@@ -1167,12 +1196,11 @@ struct FxColumn {       // per column: left shifts (negative: right) of the line
 __device__ __forceinline__ long long fx_shl(long long v, int s) {   // v 2^s, rounded for s < 0
   return s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
 }
-// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split)
+// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split): the
+// floors of the two products' cross terms cancel in the mean
 __device__ __forceinline__ long long fx_det(fxsplit a, fxsplit b, fxsplit c, fxsplit d) {
-  const int nh = -d.h, nl = -d.l;
-  int t = fx_madhi(a.l, b.h, fx_madhi(a.h, b.l, 2));
-  t = fx_madhi(c.l, nh, fx_madhi(c.h, nl, t));
-  return fx_wide(a.h, b.h) + fx_wide(c.h, nh) + (long long)t;
+  const int t = fx_madhi(a.l, b.h, fx_madhi(a.h, b.l, 0)), u = fx_madhi(c.l, d.h, fx_madhi(c.h, d.l, 0));
+  return fx_wide(a.h, b.h) - fx_wide(c.h, d.h) + (long long)(t - u);
 }
 // bits of a field whose high words' magnitudes OR to m, line exponent q
 __device__ __forceinline__ int fx_field_bits(int q, int m) { return q + 64 - __clz(m); }
@@ -1188,7 +1216,7 @@ template <int M, int CP> struct P3X {
   static constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
   static constexpr int TW = NI * LP;                                 // in units of fx2
   static constexpr int INTS = TW + twtab_elems<double, true>(M);
-  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn);
+  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn) + (NI * M / 128 + 1) * 4;
   __device__ __forceinline__ static fx2* lines() {
     extern __shared__ __align__(16) unsigned char vk_smem[];
     return reinterpret_cast<fx2*>(vk_smem);
@@ -1197,6 +1225,7 @@ template <int M, int CP> struct P3X {
   __device__ __forceinline__ static int* line_s() { return reinterpret_cast<int*>(lines() + INTS); }
   __device__ __forceinline__ static int* field_m() { return line_s() + NI; }
   __device__ __forceinline__ static FxColumn* cols() { return reinterpret_cast<FxColumn*>(field_m() + 2 * NI); }
+  __device__ __forceinline__ static int* part() { return reinterpret_cast<int*>(cols() + NC); }   // FxLines::PARTS
 };
 // Second stage of nl lines at stride ls, from xs to ds (element offsets), with
 // the fields' magnitudes where they are wanted.  Not inlined: both directions
@@ -1205,6 +1234,7 @@ template <int M, int CP, int NT>
 __device__ __forceinline__ void p3x_second(int xs, int ds, int ls, int nl, bool maxima) {
   using P = P3X<M, CP>;
   using Inv = FxLines<M, false, NT, P::NI, MapContig<double, M, P::NI>, true, 0, 0>;
+  if constexpr (Inv::ST == 3) Inv::middle_rt(P::lines() + xs, ls, nl, P::twiddles());
   Inv::back_rt(P::lines() + xs, ls, nl, P::twiddles(), [&](const fx2* u, int l, int j) {
     fx2* dst = P::lines() + ds + l * ls;
     int mx = 0, my = 0;
@@ -1260,7 +1290,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
         if (p == 0) return make_double2(r.b.x, r.a.x);
         return p < H ? make_double2(r.a.y + r.b.x, r.a.x - r.b.y) : make_double2(r.b.x - r.a.y, r.a.x + r.b.y);
       };
-      Inv::front(A, FxFill<M, true, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, nullptr, line_s, 0);
+      Inv::front(A, FxFill<M, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, P::part(), line_s, 0);
   }
   __syncthreads();
   p3x_second<M, CP, NT>(0, 0, LP, NI, true);
@@ -1338,7 +1368,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
         sum += (sum >> 2) + (sum >> 3) + (sum >> 4) + 3;   // times 1.4375 > sqrt(2), rounded up
       }
       // |z| sums below 2^(37 + bits); to 2^62
-      const int sh = max(0, 37 + 32 - __clz(Fwd::line_max(sum, nullptr)) - 62);
+      const int sh = max(0, 37 + 32 - __clz(Fwd::line_max(sum, P::part())) - 62);
       if (act) {
         const long long half = (1ll << sh) >> 1;
 #pragma unroll
@@ -1351,7 +1381,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
           const int e = t == 0 ? ca.e : t == 1 ? max(ca.e, cb.e) : cb.e;
           int code = t == 0 ? ca.code : t == 2 ? cb.code : ca.code == FX_NAN || cb.code == FX_NAN ? FX_NAN
                    : ca.code == FX_ZERO && cb.code == FX_ZERO ? FX_ZERO : FX_PLAIN;
-          int q = e + sh + Fwd::GR - 1;   // the modes are halved by the unpacking
+          int q = e + sh + Fwd::TG - 1;   // the modes are halved by the unpacking
           if (code == FX_PLAIN && (q < -950 || q > 900)) {   // near the ends of the double range, or beyond
             code = q < -950 - FX_RANGE ? FX_ZERO : q < 0 ? FX_TINY : q <= 900 + FX_RANGE ? FX_HUGE : FX_NAN;
             q += q < 0 ? FX_RANGE : -FX_RANGE;
@@ -1532,11 +1562,11 @@ template <typename R, int L> __host__ __device__ constexpr int fz_pairs() {
   for (int s = 1; s < rstages<R, true>(L); ++s) rad = cmin(rad, rradix<R, true>(L, s));
   return cmax(1, 192 * rad / L);
 }
-template <typename R, int NT>
-__host__ __device__ constexpr int fz_min_blocks() { return cmax(1, (sizeof(R) == 8 ? 384 : 768) / NT); }
+template <typename R, int L, int NT>
+__host__ __device__ constexpr int fz_min_blocks() { return sizeof(R) == 8 ? fx_min_blocks<L, NT>() : cmax(1, 768 / NT); }
 
 template <typename R, int L, int CP, int NT>
-__global__ void __launch_bounds__(NT, fz_min_blocks<R, NT>()) k_fz_r2c(FZArgs<R> a, const C2<R>* __restrict__ tw) {
+__global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_r2c(FZArgs<R> a, const C2<R>* __restrict__ tw) {
   constexpr int H = L / 2 + 1;
   constexpr int LP = zpad_len<R>(L);
   extern __shared__ __align__(16) unsigned char vk_smem[];
@@ -1563,7 +1593,7 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, NT>()) k_fz_r2c(FZArgs<R>
 }
 
 template <typename R, int L, int CP, int NT>
-__global__ void __launch_bounds__(NT, fz_min_blocks<R, NT>()) k_fz_c2r(FZArgs<R> a, const C2<R>* __restrict__ tw) {
+__global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_c2r(FZArgs<R> a, const C2<R>* __restrict__ tw) {
   constexpr int H = L / 2 + 1;
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, true>(L)];
