@@ -376,9 +376,9 @@ template <typename R> struct A5Args {
   AdjStageArgs<R> st;
 };
 
-template <typename R> struct A5Lines { static constexpr int value = sizeof(R) == 8 ? 4 : 8; };
+template <typename R> struct A5Lines { static constexpr int value = 8; };
 
-// Transposed P5 for the six cotangent fields (a_bar, o_bar): x-forward, keep
+// Transposed P5 (FP32) for the six cotangent fields (a_bar, o_bar): x-forward, keep
 // N of M modes, weight, and y = a_bar + i k x o_bar accumulated field by field
 // in shared memory (three accumulators; the thread producing output ix of a
 // field is the one that holds ix of every field, so the accumulation needs
@@ -404,38 +404,6 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
     const R ky = a.ks * (R)signed_k(iy, N);
     const R kz = a.ks * (R)z;
     const R wgt = a.s_out * (z == 0 ? R(1) : R(2));
-    if constexpr (sizeof(R) == 8) {
-      // one loop body for the six fields (the FP64 transform's code is large);
-      // wave numbers from shared memory (their conversion is an FP64 operation)
-      __shared__ double kx_s[N];
-      for (int i = threadIdx.x; i < N; i += NT) kx_s[i] = a.ks * (double)signed_k(i, N);   // ordered by the first FFT's barriers
-#pragma unroll 1
-      for (int c = 0; c < 6; ++c) {
-        if (c > 0) __syncthreads();   // xb is reused
-        const double2* src = a.in + (size_t)c * a.fsin + (iy * H + z);
-        // i k x o_bar (spectral_ops.rs:92-104), one o_bar component at a time:
-        // y_p += i kp o, y_q -= i kq o with (p, q) = (y, z), (z, x), (x, y)
-        const int p = c < 3 ? c : (c - 2) % 3, q = c < 3 ? c : (c - 1) % 3;
-        fft_lines<R, L, false, NT, NLINES, MapInterleaved<R, L, NLINES>, false, true>(
-            xb, tw_s, [&](int, int pos) { return src[pos * (N * H)]; }, PrepNone{},
-            [&](int, int pos, double2 v) {
-              const int ix = unpad_pos(pos, N, L);
-              if (ix < 0) return;
-              v = make_double2(v.x * wgt, v.y * wgt);
-              double2* yp = acc + (p * N + ix) * NLINES + l;
-              if (c < 3) {
-                *yp = v;
-              } else {
-                double2* yq = acc + (q * N + ix) * NLINES + l;
-                const double kx = kx_s[ix];
-                const double kp = c == 3 ? kz : c == 4 ? kx : ky, kq = c == 3 ? ky : c == 4 ? kz : kx;
-                const double2 a1 = *yp, a2 = *yq;
-                *yp = make_double2(fma(-kp, v.y, a1.x), fma(kp, v.x, a1.y));
-                *yq = make_double2(fma(kq, v.y, a2.x), fma(-kq, v.x, a2.y));
-              }
-            });
-      }
-    } else {
     sfor<6>([&](auto cc) {
       constexpr int C = decltype(cc)::value;
       if (C > 0) __syncthreads();   // xb is reused
@@ -465,7 +433,6 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
             }
           });
     });
-    }
   }
   __syncthreads();
 #pragma unroll 1
@@ -478,6 +445,40 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
     const int kxi = signed_k(ix, N), kyi = signed_k(iy, N);
     C2<R> y[3] = {acc[e], acc[N * NLINES + e], acc[2 * N * NLINES + e]};
     adj_stage_apply<R>(a.st, ((size_t)ix * N + iy) * H + z, kxi * kxi + kyi * kyi + z * z, y);
+  }
+}
+
+// A5 in the FP64 form: k_lines<OpXFwdTrunc> on the six fields, then this kernel,
+// y = w_M (a_bar + i k x o_bar) / N^3 (curl: spectral_ops.rs:92-104) and the
+// adjoint stage mode by mode (the split of P5, for the same reason).
+template <int N>
+__global__ void __launch_bounds__(StageGrid<double, N>::NT, StageGrid<double, N>::MB)
+k_adj_stage_f64(A5Args<double> a) {
+  constexpr int H = N / 2 + 1, NT = StageGrid<double, N>::NT, PER = StageGrid<double, N>::PER;
+  constexpr int TOTAL = N * N * H;
+  __shared__ double kxy[N], kz_s[H];
+  for (int i = threadIdx.x; i < N; i += NT) kxy[i] = a.ks * (double)signed_k(i, N);
+  for (int i = threadIdx.x; i < H; i += NT) kz_s[i] = a.ks * (double)i;
+  __syncthreads();
+  const int end = min((int)(blockIdx.x + 1) * PER, TOTAL);
+#pragma unroll 1
+  for (unsigned e = blockIdx.x * PER + threadIdx.x; e < (unsigned)end; e += NT) {
+    double2 f[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) f[c] = a.in[(size_t)c * a.fsin + e];
+    const unsigned row = e / (unsigned)H;
+    const int z = (int)(e - row * H), iy = (int)(row % N), ix = (int)(row / N);
+    const double kx = kxy[ix], ky = kxy[iy], kz = kz_s[z];
+    const double w = a.s_out * (z == 0 ? 1.0 : 2.0);
+    // i k x o = i (ky o_z - kz o_y, kz o_x - kx o_z, kx o_y - ky o_x)
+    const auto curl = [](double2 v, double p, double2 g, double q, double2 h) {   // v + i (p g - q h)
+      return make_double2(fma(q, h.y, fma(-p, g.y, v.x)), fma(-q, h.x, fma(p, g.x, v.y)));
+    };
+    double2 y[3] = {curl(f[0], ky, f[5], kz, f[4]), curl(f[1], kz, f[3], kx, f[5]), curl(f[2], kx, f[4], ky, f[3])};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = make_double2(w * y[c].x, w * y[c].y);
+    const int kxi = signed_k(ix, N), kyi = signed_k(iy, N);
+    adj_stage_apply<double>(a.st, e, kxi * kxi + kyi * kyi + z * z, y);
   }
 }
 

@@ -157,7 +157,7 @@ struct vk_ctx {
   int red_blocks = 0;
   int n_shells = 0;
   double* dspec = nullptr;
-  // diagnostics fused into the final stage of a step (partial rows of k_p5)
+  // diagnostics fused into the final stage of a step (partial rows of k_stage)
   double* dpart = nullptr;
   int dpart_rows = 0;
   int diag_valid = 0;                 // DiagBits the rows hold for the current state
@@ -653,7 +653,7 @@ int vk_create(const vk_config* cfg, vk_ctx** out) {
   if ((e = cudaMalloc(&c->part, (size_t)c->red_blocks * width * sizeof(double))) != cudaSuccess)
     return bail(e, "cudaMalloc(partials)");
   if ((e = cudaMalloc(&c->dspec, width * sizeof(double))) != cudaSuccess) return bail(e, "cudaMalloc(spectrum)");
-  c->dpart_rows = vk::p5_ctas(n, c->fp32);   // rows of k_p5 at this grid
+  c->dpart_rows = vk::p5_ctas(n, c->fp32);   // rows of k_stage at this grid
   if ((e = cudaMalloc(&c->dpart, (size_t)c->dpart_rows * (4 + c->n_shells) * sizeof(double))) != cudaSuccess)
     return bail(e, "cudaMalloc(fused diagnostics)");
   // the twiddle tables' copies (pageable memory, legacy stream)

@@ -231,25 +231,22 @@ inline cudaError_t nle_n(const NleParams<R>& p, cudaStream_t s) {
   }
   {
     TimerScope ts(p.timer, PASS_P5, s);
-    constexpr int NL = P5Lines<R, M>::value;
-    constexpr int NT = p5_threads<R, M, NL>();
-    const int nlines = N * H;
-    const bool diag = p.st.diag != 0;
-    const size_t smem = (size_t)(rsmem_elems<R, M, NL>() + 3 * N * NL) * sizeof(C2<R>) +
-                        (diag ? (size_t)p.st.nsh * sizeof(double) : 0);
+    const size_t fsA5 = (size_t)N * N * H;
+    OpXFwdTrunc<R, N, M> o{3, H, N, M, p.bufB, fsB4, p.bufA, fsA5};
+    e = launch_lines<R, M, false, true>(o, N, p.twM, s);
+    if (e != cudaSuccess) return e;
     const double scale = (double)M * M * M / ((double)N * N * N);
-    P5Args<R> a{N, M, H, nlines, (R)(1.0 / scale), ks, p.bufB, fsB4, p.st};
-    const int ntiles = (nlines + NL - 1) / NL;
-    if (diag) {
-      constexpr auto kern = k_p5<R, M, NL, NT, true>;
+    P5Args<R> a{(R)(1.0 / scale), ks, p.bufA, fsA5, p.st};
+    constexpr int NT = StageGrid<R, N>::NT;
+    const int nb = p5_ctas(N, sizeof(R) == 4);
+    if (p.st.diag != 0) {
+      const size_t smem = (size_t)p.st.nsh * sizeof(double);
+      constexpr auto kern = k_stage<R, N, true>;
       e = prepare_kernel<kern>(smem);
       if (e != cudaSuccess) return e;
-      kern<<<ntiles, NT, smem, s>>>(a, p.twM);
+      kern<<<nb, NT, smem, s>>>(a);
     } else {
-      constexpr auto kern = k_p5<R, M, NL, NT, false>;
-      e = prepare_kernel<kern>(smem);
-      if (e != cudaSuccess) return e;
-      kern<<<ntiles, NT, smem, s>>>(a, p.twM);
+      k_stage<R, N, false><<<nb, NT, 0, s>>>(a);
     }
     e = cudaGetLastError();
   }
@@ -305,7 +302,16 @@ inline cudaError_t nla_n(const NlaParams<R>& p, cudaStream_t s) {
     e = launch_lines<R, M, false>(o, M, p.twM, s);
     if (e != cudaSuccess) return e;
   }
-  {
+  if constexpr (sizeof(R) == 8) {
+    TimerScope ts(p.timer, PASS_A5, s);
+    const size_t fsA5 = (size_t)N * N * H;
+    OpXFwdTrunc<R, N, M> o{6, H, N, M, p.bufB, fsB4, p.bufA, fsA5};
+    e = launch_lines<R, M, false, true>(o, N, p.twM, s);
+    if (e != cudaSuccess) return e;
+    A5Args<R> a{N, M, H, N * H, (R)(1.0 / ((double)N * N * N)), ks, p.bufA, fsA5, p.st};
+    k_adj_stage_f64<N><<<p5_ctas(N, false), StageGrid<double, N>::NT, 0, s>>>(a);
+    e = cudaGetLastError();
+  } else {
     TimerScope ts(p.timer, PASS_A5, s);
     constexpr int NL = A5Lines<R>::value;
     constexpr int NT = cmin(rthreads<R, M, NL>(), 384);

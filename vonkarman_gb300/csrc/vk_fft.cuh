@@ -364,7 +364,9 @@ __device__ __forceinline__ void dft(C2<R>* v, const C2<R>* w) {
 // one padding element per 128-byte row of the line: 8 complex doubles or 16
 // complex floats
 template <typename R> __host__ __device__ constexpr int zrow() { return 128 / (2 * (int)sizeof(R)); }
-template <typename R> __host__ __device__ constexpr int zi(int p) { return p + p / zrow<R>(); }
+template <typename R> __host__ __device__ constexpr int zi(int p) {   // p >= 0
+  return p + (int)((unsigned)p / (unsigned)zrow<R>());
+}
 template <typename R> __host__ __device__ constexpr int zpad_len(int L) { return L + L / zrow<R>(); }
 
 }  // namespace vk

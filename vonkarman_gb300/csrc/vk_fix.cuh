@@ -323,11 +323,15 @@ template <bool INV> struct FxDft<12, INV> {
 // left-aligned at bit 62, shifted right by K - exponent.  Zeros (and
 // denormals, far below the quantum of a line of normal range) shift out.
 VK_FIX_HD long long fx_from_double(int hi, int lo, int k) {
-  const int e = (hi >> 20) & 0x7ff;
+  // k - exponent, from the sign-cleared high word (its mantissa bits add less than one)
+  const int r = ((k << 20) + 0xfffff - (hi & 0x7fffffff)) >> 20;
   const unsigned mh = ((((unsigned)hi << 10) | ((unsigned)lo >> 22)) & 0x3fffffffu) | 0x40000000u;
   unsigned long long m = ((unsigned long long)mh << 32) | ((unsigned)lo << 10);
-  const int r = k - e;
-  m >>= r < 63 ? r : 63;   // m < 2^63
+#ifdef __CUDA_ARCH__
+  asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(m), "r"(r));   // clamps at 64
+#else
+  m = r > 63 ? 0ull : m >> r;
+#endif
   const long long s = (long long)(hi >> 31);
   return ((long long)m ^ s) - s;
 }

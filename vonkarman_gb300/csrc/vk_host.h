@@ -74,9 +74,8 @@ template <typename R> struct StageArgs {
   double ks;                       // 2 pi / L (shells of boxes other than 2 pi)
 };
 
-// Modes per CTA of the final pass (k_p5: N / 2 + 1 consecutive z per x line,
-// lines tiled by this many) and its CTA count, which sizes the fused
-// diagnostics' partial rows.
+// CTA size of the stage epilogue (k_stage): p5_lines(n) n consecutive modes per
+// CTA; its CTA count sizes the fused diagnostics' partial rows.
 inline constexpr int p5_lines(int n, bool fp32) { return (void)n, fp32 ? 8 : 4; }
 inline constexpr int p5_ctas(int n, bool fp32) { return (n * (n / 2 + 1) + p5_lines(n, fp32) - 1) / p5_lines(n, fp32); }
 enum DiagBits : int { DIAG_TIER1 = 1, DIAG_SPECTRUM = 2 };

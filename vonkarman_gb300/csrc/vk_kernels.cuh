@@ -210,6 +210,26 @@ template <typename R, int GN = 0, int GM = 0> struct OpYFwdTrunc {
   }
 };
 
+// First half of P5 in the FP64 form: x-forward of the cross-product fields, keep
+// N of M modes.
+template <typename R, int GN = 0, int GM = 0> struct OpXFwdTrunc {
+  int nfields, hz;
+  int N, M;
+  const C2<R>* in; size_t fsin;   // (M, N, H)
+  C2<R>* out; size_t fsout;       // (N, N, H)
+  static constexpr int NKIND = 1;
+  VK_GRID_DIMS(GN, GM)
+  __host__ __device__ __forceinline__ int kind(int) const { return 0; }
+  template <int K> __device__ __forceinline__ C2<R> load(int f, int iy, int z, int p) const {
+    return in[(size_t)f * fsin + ((p * n_() + iy) * h_() + z)];
+  }
+  template <int K> __device__ __forceinline__ C2<R> prep(int, int, int, int, C2<R> v) const { return v; }
+  __device__ __forceinline__ int out_index(int p) const { return unpad_pos(p, n_(), m_()); }
+  __device__ __forceinline__ void store(int f, int iy, int z, int i, C2<R> v) const {
+    out[(size_t)f * fsout + ((i * n_() + iy) * h_() + z)] = v;
+  }
+};
+
 // Standalone FFT backend: C2C along x (AXIS 0) or y (AXIS 1) of an
 // (nx, ny, hz) complex array, in place.
 template <typename R, int AXIS> struct OpPlainC2C {
@@ -444,7 +464,6 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 // the mode's global reads, apply() the arithmetic and the stores.
 struct StageF64 {
   struct Mode {
-    bool ok;
     int m;
     size_t idx;
     double ik2;                       // 1 / |k|^2, 0 at k = 0
@@ -461,7 +480,6 @@ struct StageF64 {
     for (int c = 0; c < 3; ++c) v[c] = p[c * s.cs + md.idx];
   }
   __device__ __forceinline__ void load(Mode& md) const {
-    if (!md.ok) return;
     const double* e = s.etd + (size_t)md.m * ETD_STRIDE;
     md.ik2 = e[E_IK2];
     if (s.op == ST_NL_OUT) return;

@@ -1,6 +1,6 @@
 // Register-resident batched line FFT and the pass kernels built on it
-// (k_lines: strided x / y passes; k_p5: x-forward with the stage epilogue;
-// k_p3: the z pass with the cross product; k_nz_max: the N-grid z pass).
+// (k_lines: strided x / y passes; k_stage: the stage epilogue; k_p3, k_p3x: the
+// z pass with the cross product; k_nz_max: the N-grid z pass).
 //
 // NLINES lines of length L are transformed by a Stockham auto-sort whose
 // stages live in registers: the first stage reads its butterfly inputs
@@ -153,6 +153,7 @@ struct MapInterleaved {
   template <int NB> __device__ __forceinline__ static int line(int g) { return g % NLINES; }
   template <int NB> __device__ __forceinline__ static int bfly(int g) { return g / NLINES; }
   template <int S> __device__ __forceinline__ static int idx(int pos, int l) { return ridx<R, L, NLINES, S>(pos, l); }
+  template <int STEP, int BASE> __device__ __forceinline__ static int step(int, int r) { return r * STEP * NLINES; }
   static constexpr int elems() { return rsmem_elems<R, L, NLINES>(); }
 };
 // Contiguous lines (z passes, element p of line l at l * LP + zi(p), one
@@ -165,6 +166,12 @@ struct MapContig {
   template <int NB> __device__ __forceinline__ static int bfly(int g) { return g % NB; }
   template <int S> __device__ __forceinline__ static int idx(int pos, int l) { return l * zpad_len<R>(L) + zi<R>(pos); }
   static constexpr int elems() { return NLINES * zpad_len<R>(L); }
+  // offset of position pos + r STEP from that of pos (BASE divides pos): a
+  // constant where whole padding rows are stepped over, or none is left
+  template <int STEP, int BASE> __device__ __forceinline__ static int step(int pos, int r) {
+    return STEP % zrow<R>() == 0 || (BASE % zrow<R>() == 0 && (r + 1) * STEP <= zrow<R>())
+               ? zi<R>(r * STEP) : zi<R>(pos + r * STEP) - zi<R>(pos);
+  }
 };
 
 // Inputs of the first stage at positions p in [Z0, Z1) are known to be zero
@@ -431,18 +438,19 @@ struct FxLines {
         }
       }
       if (MAP::CONTIG && j0 == 0) line_s[l0] = pack_state(q, code);
-      first_dft(v, [&](int p, fx2 z) { xb[MAP::template idx<0>(p, l0)] = z; }, j0);
+      fx2* dst = xb + MAP::template idx<0>(j0 * R0, l0);
+      first_dft(v, [&](int r, fx2 z) { dst[MAP::template step<1, R0>(j0 * R0, r)] = z; });
     }
     return State{q, code};
   }
-  // first-stage butterfly j: put(position, value) into the exchange
+  // a first-stage butterfly: put(r, value) into the exchange
   template <class PUT>
-  __device__ __forceinline__ static void first_dft(fx2* v, const PUT& put, int j) {
+  __device__ __forceinline__ static void first_dft(fx2* v, const PUT& put) {
     FxDft<R0, INV>::run(v);
     sfor<R0>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
       if constexpr (r == 0) v[r] = fx_multiple<GN>(v[r]);
-      put(j * R0 + r, v[r]);
+      put(r, v[r]);
     });
   }
   // twiddles and DFT of a later stage's butterfly: twiddle index k of ns
@@ -468,16 +476,19 @@ struct FxLines {
     if (act) {
       __builtin_assume(j >= 0 && j < NBM);
       __builtin_assume(l >= 0 && l < NLINES);
+      const fx2* src = xb + MAP::template idx<0>(j, l);
 #pragma unroll
-      for (int r = 0; r < RM; ++r) u[r] = xb[MAP::template idx<0>(j + r * NBM, l)];
+      for (int r = 0; r < RM; ++r) u[r] = src[MAP::template step<NBM, 1>(j, r)];
     }
     __syncthreads();
     if (act) {
       const int k = j % R0;
       later_dft<RM, 0>(u, tw, k, R0);
       u[0] = fx_multiple<GR>(u[0]);
+      const int p0 = (j - k) * RM + k;
+      fx2* dst = xb + MAP::template idx<0>(p0, l);
 #pragma unroll
-      for (int r = 0; r < RM; ++r) xb[MAP::template idx<0>((j - k) * RM + k + r * R0, l)] = u[r];
+      for (int r = 0; r < RM; ++r) dst[MAP::template step<R0, 1>(p0, r)] = u[r];
     }
     __syncthreads();
   }
@@ -491,16 +502,19 @@ struct FxLines {
     const bool act = l < nl;
     fx2 u[RM];
     if (act) {
+      const fx2* src = xs + l * ls + zi<double>(j);
 #pragma unroll
-      for (int r = 0; r < RM; ++r) u[r] = xs[l * ls + zi<double>(j + r * NBM)];
+      for (int r = 0; r < RM; ++r) u[r] = src[MAP::template step<NBM, 1>(j, r)];
     }
     __syncthreads();
     if (act) {
       const int k = j % R0;
       later_dft<RM, 0>(u, tw, k, R0);
       u[0] = fx_multiple<GR>(u[0]);
+      const int p0 = (j - k) * RM + k;
+      fx2* dst = xs + l * ls + zi<double>(p0);
 #pragma unroll
-      for (int r = 0; r < RM; ++r) xs[l * ls + zi<double>((j - k) * RM + k + r * R0)] = u[r];
+      for (int r = 0; r < RM; ++r) dst[MAP::template step<R0, 1>(p0, r)] = u[r];
     }
     __syncthreads();
   }
@@ -527,8 +541,9 @@ struct FxLines {
         __builtin_assume(j >= 0 && j < NB1);
         __builtin_assume(l >= 0 && l < NLINES);
         if (MAP::CONTIG) st = unpack_state(line_s[l]);
+        const fx2* src = xb + MAP::template idx<0>(j, l);
 #pragma unroll
-        for (int r = 0; r < R1; ++r) u[r] = xb[MAP::template idx<0>(j + r * NB1, l)];
+        for (int r = 0; r < R1; ++r) u[r] = src[MAP::template step<NB1, 1>(j, r)];
       }
       if constexpr (SL) __syncthreads();
       if (act) {
@@ -552,8 +567,9 @@ struct FxLines {
       const bool act = lr < RL && l < nl;
       fx2 u[R1];
       if (act) {
+        const fx2* src = xs + l * ls + zi<double>(j);
 #pragma unroll
-        for (int r = 0; r < R1; ++r) u[r] = xs[l * ls + zi<double>(j + r * NB1)];
+        for (int r = 0; r < R1; ++r) u[r] = src[MAP::template step<NB1, 1>(j, r)];
       }
       __syncthreads();
       if (act) {
@@ -750,235 +766,173 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
 }
 
 // ---------------------------------------------------------------------------
-// P5: x-forward of the three cross-product fields, keep N of M modes, scale
-// N^3/M^3 (dealiased.rs:102-109), Leray projection (spectral_ops.rs:114-151)
-// and the stage epilogue.  A CTA takes NLINES consecutive (iy, z) lines; the
-// fields are transformed one after another into shared memory (kept modes
-// only), then the epilogue runs over the CTA's N x NLINES modes with
-// consecutive lanes on consecutive z.
+// P5 is two kernels: k_lines<OpXFwdTrunc> (x-forward of the three cross-product
+// fields, keep N of M modes) and k_stage, mode by mode: scale N^3/M^3
+// (dealiased.rs:102-109), Leray projection (spectral_ops.rs:114-151) and the
+// stage epilogue.  Fused, one CTA held the transform's and the epilogue's
+// registers and the kept modes of three fields in shared memory and ran the two
+// one after the other at 12 to 24 warps per SM.  Apart they cost one more write
+// and read of the three fields (6 N^2 H elements) and are faster: FP64 (FP64
+// pipe, about 38 operations per mode) N = 256 1.09 -> 0.98 ms, N = 128 0.164 ->
+// 0.140, N = 64 0.037 -> 0.031; FP32 (memory) N = 512 3.04 -> 2.37, N = 256
+// 0.294 -> 0.261, N = 128 0.043 -> 0.041.
 // ---------------------------------------------------------------------------
 template <typename R> struct P5Args {
-  int N, M, H, nlines;
   R s_out, ks;
-  const C2<R>* in; size_t fsin;   // (M, N, H)
+  const C2<R>* in; size_t fsin;   // (N, N, H), kept modes
   StageArgs<R> st;
 };
 
-// lines per CTA of k_p5 at padded length L (the grid N = 2 L / 3), shared
-// with the host's sizing of the fused-diagnostics rows
-template <typename R, int L> struct P5Lines { static constexpr int value = p5_lines(2 * L / 3, sizeof(R) == 4); };
-// Threads of k_p5: one butterfly per thread in the widest FFT stage; FP32 up
-// to 384 points doubles them (measured 4 % faster at 384: the epilogue keeps
-// the same modes in flight per CTA with one mode per thread, and twice the
-// warps hide its arithmetic), two CTAs per SM.  FP64 takes at least 128, for
-// its epilogue, and as many CTAs as shared memory allows (three at 384 points).
-template <typename R, int L, int NLINES>
-__host__ __device__ constexpr int p5_threads() {
-  return sizeof(R) == 8 ? cmax(128, rthreads<R, L, NLINES>())
-       : L <= 384 ? cmin(2 * rthreads<R, L, NLINES>(), 384) : cmin(rthreads<R, L, NLINES>(), 384);
-}
-template <typename R, int L, int NLINES, int NT>
-__host__ __device__ constexpr int p5_min_blocks() {
-  return sizeof(R) == 8 ? (L >= 768 ? 1 : 3)
-       : NT >= 2 * rthreads<R, L, NLINES>() ? 2 : lines_min_blocks<R, L, NT, true>();
-}
-
-// DIAG: the instance for final stages whose new state also feeds the fused
-// diagnostics (a.st.diag bits): per thread FP64 sums of the Tier-1 terms and a
-// per-CTA FP64 shell histogram in shared memory (nsh doubles after the FFT
-// buffers), written as row blockIdx.x of a.st.dpart; the rows are added by the
-// Neumaier column reduction, as the separate reduction passes do.
-template <typename R, int L, int NLINES, int NT, bool DIAG = false>
-__global__ void __launch_bounds__(NT, p5_min_blocks<R, L, NLINES, NT>())
-k_p5(P5Args<R> a, const C2<R>* __restrict__ tw) {
-  constexpr int N = 2 * L / 3;
-  static_assert(NT % NLINES == 0, "a thread keeps one line in every stage");
-  extern __shared__ __align__(16) unsigned char vk_smem[];
-  __shared__ C2<R> tw_s[twtab_elems<R, false>(L)];
-  load_twtab<R, L, false, NT>(tw_s, tw);
-  C2<R>* xb = reinterpret_cast<C2<R>*>(vk_smem);
-  C2<R>* keep = xb + rsmem_elems<R, L, NLINES>();   // 3 fields x N x NLINES
-  constexpr int H = N / 2 + 1;   // a.H of the launch
-  double* hist = reinterpret_cast<double*>(keep + 3 * N * NLINES);   // DIAG: nsh shells
-  const bool d_t1 = DIAG && (a.st.diag & DIAG_TIER1);
-  const bool d_sp = DIAG && (a.st.diag & DIAG_SPECTRUM);
-  if constexpr (DIAG) {
-    if (d_sp)
-      for (int i = threadIdx.x; i < a.st.nsh; i += NT) hist[i] = 0.0;   // ordered by the FFTs' barriers
-  }
-  double dsum[4] = {0.0, 0.0, 0.0, 0.0};
-  const bool ks_one = a.st.ks == 1.0;
-  {
-    const int lam = blockIdx.x * NLINES + (int)(threadIdx.x % NLINES);
-    const bool ok = lam < a.nlines;
-    const int iy = ok ? lam / H : 0;
-    const int z = ok ? lam - iy * H : 0;
-    if constexpr (sizeof(R) == 8) {
-      // (a loop, not unrolled: the FP64 transform's code is large)
-#pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        if (c > 0) __syncthreads();   // xb is reused
-        const C2<R>* src = a.in + (size_t)c * a.fsin + (iy * H + z);
-        fft_lines<R, L, false, NT, NLINES, MapInterleaved<R, L, NLINES>, false, true>(
-            xb, tw_s, [&](int, int p) { return src[p * (N * H)]; }, PrepNone{},
-            [&](int, int p, C2<R> v) {
-              const int ix = unpad_pos(p, N, L);
-              if (ix >= 0) keep[(c * N + ix) * NLINES + (int)(threadIdx.x % NLINES)] = v;
-            });
-      }
-    } else {
-    sfor<3>([&](auto cc) {
-      constexpr int C = decltype(cc)::value;
-      if (C > 0) __syncthreads();   // xb is reused
-      const C2<R>* src = a.in + (size_t)C * a.fsin + (iy * H + z);
-      fft_lines<R, L, false, NT, NLINES, MapInterleaved<R, L, NLINES>, false, true>(
-          xb, tw_s, [&](int, int p) { return src[p * (N * H)]; }, PrepNone{},
-          [&](int, int p, C2<R> v) {
-            const int ix = unpad_pos(p, N, L);
-            if (ix >= 0) keep[(C * N + ix) * NLINES + (int)(threadIdx.x % NLINES)] = v;
-          });
-    });
+// The CTA's row of the fused diagnostics: Tier-1 sums by a fixed shuffle /
+// warp-order tree, then the shell histogram.
+template <int NT, typename R>
+__device__ __forceinline__ void diag_row(const StageArgs<R>& st, bool d_t1, bool d_sp, const double* dsum,
+                                         const double* hist) {
+  __shared__ double wsum[4][NT / 32];
+  const bool has_row = (int)blockIdx.x < st.dpart_rows;
+  double* row = st.dpart + (size_t)(has_row ? blockIdx.x : 0) * (4 + st.nsh);
+  if (d_t1) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double v = dsum[j];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) == 0) wsum[j][threadIdx.x / 32] = v;
     }
   }
   __syncthreads();
+  if (d_t1 && has_row && threadIdx.x < 4) {
+    double v = 0.0;
+    for (int w = 0; w < NT / 32; ++w) v += wsum[threadIdx.x][w];
+    row[threadIdx.x] = v;
+  }
+  if (d_sp && has_row)
+    for (int i = threadIdx.x; i < st.nsh; i += NT) row[4 + i] = hist[i];
+}
+
+// Modes and threads per CTA of k_stage: CTA b takes modes [b, b + 1) PER of the
+// (N, N, H) array (p5_ctas CTAs, which also sizes the diagnostics' rows).
+template <typename R, int N> struct StageGrid {
+  // modes per thread and iteration: FP32 keeps the loads of two in flight (N =
+  // 256 0.286 -> 0.261 ms), FP64 has no registers for it (0.978 -> 1.006 ms)
+  static constexpr int EM = sizeof(R) == 4 ? 2 : 1;
+  static constexpr int PER = p5_lines(N, sizeof(R) == 4) * N;
+  static constexpr int NT = cmin(256, cmax(32, PER / EM));
+  static constexpr int MB = cmin(16, 768 / NT);   // 84 registers
+};
+
+// DIAG: the instance for final stages whose new state also feeds the fused
+// diagnostics (a.st.diag bits): per thread FP64 sums of the Tier-1 terms and a
+// per-CTA FP64 shell histogram in shared memory (nsh doubles), written as row
+// blockIdx.x of a.st.dpart; the rows are added by the Neumaier column reduction,
+// as the separate reduction passes do.
+template <typename R, int N, bool DIAG>
+__global__ void __launch_bounds__(StageGrid<R, N>::NT, DIAG ? 1 : StageGrid<R, N>::MB) k_stage(P5Args<R> a) {
+  constexpr int H = N / 2 + 1, NT = StageGrid<R, N>::NT, PER = StageGrid<R, N>::PER, EM = StageGrid<R, N>::EM;
+  constexpr int TOTAL = N * N * H;
+  __shared__ R kxy[N], kz_s[H];   // wave numbers (their conversion is an FP64 operation in the FP64 form)
+  extern __shared__ __align__(16) unsigned char vk_smem[];
+  double* hist = reinterpret_cast<double*>(vk_smem);   // DIAG: nsh shells
+  const bool d_t1 = DIAG && (a.st.diag & DIAG_TIER1);
+  const bool d_sp = DIAG && (a.st.diag & DIAG_SPECTRUM);
+  for (int i = threadIdx.x; i < N; i += NT) kxy[i] = a.ks * (R)signed_k(i, N);
+  for (int i = threadIdx.x; i < H; i += NT) kz_s[i] = a.ks * (R)i;
+  if (d_sp)
+    for (int i = threadIdx.x; i < a.st.nsh; i += NT) hist[i] = 0.0;
+  __syncthreads();
+  double dsum[4] = {0.0, 0.0, 0.0, 0.0};
+  const bool ks_one = a.st.ks == 1.0;
+  const int end = min((int)(blockIdx.x + 1) * PER, TOTAL);
+  // diagnostics of a new mode u at (kx, ky, z)
+  const auto diag = [&](int kx, int ky, int z, const C2<R>* u) {
+    const R w = (z == 0 || z == N / 2) ? R(1) : R(2);   // R2C weight, exact in R
+    if (d_t1) {
+      R e, en, he, sh;
+      tier1_terms<R>(a.ks * (R)kx, a.ks * (R)ky, a.ks * (R)z, u, e, en, he, sh);
+      dsum[0] += (double)(w * e); dsum[1] += (double)(w * en);
+      dsum[2] += (double)(w * he); dsum[3] += (double)(w * sh);
+    }
+    if (d_sp) {
+      const int shell = shell_of(kx, ky, z, a.st.ks, ks_one);
+      if (shell < a.st.nsh) atomicAdd(&hist[shell], (double)(w * spectrum_term<R>(u)));
+    }
+  };
+  const auto locate = [](unsigned i, int& ix, int& iy, int& z) {
+    const unsigned row = i / (unsigned)H;
+    z = (int)(i - row * H);
+    iy = (int)(row % N);
+    ix = (int)(row / N);
+  };
   if constexpr (sizeof(R) == 8) {
-    // two modes per iteration with 128 threads, so that the loads of both are in flight together
-    constexpr int EM = NT > 128 ? 1 : 2;
-    const int l = threadIdx.x % NLINES;
-    const int lam = blockIdx.x * NLINES + l;
-    const bool line_ok = lam < a.nlines;
-    const int iy = line_ok ? lam / H : 0;
-    const int z = line_ok ? lam - iy * H : 0;
-    const int kyi = signed_k(iy, N);
-    const double ky = a.ks * (double)kyi, kz = a.ks * (double)z;
-    const double w = (z == 0 || z == N / 2) ? 1.0 : 2.0;   // R2C weight
-    StageF64 stage(a.st, a.s_out);
+    const StageF64 stage(a.st, a.s_out);
 #pragma unroll 1
-    for (int ix0 = threadIdx.x / NLINES; ix0 < N; ix0 += EM * (NT / NLINES)) {
-      StageF64::Mode md[EM];
+    for (int e = blockIdx.x * PER + threadIdx.x; e < end; e += NT) {
+      int ix, iy, z;
+      locate(e, ix, iy, z);
+      const int kxi = signed_k(ix, N), kyi = signed_k(iy, N);
+      StageF64::Mode md;
+      md.idx = e;
+      md.m = kxi * kxi + kyi * kyi + z * z;
+      stage.load(md);
+      double2 v[3];
 #pragma unroll
-      for (int q = 0; q < EM; ++q) {
-        const int ix = ix0 + q * (NT / NLINES);
-        const int kxi = signed_k(ix < N ? ix : 0, N);
-        md[q].ok = line_ok && ix < N;
-        md[q].idx = ((size_t)(ix < N ? ix : 0) * N + iy) * H + z;
-        md[q].m = kxi * kxi + kyi * kyi + z * z;
-        stage.load(md[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < EM; ++q) {
-        if (!md[q].ok) continue;
-        const int ix = ix0 + q * (NT / NLINES);
-        const int e = ix * NLINES + l;
-        const int kxi = signed_k(ix, N);
-        const double kx = a.ks * (double)kxi;
-        const double2 x = keep[e], y = keep[N * NLINES + e], v = keep[2 * N * NLINES + e];
-        const double dr = fma(kz, v.x, fma(ky, y.x, kx * x.x)) * md[q].ik2;
-        const double di = fma(kz, v.y, fma(ky, y.y, kx * x.y)) * md[q].ik2;
-        const double2 nl[3] = {make_double2(fma(-kx, dr, x.x), fma(-kx, di, x.y)),
-                               make_double2(fma(-ky, dr, y.x), fma(-ky, di, y.y)),
-                               make_double2(fma(-kz, dr, v.x), fma(-kz, di, v.y))};
-        double2 un[3];
-        stage.apply(md[q], nl, un);
-        if constexpr (DIAG) {
-          if (d_t1) {
-            double te, en, he, sh;
-            tier1_terms<double>(kx, ky, kz, un, te, en, he, sh);
-            dsum[0] += w * te; dsum[1] += w * en; dsum[2] += w * he; dsum[3] += w * sh;
-          }
-          if (d_sp) {
-            const int shell = shell_of(kxi, kyi, z, a.st.ks, ks_one);
-            if (shell < a.st.nsh) atomicAdd(&hist[shell], w * spectrum_term<double>(un));
-          }
-        }
-      }
+      for (int c = 0; c < 3; ++c) v[c] = a.in[(size_t)c * a.fsin + e];
+      const double kx = kxy[ix], ky = kxy[iy], kz = kz_s[z];
+      const double dr = fma(kz, v[2].x, fma(ky, v[1].x, kx * v[0].x)) * md.ik2;
+      const double di = fma(kz, v[2].y, fma(ky, v[1].y, kx * v[0].y)) * md.ik2;
+      const double2 nl[3] = {make_double2(fma(-kx, dr, v[0].x), fma(-kx, di, v[0].y)),
+                             make_double2(fma(-ky, dr, v[1].x), fma(-ky, di, v[1].y)),
+                             make_double2(fma(-kz, dr, v[2].x), fma(-kz, di, v[2].y))};
+      double2 un[3];
+      stage.apply(md, nl, un);
+      if constexpr (DIAG) diag(kxi, kyi, z, un);
     }
   } else {
-  // FP32 with the FFT's thread count: two modes per iteration, so that the
-  // epilogue's loads of both are in flight together (doubled threads keep one)
-  constexpr int EM = NT < 2 * rthreads<R, L, NLINES>() ? 2 : 1;
 #pragma unroll 1
-  for (int e0 = threadIdx.x; e0 < N * NLINES; e0 += EM * NT) {
-    size_t idx[EM];
-    int mm[EM];
-    R kk[EM];
-    C2<R> nl[EM][3];
-    bool ok[EM];
-    int kxq[EM], kyq[EM], kzq[EM];
-#pragma unroll
-    for (int q = 0; q < EM; ++q) {
-      const int e = e0 + q * NT;
-      const int ix = e / NLINES, l = e % NLINES;
-      const int lam = blockIdx.x * NLINES + l;
-      ok[q] = e < N * NLINES && lam < a.nlines;
-      const int iy = ok[q] ? lam / H : 0;
-      const int z = ok[q] ? lam - iy * H : 0;
-      const int kxi = signed_k(ok[q] ? ix : 0, N), kyi = signed_k(iy, N);
-      const R kx = a.ks * (R)kxi, ky = a.ks * (R)kyi, kz = a.ks * (R)z;
-      const int ee = ok[q] ? e : 0;
-      nl[q][0] = cscale<R>(keep[ee], a.s_out);
-      nl[q][1] = cscale<R>(keep[N * NLINES + ee], a.s_out);
-      nl[q][2] = cscale<R>(keep[2 * N * NLINES + ee], a.s_out);
-      const R k2 = (kx * kx + ky * ky) + kz * kz;
-      if (!(k2 < R(1e-30))) {
-        const R inv = R(1) / k2;
-        const C2<R> kd = cmk<R>((kx * nl[q][0].x + ky * nl[q][1].x) + kz * nl[q][2].x,
-                                (kx * nl[q][0].y + ky * nl[q][1].y) + kz * nl[q][2].y);
-        nl[q][0] = cmk<R>(nl[q][0].x - kx * kd.x * inv, nl[q][0].y - kx * kd.y * inv);
-        nl[q][1] = cmk<R>(nl[q][1].x - ky * kd.x * inv, nl[q][1].y - ky * kd.y * inv);
-        nl[q][2] = cmk<R>(nl[q][2].x - kz * kd.x * inv, nl[q][2].y - kz * kd.y * inv);
-      }
-      kk[q] = k2;
-      mm[q] = kxi * kxi + kyi * kyi + z * z;
-      idx[q] = ((size_t)(ok[q] ? ix : 0) * N + iy) * H + z;
-      kxq[q] = kxi; kyq[q] = kyi; kzq[q] = z;
-    }
-    if constexpr (!DIAG) {
-      stage_apply_n<R, EM>(a.st, idx, mm, kk, nl, ok);
-    } else {
-      C2<R> un[EM][3];
-      stage_apply_n<R, EM, true>(a.st, idx, mm, kk, nl, ok, un);
+    for (int e0 = blockIdx.x * PER + threadIdx.x; e0 < end; e0 += EM * NT) {
+      size_t idx[EM];
+      int mm[EM], ix[EM], iy[EM], z[EM];
+      R kk[EM];
+      C2<R> nl[EM][3];
+      bool ok[EM];
 #pragma unroll
       for (int q = 0; q < EM; ++q) {
-        if (!ok[q]) continue;
-        const R w = (kzq[q] == 0 || kzq[q] == N / 2) ? R(1) : R(2);   // R2C weight, exact in R
-        if (d_t1) {
-          R e, en, he, sh;
-          tier1_terms<R>(a.ks * (R)kxq[q], a.ks * (R)kyq[q], a.ks * (R)kzq[q], un[q], e, en, he, sh);
-          dsum[0] += (double)(w * e); dsum[1] += (double)(w * en);
-          dsum[2] += (double)(w * he); dsum[3] += (double)(w * sh);
-        }
-        if (d_sp) {
-          const int shell = shell_of(kxq[q], kyq[q], kzq[q], a.st.ks, ks_one);
-          if (shell < a.st.nsh) atomicAdd(&hist[shell], (double)(w * spectrum_term<R>(un[q])));
-        }
-      }
-    }
-  }
-  }
-  if constexpr (DIAG) {
-    // the CTA's row: Tier-1 sums by a fixed shuffle / warp-order tree, then
-    // the shell histogram
-    __shared__ double wsum[4][NT / 32];
-    const bool has_row = (int)blockIdx.x < a.st.dpart_rows;
-    double* row = a.st.dpart + (size_t)(has_row ? blockIdx.x : 0) * (4 + a.st.nsh);
-    if (d_t1) {
+        const int e = e0 + q * NT;
+        ok[q] = e < end;
+        idx[q] = ok[q] ? e : e0;
+        locate((unsigned)idx[q], ix[q], iy[q], z[q]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        double v = dsum[j];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) wsum[j][threadIdx.x / 32] = v;
+        for (int c = 0; c < 3; ++c) nl[q][c] = a.in[(size_t)c * a.fsin + idx[q]];
+      }
+#pragma unroll
+      for (int q = 0; q < EM; ++q) {
+        const int kxi = signed_k(ix[q], N), kyi = signed_k(iy[q], N);
+        const R kx = kxy[ix[q]], ky = kxy[iy[q]], kz = kz_s[z[q]];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) nl[q][c] = cscale<R>(nl[q][c], a.s_out);
+        const R k2 = (kx * kx + ky * ky) + kz * kz;
+        if (!(k2 < R(1e-30))) {
+          const R inv = R(1) / k2;
+          const C2<R> kd = cmk<R>((kx * nl[q][0].x + ky * nl[q][1].x) + kz * nl[q][2].x,
+                                  (kx * nl[q][0].y + ky * nl[q][1].y) + kz * nl[q][2].y);
+          nl[q][0] = cmk<R>(nl[q][0].x - kx * kd.x * inv, nl[q][0].y - kx * kd.y * inv);
+          nl[q][1] = cmk<R>(nl[q][1].x - ky * kd.x * inv, nl[q][1].y - ky * kd.y * inv);
+          nl[q][2] = cmk<R>(nl[q][2].x - kz * kd.x * inv, nl[q][2].y - kz * kd.y * inv);
+        }
+        kk[q] = k2;
+        mm[q] = kxi * kxi + kyi * kyi + z[q] * z[q];
+      }
+      if constexpr (!DIAG) {
+        stage_apply_n<R, EM>(a.st, idx, mm, kk, nl, ok);
+      } else {
+        C2<R> un[EM][3];
+        stage_apply_n<R, EM, true>(a.st, idx, mm, kk, nl, ok, un);
+#pragma unroll
+        for (int q = 0; q < EM; ++q)
+          if (ok[q]) diag(signed_k(ix[q], N), signed_k(iy[q], N), z[q], un[q]);
       }
     }
-    __syncthreads();
-    if (d_t1 && has_row && threadIdx.x < 4) {
-      double v = 0.0;
-      for (int w = 0; w < NT / 32; ++w) v += wsum[threadIdx.x][w];
-      row[threadIdx.x] = v;
-    }
-    if (d_sp && has_row)
-      for (int i = threadIdx.x; i < a.st.nsh; i += NT) row[4 + i] = hist[i];
   }
+  if constexpr (DIAG) diag_row<NT>(a.st, d_t1, d_sp, dsum, hist);
 }
 
 // ---------------------------------------------------------------------------
@@ -1190,17 +1144,29 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
 // one, both of which belong to that pair.
 // ---------------------------------------------------------------------------
 struct FxColumn {       // per column: left shifts (negative: right) of the lines' fields, exponent of the products
-  int s1, s2u, s2w, s3;
+  int s1, s2u, s2w, s3, smin;
   int e, code;
 };
+template <bool LEFT>   // s >= 0
 __device__ __forceinline__ long long fx_shl(long long v, int s) {   // v 2^s, rounded for s < 0
-  return s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
+  return LEFT || s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
 }
 // a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split): the
 // floors of the two products' cross terms cancel in the mean
 __device__ __forceinline__ long long fx_det(fxsplit a, fxsplit b, fxsplit c, fxsplit d) {
   const int t = fx_madhi(a.l, b.h, fx_madhi(a.h, b.l, 0)), u = fx_madhi(c.l, d.h, fx_madhi(c.h, d.l, 0));
   return fx_wide(a.h, b.h) - fx_wide(c.h, d.h) + (long long)(t - u);
+}
+// u x omega at one position of a column (parts exchanged), lines at stride ls
+template <bool LEFT>
+__device__ __forceinline__ void fx_cross(const fx2* x, int ls, const FxColumn& f, long long* c) {
+  const fx2 z1 = x[0], z2 = x[ls], z3 = x[2 * ls];
+  const fxsplit ux = fx_split(fx_shl<LEFT>(z1.y, f.s1)), uy = fx_split(fx_shl<LEFT>(z1.x, f.s1));
+  const fxsplit uz = fx_split(fx_shl<LEFT>(z2.y, f.s2u)), wx = fx_split(fx_shl<LEFT>(z2.x, f.s2w));
+  const fxsplit wy = fx_split(fx_shl<LEFT>(z3.y, f.s3)), wz = fx_split(fx_shl<LEFT>(z3.x, f.s3));
+  c[0] = fx_det(uy, wz, uz, wy);
+  c[1] = fx_det(uz, wx, ux, wz);
+  c[2] = fx_det(ux, wy, uy, wx);
 }
 // bits of a field whose high words' magnitudes OR to m, line exponent q
 __device__ __forceinline__ int fx_field_bits(int q, int m) { return q + 64 - __clz(m); }
@@ -1236,18 +1202,24 @@ __device__ __forceinline__ void p3x_second(int xs, int ds, int ls, int nl, bool 
   using Inv = FxLines<M, false, NT, P::NI, MapContig<double, M, P::NI>, true, 0, 0>;
   if constexpr (Inv::ST == 3) Inv::middle_rt(P::lines() + xs, ls, nl, P::twiddles());
   Inv::back_rt(P::lines() + xs, ls, nl, P::twiddles(), [&](const fx2* u, int l, int j) {
-    fx2* dst = P::lines() + ds + l * ls;
+    fx2* dst = P::lines() + ds + l * ls + zi<double>(j);
     int mx = 0, my = 0;
 #pragma unroll
     for (int r = 0; r < Inv::R1; ++r) {
       const int hx = (int)(u[r].x >> 32), hy = (int)(u[r].y >> 32);
       mx |= hx ^ (hx >> 31);
       my |= hy ^ (hy >> 31);
-      dst[zi<double>(j + r * Inv::NB1)] = u[r];
+      dst[MapContig<double, M, P::NI>::template step<Inv::NB1, 1>(j, r)] = u[r];
     }
-    if (maxima) {
-      atomicOr(P::field_m() + 2 * l, my);   // (parts exchanged)
-      atomicOr(P::field_m() + 2 * l + 1, mx);
+    if (maxima) {   // (parts exchanged)
+      if constexpr (Inv::NB1 % 32 == 0) {   // a warp holds butterflies of one line
+        mx = __reduce_or_sync(0xffffffffu, mx);
+        my = __reduce_or_sync(0xffffffffu, my);
+      }
+      if (Inv::NB1 % 32 != 0 || threadIdx.x % 32 == 0) {
+        atomicOr(P::field_m() + 2 * l, my);
+        atomicOr(P::field_m() + 2 * l + 1, mx);
+      }
     }
   });
 }
@@ -1321,31 +1293,28 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
       c.code = code[0] == FX_NAN || code[1] == FX_NAN || code[2] == FX_NAN ? FX_NAN
              : bu == NONE || bw == NONE ? FX_ZERO : FX_PLAIN;
       c.e = c.code == FX_PLAIN ? (bu - 62) + (bw - 61) + 64 : NONE;
+      c.smin = min(min(c.s1, c.s2u), min(c.s2w, c.s3));
       cols[tid] = c;
     }
     __syncthreads();
     for (int e = tid; e < CP * M; e += NT) {
       const int pr = e / M, p = e % M;
       const int zp = zi<double>(p);
-      const int ez = max(cols[2 * pr].e, cols[2 * pr + 1].e);
-      long long c[2][3];
-#pragma unroll 1
-      for (int cc = 0; cc < 2; ++cc) {
-        const int col = 2 * pr + cc;
-        const FxColumn& fc = cols[col];
-        const fx2 z1 = A[col * LP + zp], z2 = A[(NC + col) * LP + zp], z3 = A[(2 * NC + col) * LP + zp];
-        // (parts exchanged)
-        const fxsplit ux = fx_split(fx_shl(z1.y, fc.s1)), uy = fx_split(fx_shl(z1.x, fc.s1));
-        const fxsplit uz = fx_split(fx_shl(z2.y, fc.s2u)), wx = fx_split(fx_shl(z2.x, fc.s2w));
-        const fxsplit wy = fx_split(fx_shl(z3.y, fc.s3)), wz = fx_split(fx_shl(z3.x, fc.s3));
-        c[0][0] = c[1][0]; c[0][1] = c[1][1]; c[0][2] = c[1][2];
-        c[1][0] = fx_det(uy, wz, uz, wy);
-        c[1][1] = fx_det(uz, wx, ux, wz);
-        c[1][2] = fx_shl(fx_det(ux, wy, uy, wx), fc.e - ez);
+      const FxColumn& fa = cols[2 * pr];
+      const FxColumn& fb = cols[2 * pr + 1];
+      fx2* x = A + 2 * pr * LP + zp;   // lines of the pair: t NC LP + column LP
+      const int ez = max(fa.e, fb.e);
+      long long ca[3], cb[3];
+      if (min(fa.smin, fb.smin) >= 0) {   // (the same for a pair's positions: no divergence within a column)
+        fx_cross<true>(x, NC * LP, fa, ca);
+        fx_cross<true>(x + LP, NC * LP, fb, cb);
+      } else {
+        fx_cross<false>(x, NC * LP, fa, ca);
+        fx_cross<false>(x + LP, NC * LP, fb, cb);
       }
-      A[2 * pr * LP + zp] = fx2{c[0][0], c[0][1]};
-      A[(NC + 2 * pr) * LP + zp] = fx2{c[0][2], c[1][2]};
-      A[(2 * NC + 2 * pr) * LP + zp] = fx2{c[1][0], c[1][1]};
+      x[0] = fx2{ca[0], ca[1]};
+      x[NC * LP] = fx2{fx_shl<false>(ca[2], fa.e - ez), fx_shl<false>(cb[2], fb.e - ez)};
+      x[2 * NC * LP] = fx2{cb[0], cb[1]};
     }
     __syncthreads();
   {
@@ -1360,7 +1329,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
         __builtin_assume(l >= 0 && l < NF);
 #pragma unroll
         for (int r = 0; r < Fwd::R0; ++r) {
-          v[r] = A[2 * l * LP + zi<double>(j + r * Fwd::NB0)];
+          v[r] = A[2 * l * LP + zi<double>(j) + MapContig<double, M, NF>::template step<Fwd::NB0, 1>(j, r)];
           const int hx = (int)(v[r].x >> 32), hy = (int)(v[r].y >> 32);
           sum += max(hx ^ (hx >> 31), hy ^ (hy >> 31)) >> 5;
         }
@@ -1373,7 +1342,10 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
         const long long half = (1ll << sh) >> 1;
 #pragma unroll
         for (int r = 0; r < Fwd::R0; ++r) v[r] = fx2{(v[r].x + half) >> sh, (v[r].y + half) >> sh};
-        Fwd::first_dft(v, [&](int p, fx2 z) { A[(2 * l + 1) * LP + zi<double>(p)] = z; }, j);
+        fx2* dst = A + (2 * l + 1) * LP + zi<double>(j * Fwd::R0);
+        Fwd::first_dft(v, [&](int r, fx2 z) {
+          dst[MapContig<double, M, NF>::template step<1, Fwd::R0>(j * Fwd::R0, r)] = z;
+        });
         if (j == 0) {
           const int t = l / CP, pr = l - t * CP;
           const FxColumn& ca = cols[2 * pr];
