@@ -74,10 +74,12 @@ template <typename R> struct StageArgs {
   double ks;                       // 2 pi / L (shells of boxes other than 2 pi)
 };
 
-// CTA size of the stage epilogue (k_stage): p5_lines(n) n consecutive modes per
-// CTA; its CTA count sizes the fused diagnostics' partial rows.
-inline constexpr int p5_lines(int n, bool fp32) { return (void)n, fp32 ? 8 : 4; }
-inline constexpr int p5_ctas(int n, bool fp32) { return (n * (n / 2 + 1) + p5_lines(n, fp32) - 1) / p5_lines(n, fp32); }
+// CTAs of the stage epilogue (k_stage): each takes P5_LINES n modes (FP32:
+// pairs of modes, kx >= 0); sizes the fused diagnostics' partial rows.
+constexpr int P5_LINES = 4;
+inline constexpr int p5_ctas(int n, bool fp32) {
+  return ((fp32 ? n / 2 + 1 : n) * (n / 2 + 1) + P5_LINES - 1) / P5_LINES;
+}
 enum DiagBits : int { DIAG_TIER1 = 1, DIAG_SPECTRUM = 2 };
 
 // Per-pass timing hook (profiling mode): brackets each kernel launch with

@@ -275,11 +275,12 @@ __device__ __forceinline__ void flag_nonfinite(const StageArgs<R>& s, C2<R> v) {
 // Stage epilogue of NM modes at once: the inputs of all modes and all three
 // components are loaded before any result is stored (a store may alias a
 // later load as far as the compiler knows, so interleaving them would
-// serialise the loads).  ok[q] = false skips mode q.
+// serialise the loads).  ok[q] = false skips mode q.  The modes share |k|^2: k2
+// and the table index m are those of all of them.
 // KEEP: the final stages (ST_ETD_4, ST_RK4_4) also return the new state of
 // each mode in un[q][c] (for diagnostics fused into the same pass).
 template <typename R, int NM, bool KEEP = false>
-__device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_t* idx, const int* m, const R* k2,
+__device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_t* idx, int m, R k2,
                                               const C2<R> (*nl)[3], const bool* ok, C2<R> (*un)[3] = nullptr) {
   const size_t cs = s.cs;
   if (s.op == ST_NL_OUT) {
@@ -314,7 +315,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 #pragma unroll
     for (int q = 0; q < NM; ++q) {
       if (!ok[q]) continue;
-      const R visc = (R)(-s.nu) * k2[q];
+      const R visc = (R)(-s.nu) * k2;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const size_t i = c * cs + idx[q];
@@ -337,17 +338,15 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
     }
     return;
   }
-  // ETD coefficients of each mode (table keyed by the |k|^2 index)
-  const double* e[NM];
-#pragma unroll
-  for (int q = 0; q < NM; ++q) e[q] = s.etd + (size_t)(ok[q] ? m[q] : 0) * ETD_STRIDE;
+  // ETD coefficients of the modes (table keyed by the |k|^2 index)
+  const double* e = s.etd + (size_t)m * ETD_STRIDE;
   switch (s.op) {
     case ST_ETD_REF_1:    // solver.rs:264-281
     case ST_ETD_CM_1: {   // textbook: a = E2 u + (h/2) phi1(z/2) N1
       const double f = s.op == ST_ETD_REF_1 ? dt : 0.5 * dt;
       R eh[NM], qq[NM];
 #pragma unroll
-      for (int q = 0; q < NM; ++q) { eh[q] = (R)e[q][E_HALF]; qq[q] = (R)(f * e[q][E_A21]); }
+      for (int q = 0; q < NM; ++q) { eh[q] = (R)e[E_HALF]; qq[q] = (R)(f * e[E_A21]); }
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
         if (!ok[q]) continue;
@@ -366,7 +365,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
       C2<R> n1[NM][3];
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        b1[q] = (R)e[q][E_B1]; b23[q] = (R)e[q][E_B23]; eh[q] = (R)e[q][E_HALF]; qq[q] = (R)(f * e[q][E_A21]);
+        b1[q] = (R)e[E_B1]; b23[q] = (R)e[E_B23]; eh[q] = (R)e[E_HALF]; qq[q] = (R)(f * e[E_A21]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) n1[q][c] = ok[q] ? s.n1[c * cs + idx[q]] : czero<R>();
       }
@@ -386,7 +385,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
       C2<R> n1[NM][3], a[NM][3];
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        b23[q] = (R)e[q][E_B23]; ef[q] = (R)e[q][E_FULL]; qq[q] = (R)(dt * e[q][E_A41]);
+        b23[q] = (R)e[E_B23]; ef[q] = (R)e[E_FULL]; qq[q] = (R)(dt * e[E_A41]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           n1[q][c] = ok[q] ? s.n1[c * cs + idx[q]] : czero<R>();
@@ -410,7 +409,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
       C2<R> a[NM][3];
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        b4[q] = (R)e[q][E_B4]; ef[q] = (R)e[q][E_FULL];
+        b4[q] = (R)e[E_B4]; ef[q] = (R)e[E_FULL];
 #pragma unroll
         for (int c = 0; c < 3; ++c) a[q][c] = ok[q] ? s.acc[c * cs + idx[q]] : czero<R>();
       }
@@ -433,7 +432,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
       C2<R> n1[NM][3], ac[NM][3];
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        b23[q] = (R)e[q][E_B23]; eh[q] = (R)e[q][E_HALF]; qq[q] = (R)(0.5 * dt * e[q][E_A21]);
+        b23[q] = (R)e[E_B23]; eh[q] = (R)e[E_HALF]; qq[q] = (R)(0.5 * dt * e[E_A21]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           n1[q][c] = ok[q] ? s.n1[c * cs + idx[q]] : czero<R>();

@@ -809,15 +809,17 @@ __device__ __forceinline__ void diag_row(const StageArgs<R>& st, bool d_t1, bool
     for (int i = threadIdx.x; i < st.nsh; i += NT) row[4 + i] = hist[i];
 }
 
-// Modes and threads per CTA of k_stage: CTA b takes modes [b, b + 1) PER of the
-// (N, N, H) array (p5_ctas CTAs, which also sizes the diagnostics' rows).
+// Work and threads per CTA of k_stage (p5_ctas CTAs, which also sizes the
+// diagnostics' rows).  FP64: one mode per thread and iteration, in array order
+// (two need registers that it has not: N = 256 0.978 -> 1.006 ms).  FP32: the
+// two modes (kx, ky, kz) and (-kx, ky, kz), whose loads are in flight together
+// and which share |k|^2 and the coefficients: a gather from the table touches
+// 32 cache lines per warp.
 template <typename R, int N> struct StageGrid {
-  // modes per thread and iteration: FP32 keeps the loads of two in flight (N =
-  // 256 0.286 -> 0.261 ms), FP64 has no registers for it (0.978 -> 1.006 ms)
-  static constexpr int EM = sizeof(R) == 4 ? 2 : 1;
-  static constexpr int PER = p5_lines(N, sizeof(R) == 4) * N;
-  static constexpr int NT = cmin(256, cmax(32, PER / EM));
+  static constexpr int PER = P5_LINES * N;
+  static constexpr int NT = cmin(256, cmax(32, PER));
   static constexpr int MB = cmin(16, 768 / NT);   // 84 registers
+  static constexpr int TOTAL = (sizeof(R) == 4 ? N / 2 + 1 : N) * N * (N / 2 + 1);
 };
 
 // DIAG: the instance for final stages whose new state also feeds the fused
@@ -827,8 +829,8 @@ template <typename R, int N> struct StageGrid {
 // as the separate reduction passes do.
 template <typename R, int N, bool DIAG>
 __global__ void __launch_bounds__(StageGrid<R, N>::NT, DIAG ? 1 : StageGrid<R, N>::MB) k_stage(P5Args<R> a) {
-  constexpr int H = N / 2 + 1, NT = StageGrid<R, N>::NT, PER = StageGrid<R, N>::PER, EM = StageGrid<R, N>::EM;
-  constexpr int TOTAL = N * N * H;
+  constexpr int H = N / 2 + 1, NT = StageGrid<R, N>::NT, PER = StageGrid<R, N>::PER;
+  constexpr int TOTAL = StageGrid<R, N>::TOTAL;
   __shared__ R kxy[N], kz_s[H];   // wave numbers (their conversion is an FP64 operation in the FP64 form)
   extern __shared__ __align__(16) unsigned char vk_smem[];
   double* hist = reinterpret_cast<double*>(vk_smem);   // DIAG: nsh shells
@@ -888,47 +890,40 @@ __global__ void __launch_bounds__(StageGrid<R, N>::NT, DIAG ? 1 : StageGrid<R, N
     }
   } else {
 #pragma unroll 1
-    for (int e0 = blockIdx.x * PER + threadIdx.x; e0 < end; e0 += EM * NT) {
-      size_t idx[EM];
-      int mm[EM], ix[EM], iy[EM], z[EM];
-      R kk[EM];
-      C2<R> nl[EM][3];
-      bool ok[EM];
+    for (int e = blockIdx.x * PER + threadIdx.x; e < end; e += NT) {
+      int ix, iy, z;   // ix <= N / 2
+      locate((unsigned)e, ix, iy, z);
+      const bool ok[2] = {true, ix > 0 && ix < N / 2};
+      const size_t idx[2] = {(size_t)e, ok[1] ? ((size_t)(N - ix) * N + iy) * H + z : (size_t)e};
+      const int kxi = signed_k(ix, N), kyi = signed_k(iy, N);
+      const R kx = kxy[ix], ky = kxy[iy], kz = kz_s[z];
+      C2<R> nl[2][3];
 #pragma unroll
-      for (int q = 0; q < EM; ++q) {
-        const int e = e0 + q * NT;
-        ok[q] = e < end;
-        idx[q] = ok[q] ? e : e0;
-        locate((unsigned)idx[q], ix[q], iy[q], z[q]);
+      for (int q = 0; q < 2; ++q) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) nl[q][c] = a.in[(size_t)c * a.fsin + idx[q]];
       }
+      const R k2 = (kx * kx + ky * ky) + kz * kz;
+      const R inv = k2 < R(1e-30) ? R(0) : R(1) / k2;
 #pragma unroll
-      for (int q = 0; q < EM; ++q) {
-        const int kxi = signed_k(ix[q], N), kyi = signed_k(iy[q], N);
-        const R kx = kxy[ix[q]], ky = kxy[iy[q]], kz = kz_s[z[q]];
+      for (int q = 0; q < 2; ++q) {
+        const R k = q == 0 ? kx : -kx;
 #pragma unroll
         for (int c = 0; c < 3; ++c) nl[q][c] = cscale<R>(nl[q][c], a.s_out);
-        const R k2 = (kx * kx + ky * ky) + kz * kz;
-        if (!(k2 < R(1e-30))) {
-          const R inv = R(1) / k2;
-          const C2<R> kd = cmk<R>((kx * nl[q][0].x + ky * nl[q][1].x) + kz * nl[q][2].x,
-                                  (kx * nl[q][0].y + ky * nl[q][1].y) + kz * nl[q][2].y);
-          nl[q][0] = cmk<R>(nl[q][0].x - kx * kd.x * inv, nl[q][0].y - kx * kd.y * inv);
-          nl[q][1] = cmk<R>(nl[q][1].x - ky * kd.x * inv, nl[q][1].y - ky * kd.y * inv);
-          nl[q][2] = cmk<R>(nl[q][2].x - kz * kd.x * inv, nl[q][2].y - kz * kd.y * inv);
-        }
-        kk[q] = k2;
-        mm[q] = kxi * kxi + kyi * kyi + z[q] * z[q];
+        const C2<R> kd = cmk<R>((k * nl[q][0].x + ky * nl[q][1].x) + kz * nl[q][2].x,
+                                (k * nl[q][0].y + ky * nl[q][1].y) + kz * nl[q][2].y);
+        nl[q][0] = cmk<R>(nl[q][0].x - k * kd.x * inv, nl[q][0].y - k * kd.y * inv);
+        nl[q][1] = cmk<R>(nl[q][1].x - ky * kd.x * inv, nl[q][1].y - ky * kd.y * inv);
+        nl[q][2] = cmk<R>(nl[q][2].x - kz * kd.x * inv, nl[q][2].y - kz * kd.y * inv);
       }
+      const int m = kxi * kxi + kyi * kyi + z * z;
       if constexpr (!DIAG) {
-        stage_apply_n<R, EM>(a.st, idx, mm, kk, nl, ok);
+        stage_apply_n<R, 2>(a.st, idx, m, k2, nl, ok);
       } else {
-        C2<R> un[EM][3];
-        stage_apply_n<R, EM, true>(a.st, idx, mm, kk, nl, ok, un);
-#pragma unroll
-        for (int q = 0; q < EM; ++q)
-          if (ok[q]) diag(signed_k(ix[q], N), signed_k(iy[q], N), z[q], un[q]);
+        C2<R> un[2][3];
+        stage_apply_n<R, 2, true>(a.st, idx, m, k2, nl, ok, un);
+        diag(kxi, kyi, z, un[0]);
+        if (ok[1]) diag(-kxi, kyi, z, un[1]);
       }
     }
   }
