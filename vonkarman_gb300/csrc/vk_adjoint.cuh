@@ -207,6 +207,7 @@ k_adj_z(A3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
       prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fsin + (size_t)b * (2 * CP * H), 2 * CP * H * sizeof(C2<R>));
   }
   load_twtab<R, M, true, NT>(tw_s, tw);
+  grid_depend();
   C2<R>* A = reinterpret_cast<C2<R>*>(vk_smem);   // NI lines
   C2<R>* B = A + NI * LP;                          // NF lines
   const int col0 = blockIdx.x * 2 * CP;
@@ -392,6 +393,7 @@ k_adj_p5(A5Args<R> a, const C2<R>* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, false>(L)];
   load_twtab<R, L, false, NT>(tw_s, tw);
+  grid_depend();
   C2<R>* xb = reinterpret_cast<C2<R>*>(vk_smem);
   C2<R>* acc = xb + rsmem_elems<R, L, NLINES>();   // 3 components x N x NLINES
   constexpr int H = N / 2 + 1;   // a.H of the launch
@@ -459,6 +461,7 @@ k_adj_stage_f64(A5Args<double> a) {
   __shared__ double kxy[N], kz_s[H];
   for (int i = threadIdx.x; i < N; i += NT) kxy[i] = a.ks * (double)signed_k(i, N);
   for (int i = threadIdx.x; i < H; i += NT) kz_s[i] = a.ks * (double)i;
+  grid_depend();
   __syncthreads();
   const int end = min((int)(blockIdx.x + 1) * PER, TOTAL);
 #pragma unroll 1

@@ -34,6 +34,12 @@ namespace vk {
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
+// Kernels launched with launch_overlapped: waits until the kernel before is
+// complete and its writes are visible.  Before it a kernel reads only tables
+// that no kernel writes, and writes nothing but shared memory.
+__device__ __forceinline__ void grid_depend() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 __device__ __forceinline__ void prefetch_l2_bulk(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }

@@ -709,6 +709,8 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
   static_assert(NT % NLINES == 0, "a thread keeps one line in every stage");
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, false>(L)];
+  load_twtab<R, L, false, NT>(tw_s, tw);
+  grid_depend();
   // the input rows of the CTA pf blocks ahead (ops with prefetch_row, whole
   // tiles whose rows are whole 128-byte lines)
   if constexpr (OpHasPrefetch<Op>::value && NLINES * sizeof(C2<R>) == 128) {
@@ -719,7 +721,6 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
         for (int t = threadIdx.x; t < L; t += NT) op.prefetch_row(b % op.nfields, lam0, NLINES, t);
     }
   }
-  load_twtab<R, L, false, NT>(tw_s, tw);
   C2<R>* xb = reinterpret_cast<C2<R>*>(vk_smem);
   const int f = blockIdx.x % op.nfields;
   const int tile = blockIdx.x / op.nfields;
@@ -840,6 +841,7 @@ __global__ void __launch_bounds__(StageGrid<R, N>::NT, DIAG ? 1 : StageGrid<R, N
   for (int i = threadIdx.x; i < H; i += NT) kz_s[i] = a.ks * (R)i;
   if (d_sp)
     for (int i = threadIdx.x; i < a.st.nsh; i += NT) hist[i] = 0.0;
+  grid_depend();
   __syncthreads();
   double dsum[4] = {0.0, 0.0, 0.0, 0.0};
   const bool ks_one = a.st.ks == 1.0;
@@ -1040,6 +1042,7 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
       prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fsin + (size_t)b * (2 * CP * H), 2 * CP * H * sizeof(C2<R>));
   }
   load_twtab<R, M, true, NT>(tw_s, tw);
+  grid_depend();
   C2<R>* A = reinterpret_cast<C2<R>*>(vk_smem);
   C2<R>* B = INPL ? A : A + NI * LP;
   C2<R>* XF = INPL ? A + NF * LP : B;   // exchange of the forward transform
@@ -1235,6 +1238,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
   const int* field_m = P::field_m();
   FxColumn* cols = P::cols();
   load_twtab<double, M, true, NT>(reinterpret_cast<double2*>(P::twiddles()), reinterpret_cast<const double2*>(tw));
+  grid_depend();
   const int col0 = blockIdx.x * NC;
   const int tid = threadIdx.x;
   for (int i = tid; i < 2 * NI; i += NT) P::field_m()[i] = 0;
@@ -1427,6 +1431,7 @@ k_nz_max(NZArgs<R> a, const C2<R>* __restrict__ tw, int pf) {
       prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fs + (size_t)b * (2 * CP * H), 2 * CP * H * sizeof(C2<R>));
   }
   load_twtab<R, N, true, NT>(tw_s, tw);
+  grid_depend();
   if (threadIdx.x == 0) redn = 0;
   const int col0 = blockIdx.x * 2 * CP;
   fft_lines<R, N, true, NT, NL, MapContig<R, N, NL>, true, true>(
@@ -1539,6 +1544,7 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_r2c(FZArgs
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, true>(L)];
   load_twtab<R, L, true, NT>(tw_s, tw);
+  grid_depend();
   C2<R>* lines = reinterpret_cast<C2<R>*>(vk_smem);
   const int col0 = blockIdx.x * 2 * CP;
   fft_lines<R, L, false, NT, CP, MapContig<R, L, CP>, true, true>(
@@ -1565,6 +1571,7 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_c2r(FZArgs
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, true>(L)];
   load_twtab<R, L, true, NT>(tw_s, tw);
+  grid_depend();
   const int col0 = blockIdx.x * 2 * CP;
   fft_lines<R, L, true, NT, CP, MapContig<R, L, CP>, false, true>(
       reinterpret_cast<C2<R>*>(vk_smem), tw_s,

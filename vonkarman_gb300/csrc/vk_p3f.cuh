@@ -310,6 +310,7 @@ k_p3f(P3Args<float> a, const float2* __restrict__ tw, int pf) {
     prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fsin + (size_t)(blockIdx.x + pf) * (2 * CP * 129),
                      2 * CP * 129 * sizeof(float2));
   p3f_twiddles<CP>(twi, twf, tw);
+  grid_depend();
   float2* X = reinterpret_cast<float2*>(vk_smem);
   // the first barrier of the tile orders the twiddle loads before their use
   p3f_tile<CP>(a, blockIdx.x * 2 * CP, X, twi, twf, P3SrcGlobal{a.in, a.fsin});
