@@ -106,25 +106,28 @@ template <int B> VK_FIX_HD fx2 fx_multiple(fx2 a) {
 }
 // a / 2^B (the untwiddled input beside twiddled ones)
 template <int B> VK_FIX_HD fx2 fx_shift(fx2 a) { return fx2{fx_bump<B>(a.x) >> B, fx_bump<B>(a.y) >> B}; }
-// Plans.  From 256 points on three stages of small radices (up to 12), whose few
-// registers let three times the warps of a two-stage plan be resident: the
-// integer code is bound by latency, not by its instruction count.  Below, two
-// stages, the shortest lines with small radices (a small grid is bound by the
-// latency of one thread's work).  The first stage has 2^b or 16 c butterflies,
-// so that groups of lanes keep one contiguous line.
+// Plans.  From 192 points on three stages of small radices (up to 12), whose few
+// registers let up to three times the warps of a two-stage plan be resident: the
+// integer code is bound by latency, not by its instruction count.  (z pass with
+// the cross product, ms: N = 256 {24, 16} 2.90, {8, 8, 6} 2.65; N = 128 {12, 16}
+// 0.414, {12, 4, 4} 0.375, {6, 8, 4} 0.355.)  Below, two stages: a third one's
+// exchange costs about what it gains (N = 64 {12, 8} 0.055, {3, 8, 4} 0.062;
+// {6, 4, 4} 0.047, but its roundings drift one way).  The first stage has 2^b or
+// 16 c butterflies, so that groups of lanes keep one contiguous line.
 VK_FIX_HD constexpr int fx_radix0(int L) {
   return L == 8 ? 2 : L == 12 ? 3 : L == 16 ? 4 : L == 24 ? 6 : L == 32 ? 4 : L == 48 ? 6 : L == 64 ? 8 : L == 96 ? 12
-       : L == 128 ? 16 : L == 192 ? 12 : L == 256 ? 8 : L == 384 ? 8 : L == 512 ? 8 : L == 768 ? 12 : 0;
+       : L == 128 ? 16 : L == 192 ? 6 : L == 256 ? 8 : L == 384 ? 8 : L == 512 ? 8 : L == 768 ? 12 : 0;
 }
 VK_FIX_HD constexpr bool fx_supported(int L) { return fx_radix0(L) > 0; }
-VK_FIX_HD constexpr int fx_stages(int L) { return L >= 256 ? 3 : 2; }
+VK_FIX_HD constexpr int fx_stages(int L) { return L >= 192 ? 3 : 2; }
+VK_FIX_HD constexpr int fx_radix1(int L) { return fx_stages(L) == 2 ? L / fx_radix0(L) : 8; }
 VK_FIX_HD constexpr int fx_radix(int L, int s) {
-  return s == 0 ? fx_radix0(L) : fx_stages(L) == 2 ? L / fx_radix0(L) : s == 1 ? 8 : L / fx_radix0(L) / 8;
+  return s == 0 ? fx_radix0(L) : s == 1 ? fx_radix1(L) : L / fx_radix0(L) / fx_radix1(L);
 }
 // log2 of the factor that the twiddles of a later stage of radix r divide by;
 // their components are held in units of 2^-(64 - growth), which makes
 // fx_twiddle's a w / 2^64 the scaled product
-VK_FIX_HD constexpr int fx_growth(int r) { return r <= 4 ? 2 : r <= 8 ? 3 : r <= 16 ? 4 : 5; }
+VK_FIX_HD constexpr int fx_growth(int r) { return r <= 8 ? 3 : r <= 16 ? 4 : 5; }
 // sum of the growths of a plan's stages: the outputs' exponent above the quantum
 VK_FIX_HD constexpr int fx_total_growth(int L) {
   int g = 0;

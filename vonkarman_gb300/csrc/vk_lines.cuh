@@ -329,6 +329,10 @@ __device__ __forceinline__ double fx_to_double(long long v, int q20) {
 // State of a line between the stages: output exponent and FxCode.
 struct FxState { int q, code; };
 
+// words that the maximum over a contiguous line's threads takes in shared memory
+template <int L, int NLINES> __host__ __device__ constexpr int fx_contig_parts() {
+  return 32 % (L / fx_radix(L, 0)) == 0 ? 1 : L / fx_radix(L, 0) * NLINES / 16;
+}
 template <int L, int NT, int NLINES, class MAP>
 __host__ __device__ constexpr int fx_round_lines() {   // lines per stage-1 round (contiguous lines)
   return cmin(NT / (L / fx_radix(L, fx_stages(L) - 1)), NLINES);
@@ -351,7 +355,7 @@ struct FxLines {
   static_assert(G0 <= NT, "one first-stage butterfly per thread");
   static_assert(!MAP::CONTIG || 32 % NB0 == 0 || NB0 % 16 == 0, "groups of lanes keep one contiguous line");
   // words of the part array of front and line_max
-  static constexpr int PARTS = !MAP::CONTIG ? NW0 * NLINES : 32 % NB0 == 0 ? 1 : G0 / 16;
+  static constexpr int PARTS = MAP::CONTIG ? fx_contig_parts<L, NLINES>() : NW0 * NLINES;
   static_assert(MAP::CONTIG || (32 % NLINES == 0 && !SL), "interleaved lines tile a warp");
 
   __device__ __forceinline__ static int line_max(int m, int* part) {
@@ -1180,7 +1184,7 @@ template <int M, int CP> struct P3X {
   static constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
   static constexpr int TW = NI * LP;                                 // in units of fx2
   static constexpr int INTS = TW + twtab_elems<double, true>(M);
-  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn) + (NI * M / 128 + 1) * 4;
+  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn) + fx_contig_parts<M, NI>() * 4;
   __device__ __forceinline__ static fx2* lines() {
     extern __shared__ __align__(16) unsigned char vk_smem[];
     return reinterpret_cast<fx2*>(vk_smem);
