@@ -131,9 +131,9 @@ template <int L, int NT>
 __host__ __device__ constexpr int fx_min_blocks() { return cmax(1, (fx_stages(L) == 3 ? 1152 : 512) / NT); }
 
 // Minimum resident CTAs per SM requested from the compiler (caps registers):
-// 24 warps per SM for the strided passes where the plan allows it; one or two
-// CTAs for the long FP64 / 768-point plans and for the multi-field P5 kernels
-// (EPI), whose shared memory limits residency anyway.
+// 24 warps per SM for the strided FP32 passes where the plan allows it; one or
+// two CTAs for the 768-point plans and for the adjoint's multi-field kernel
+// (EPI), whose shared memory limits residency anyway.  FP64: fx_min_blocks.
 template <typename R, int L, int NT, bool EPI = false>
 __host__ __device__ constexpr int lines_min_blocks() {
   if constexpr (sizeof(R) == 8) {
@@ -302,10 +302,10 @@ struct RegStage {
 // Stage 0: one butterfly per thread.  Its bound of the inputs' magnitudes
 // (fx_bound) is maximised over the line's threads, by shuffles where a line's
 // butterflies share a warp (contiguous lines) and through shared memory
-// otherwise, and gives the line's exponent.  Stage 1 loops over the rest in
-// rounds of NT threads (whole lines per round where the store functor writes
-// back into the exchange buffer, SL), so that a CTA needs no more threads than
-// stage 0 keeps busy.
+// otherwise, and gives the line's exponent.  The later stages loop over their
+// butterflies in rounds of NT threads (whole lines per round where they write
+// back into the exchange buffer), so that a CTA needs no more threads than stage
+// 0 keeps busy.
 //
 // Lines whose bound is outside the comfortable range carry a code: all zero
 // (the transform's rounding compensations would leave a few units), tiny and
@@ -937,7 +937,7 @@ __global__ void __launch_bounds__(StageGrid<R, N>::NT, DIAG ? 1 : StageGrid<R, N
 }
 
 // ---------------------------------------------------------------------------
-// P3 on the register engine: per CTA CP column pairs.  Inverse lines (6 CP):
+// P3 on the register engine (FP32; FP64: k_p3x below): per CTA CP column pairs.  Inverse lines (6 CP):
 // l = t * 2CP + c, the packed pair t of column c ((u_x, u_y), (u_z, w_x),
 // (w_y, w_z)); the first stage packs straight from global memory with the
 // Hermitian extension (z-line helpers above), the last stage writes the
@@ -1139,9 +1139,8 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
 // its line right by what its largest butterfly needs (rounded), at most 6 bits.
 //
 // The inverse runs as a forward transform of lines with real and imaginary
-// parts exchanged, so that both directions share the code of the second stage:
-// CTAs of one SM are in different phases, and their instructions have to fit
-// its instruction cache.  Lines l = t 2CP + c (t: packed pair, c: column); the
+// parts exchanged, so that both directions are one text (p3x_second) and one
+// twiddle table.  Lines l = t 2CP + c (t: packed pair, c: column); the
 // forward lines (t, pair) use line t 2CP + 2 pair and exchange through the next
 // one, both of which belong to that pair.
 // ---------------------------------------------------------------------------
@@ -1177,8 +1176,7 @@ template <int M, int CP> __host__ __device__ constexpr int p3x_threads() {
   return rthreads<double, M, 6 * CP, true>();
 }
 
-// Dynamic shared memory of k_p3x (one array, so that the second stage, a
-// function of its own, addresses it as shared memory).
+// Dynamic shared memory of k_p3x.
 template <int M, int CP> struct P3X {
   static constexpr int LP = zpad_len<double>(M);
   static constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
@@ -1195,9 +1193,10 @@ template <int M, int CP> struct P3X {
   __device__ __forceinline__ static FxColumn* cols() { return reinterpret_cast<FxColumn*>(field_m() + 2 * NI); }
   __device__ __forceinline__ static int* part() { return reinterpret_cast<int*>(cols() + NC); }   // FxLines::PARTS
 };
-// Second stage of nl lines at stride ls, from xs to ds (element offsets), with
-// the fields' magnitudes where they are wanted.  Not inlined: both directions
-// run this code.
+// Stages after the first of nl lines at stride ls, from xs to ds (element
+// offsets), with the fields' magnitudes where they are wanted.
+// Inlined twice: as one function it spills (N = 256 3.2 ms against 2.9), as a
+// loop over the directions more so (3.7).
 template <int M, int CP, int NT>
 __device__ __forceinline__ void p3x_second(int xs, int ds, int ls, int nl, bool maxima) {
   using P = P3X<M, CP>;
@@ -1247,125 +1246,125 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
   const int tid = threadIdx.x;
   for (int i = tid; i < 2 * NI; i += NT) P::field_m()[i] = 0;
   {
-      // inverse: packed pairs, positions H .. M - H are the z zero-padding
-      const auto ld = [&](int l, int p) -> C2x2<double> {
-        const int t = l / NC;
-        const int col = col0 + l % NC;
-        const bool lo = p < H;
-        C2x2<double> r{};
-        if (col < a.ncols && (lo || p > M - H)) {
-          const double2* src = a.in + (size_t)col * H + (lo ? p : M - p);
-          r.a = src[(size_t)(2 * t) * a.fsin];
-          r.b = src[(size_t)(2 * t + 1) * a.fsin];
-        }
-        return r;
-      };
-      // Z = X + i Y with the Hermitian extension, parts exchanged
-      const auto pp = [&](int, int p, const C2x2<double>& r) -> double2 {
-        if (p == 0) return make_double2(r.b.x, r.a.x);
-        return p < H ? make_double2(r.a.y + r.b.x, r.a.x - r.b.y) : make_double2(r.b.x - r.a.y, r.a.x + r.b.y);
-      };
-      Inv::front(A, FxFill<M, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, P::part(), line_s, 0);
+    // inverse: packed pairs, positions H .. M - H are the z zero-padding
+    const auto ld = [&](int l, int p) -> C2x2<double> {
+      const int t = l / NC;
+      const int col = col0 + l % NC;
+      const bool lo = p < H;
+      C2x2<double> r{};
+      if (col < a.ncols && (lo || p > M - H)) {
+        const double2* src = a.in + (size_t)col * H + (lo ? p : M - p);
+        r.a = src[(size_t)(2 * t) * a.fsin];
+        r.b = src[(size_t)(2 * t + 1) * a.fsin];
+      }
+      return r;
+    };
+    // Z = X + i Y with the Hermitian extension, parts exchanged
+    const auto pp = [&](int, int p, const C2x2<double>& r) -> double2 {
+      if (p == 0) return make_double2(r.b.x, r.a.x);
+      return p < H ? make_double2(r.a.y + r.b.x, r.a.x - r.b.y) : make_double2(r.b.x - r.a.y, r.a.x + r.b.y);
+    };
+    Inv::front(A, FxFill<M, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, P::part(), line_s, 0);
   }
   __syncthreads();
   p3x_second<M, CP, NT>(0, 0, LP, NI, true);
   __syncthreads();
-    if (tid < NC) {   // the column's shifts
-      int q[3], code[3];
+  if (tid < NC) {   // the column's shifts
+    int q[3], code[3];
 #pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        const State s = Inv::unpack_state(line_s[t * NC + tid]);
-        code[t] = s.code;
-        q[t] = s.q + (s.code == FX_TINY ? -FX_RANGE : s.code == FX_HUGE ? FX_RANGE : 0);
-      }
-      const int* m1 = field_m + 2 * tid;
-      const int* m2 = m1 + 2 * NC;
-      const int* m3 = m2 + 2 * NC;
-      constexpr int NONE = -(1 << 20);
-      int bu = code[0] == FX_ZERO ? NONE : fx_field_bits(q[0], m1[0] | m1[1]);
-      int bw = code[2] == FX_ZERO ? NONE : fx_field_bits(q[2], m3[0] | m3[1]);
-      if (code[1] != FX_ZERO) {
-        bu = max(bu, fx_field_bits(q[1], m2[0]));
-        bw = max(bw, fx_field_bits(q[1], m2[1]));
-      }
-      FxColumn c;
-      c.s1 = code[0] == FX_ZERO ? -63 : q[0] - (bu - 62);
-      c.s2u = code[1] == FX_ZERO ? -63 : q[1] - (bu - 62);
-      c.s2w = code[1] == FX_ZERO ? -63 : q[1] - (bw - 61);
-      c.s3 = code[2] == FX_ZERO ? -63 : q[2] - (bw - 61);
-      c.code = code[0] == FX_NAN || code[1] == FX_NAN || code[2] == FX_NAN ? FX_NAN
-             : bu == NONE || bw == NONE ? FX_ZERO : FX_PLAIN;
-      c.e = c.code == FX_PLAIN ? (bu - 62) + (bw - 61) + 64 : NONE;
-      c.smin = min(min(c.s1, c.s2u), min(c.s2w, c.s3));
-      cols[tid] = c;
+    for (int t = 0; t < 3; ++t) {
+      const State s = Inv::unpack_state(line_s[t * NC + tid]);
+      code[t] = s.code;
+      q[t] = s.q + (s.code == FX_TINY ? -FX_RANGE : s.code == FX_HUGE ? FX_RANGE : 0);
     }
-    __syncthreads();
-    for (int e = tid; e < CP * M; e += NT) {
-      const int pr = e / M, p = e % M;
-      const int zp = zi<double>(p);
-      const FxColumn& fa = cols[2 * pr];
-      const FxColumn& fb = cols[2 * pr + 1];
-      fx2* x = A + 2 * pr * LP + zp;   // lines of the pair: t NC LP + column LP
-      const int ez = max(fa.e, fb.e);
-      long long ca[3], cb[3];
-      if (min(fa.smin, fb.smin) >= 0) {   // (the same for a pair's positions: no divergence within a column)
-        fx_cross<true>(x, NC * LP, fa, ca);
-        fx_cross<true>(x + LP, NC * LP, fb, cb);
-      } else {
-        fx_cross<false>(x, NC * LP, fa, ca);
-        fx_cross<false>(x + LP, NC * LP, fb, cb);
-      }
-      x[0] = fx2{ca[0], ca[1]};
-      x[NC * LP] = fx2{fx_shl<false>(ca[2], fa.e - ez), fx_shl<false>(cb[2], fb.e - ez)};
-      x[2 * NC * LP] = fx2{cb[0], cb[1]};
+    const int* m1 = field_m + 2 * tid;
+    const int* m2 = m1 + 2 * NC;
+    const int* m3 = m2 + 2 * NC;
+    constexpr int NONE = -(1 << 20);
+    int bu = code[0] == FX_ZERO ? NONE : fx_field_bits(q[0], m1[0] | m1[1]);
+    int bw = code[2] == FX_ZERO ? NONE : fx_field_bits(q[2], m3[0] | m3[1]);
+    if (code[1] != FX_ZERO) {
+      bu = max(bu, fx_field_bits(q[1], m2[0]));
+      bw = max(bw, fx_field_bits(q[1], m2[1]));
     }
-    __syncthreads();
+    FxColumn c;
+    c.s1 = code[0] == FX_ZERO ? -63 : q[0] - (bu - 62);
+    c.s2u = code[1] == FX_ZERO ? -63 : q[1] - (bu - 62);
+    c.s2w = code[1] == FX_ZERO ? -63 : q[1] - (bw - 61);
+    c.s3 = code[2] == FX_ZERO ? -63 : q[2] - (bw - 61);
+    c.code = code[0] == FX_NAN || code[1] == FX_NAN || code[2] == FX_NAN ? FX_NAN
+           : bu == NONE || bw == NONE ? FX_ZERO : FX_PLAIN;
+    c.e = c.code == FX_PLAIN ? (bu - 62) + (bw - 61) + 64 : NONE;
+    c.smin = min(min(c.s1, c.s2u), min(c.s2w, c.s3));
+    cols[tid] = c;
+  }
+  __syncthreads();
+  for (int e = tid; e < CP * M; e += NT) {
+    const int pr = e / M, p = e % M;
+    const int zp = zi<double>(p);
+    const FxColumn& fa = cols[2 * pr];
+    const FxColumn& fb = cols[2 * pr + 1];
+    fx2* x = A + 2 * pr * LP + zp;   // lines of the pair: t NC LP + column LP
+    const int ez = max(fa.e, fb.e);
+    long long ca[3], cb[3];
+    if (min(fa.smin, fb.smin) >= 0) {   // (the same for a pair's positions: no divergence within a column)
+      fx_cross<true>(x, NC * LP, fa, ca);
+      fx_cross<true>(x + LP, NC * LP, fb, cb);
+    } else {
+      fx_cross<false>(x, NC * LP, fa, ca);
+      fx_cross<false>(x + LP, NC * LP, fb, cb);
+    }
+    x[0] = fx2{ca[0], ca[1]};
+    x[NC * LP] = fx2{fx_shl<false>(ca[2], fa.e - ez), fx_shl<false>(cb[2], fb.e - ez)};
+    x[2 * NC * LP] = fx2{cb[0], cb[1]};
+  }
+  __syncthreads();
   {
-      // forward lines l = t CP + pr
-      const int l = MapContig<double, M, NF>::template line<Fwd::NB0>(tid);
-      const int j = MapContig<double, M, NF>::template bfly<Fwd::NB0>(tid);
-      const bool act = tid < Fwd::G0;
-      fx2 v[Fwd::R0];
-      int sum = 0;
-      if (act) {
-        __builtin_assume(j >= 0 && j < Fwd::NB0);
-        __builtin_assume(l >= 0 && l < NF);
+    // forward lines l = t CP + pr
+    const int l = MapContig<double, M, NF>::template line<Fwd::NB0>(tid);
+    const int j = MapContig<double, M, NF>::template bfly<Fwd::NB0>(tid);
+    const bool act = tid < Fwd::G0;
+    fx2 v[Fwd::R0];
+    int sum = 0;
+    if (act) {
+      __builtin_assume(j >= 0 && j < Fwd::NB0);
+      __builtin_assume(l >= 0 && l < NF);
 #pragma unroll
-        for (int r = 0; r < Fwd::R0; ++r) {
-          v[r] = A[2 * l * LP + zi<double>(j) + MapContig<double, M, NF>::template step<Fwd::NB0, 1>(j, r)];
-          const int hx = (int)(v[r].x >> 32), hy = (int)(v[r].y >> 32);
-          sum += max(hx ^ (hx >> 31), hy ^ (hy >> 31)) >> 5;
-        }
-        sum += Fwd::R0;                                // the shifted-out bits
-        sum += (sum >> 2) + (sum >> 3) + (sum >> 4) + 3;   // times 1.4375 > sqrt(2), rounded up
+      for (int r = 0; r < Fwd::R0; ++r) {
+        v[r] = A[2 * l * LP + zi<double>(j) + MapContig<double, M, NF>::template step<Fwd::NB0, 1>(j, r)];
+        const int hx = (int)(v[r].x >> 32), hy = (int)(v[r].y >> 32);
+        sum += max(hx ^ (hx >> 31), hy ^ (hy >> 31)) >> 5;
       }
-      // |z| sums below 2^(37 + bits); to 2^62
-      const int sh = max(0, 37 + 32 - __clz(Fwd::line_max(sum, P::part())) - 62);
-      if (act) {
-        const long long half = (1ll << sh) >> 1;
+      sum += Fwd::R0;                                // the shifted-out bits
+      sum += (sum >> 2) + (sum >> 3) + (sum >> 4) + 3;   // times 1.4375 > sqrt(2), rounded up
+    }
+    // |z| sums below 2^(37 + bits); to 2^62
+    const int sh = max(0, 37 + 32 - __clz(Fwd::line_max(sum, P::part())) - 62);
+    if (act) {
+      const long long half = (1ll << sh) >> 1;
 #pragma unroll
-        for (int r = 0; r < Fwd::R0; ++r) v[r] = fx2{(v[r].x + half) >> sh, (v[r].y + half) >> sh};
-        fx2* dst = A + (2 * l + 1) * LP + zi<double>(j * Fwd::R0);
-        Fwd::first_dft(v, [&](int r, fx2 z) {
-          dst[MapContig<double, M, NF>::template step<1, Fwd::R0>(j * Fwd::R0, r)] = z;
-        });
-        if (j == 0) {
-          const int t = l / CP, pr = l - t * CP;
-          const FxColumn& ca = cols[2 * pr];
-          const FxColumn& cb = cols[2 * pr + 1];
-          const int e = t == 0 ? ca.e : t == 1 ? max(ca.e, cb.e) : cb.e;
-          int code = t == 0 ? ca.code : t == 2 ? cb.code : ca.code == FX_NAN || cb.code == FX_NAN ? FX_NAN
-                   : ca.code == FX_ZERO && cb.code == FX_ZERO ? FX_ZERO : FX_PLAIN;
-          int q = e + sh + Fwd::TG - 1;   // the modes are halved by the unpacking
-          if (code == FX_PLAIN && (q < -950 || q > 900)) {   // near the ends of the double range, or beyond
-            code = q < -950 - FX_RANGE ? FX_ZERO : q < 0 ? FX_TINY : q <= 900 + FX_RANGE ? FX_HUGE : FX_NAN;
-            q += q < 0 ? FX_RANGE : -FX_RANGE;
-          }
-          line_s[l] = Fwd::pack_state(code == FX_ZERO || code == FX_NAN ? 0 : q, code);
+      for (int r = 0; r < Fwd::R0; ++r) v[r] = fx2{(v[r].x + half) >> sh, (v[r].y + half) >> sh};
+      fx2* dst = A + (2 * l + 1) * LP + zi<double>(j * Fwd::R0);
+      Fwd::first_dft(v, [&](int r, fx2 z) {
+        dst[MapContig<double, M, NF>::template step<1, Fwd::R0>(j * Fwd::R0, r)] = z;
+      });
+      if (j == 0) {
+        const int t = l / CP, pr = l - t * CP;
+        const FxColumn& ca = cols[2 * pr];
+        const FxColumn& cb = cols[2 * pr + 1];
+        const int e = t == 0 ? ca.e : t == 1 ? max(ca.e, cb.e) : cb.e;
+        int code = t == 0 ? ca.code : t == 2 ? cb.code : ca.code == FX_NAN || cb.code == FX_NAN ? FX_NAN
+                 : ca.code == FX_ZERO && cb.code == FX_ZERO ? FX_ZERO : FX_PLAIN;
+        int q = e + sh + Fwd::TG - 1;   // the modes are halved by the unpacking
+        if (code == FX_PLAIN && (q < -950 || q > 900)) {   // near the ends of the double range, or beyond
+          code = q < -950 - FX_RANGE ? FX_ZERO : q < 0 ? FX_TINY : q <= 900 + FX_RANGE ? FX_HUGE : FX_NAN;
+          q += q < 0 ? FX_RANGE : -FX_RANGE;
         }
+        line_s[l] = Fwd::pack_state(code == FX_ZERO || code == FX_NAN ? 0 : q, code);
       }
     }
-    __syncthreads();
+  }
+  __syncthreads();
   p3x_second<M, CP, NT>(LP, 0, 2 * LP, NF, false);
   __syncthreads();
   for (int e = tid; e < CP * 3 * H; e += NT) {
