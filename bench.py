@@ -526,7 +526,9 @@ def run_ours(args, d: Dist):
     prof_steps = 2
     elem = 16 if args.precision == "fp64" else 8
     prof, passes = profile_passes(s, prof_steps, n, elem, hbm)
-    launches_per_step = sum(c for k, (t, c) in prof.items() if k not in ("spectrum", "tier1_sums")) / prof_steps
+    # (P5 is two launches, the x-forward and the stage kernel)
+    launches_per_step = sum(c * (2 if k.startswith("P5") else 1) for k, (t, c) in prof.items()
+                            if k not in ("spectrum", "tier1_sums")) / prof_steps
     gpu_launches = int(round(launches_per_step * args.steps)) + 2 * nspec
 
     mdl = pass_model(n)
@@ -647,15 +649,15 @@ def run_ours(args, d: Dist):
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (FP64: N=128 scaled by M^2 H; FP32-bulk: N=256)",
                      "peak_source": hbm_src,
                      "algorithmic_bytes_per_launch": dom_bytes, "ms_per_launch": dom_ms,
-                     "note": ("HBM fraction of the FP64 form's dominant kernel, which is bound by the FP64 pipe "
-                              "(86 % of its cycles active in ncu): see fp64_roofline")
+                     "note": ("HBM fraction of the FP64 form's dominant kernel, whose transforms run in 64-bit fixed point: "
+                              "bound by instruction issue (61 % of the slots in ncu) and latency")
                      if args.precision == "fp64" else
                      ("FP32-bulk P3 (k_p3f): issue- and latency-bound in ncu at N=256 (53 % of issue slots, "
                       "global-load latency the top stall, 4 CTAs of 96 threads per SM)"
                       if dom == "P3_z_c2r_cross_r2c" else None)},
         "fp64_roofline": {"kernel": dom, "achieved": dom_gflops, "peak": fp64_peak, "unit": "GFLOP/s",
                           "frac": dom_gflops / fp64_peak, "peak_source": "measured live (FP64 FMA probe)",
-                          "note": "the FP64 form is bound by GB300's FP64 pipe, not HBM"}
+                          "note": "nominal flops against the FP64 pipe, which the fixed-point transforms hardly use: may exceed 1"}
         if args.precision == "fp64" else None,
         "passes": passes,
         "cpu_baseline": cpu,
