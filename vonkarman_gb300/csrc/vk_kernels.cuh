@@ -465,7 +465,9 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 // FP64 form of the stage epilogue, one mode per call.  The FP64 pipe (2 per
 // clock and SM) bounds it, so every product is fused and the factor s_out of
 // the nonlinear term (nl arrives without it) goes into the coefficients; the
-// operations are explicit, so that all instances round alike.  load() issues
+// operations are explicit, so that all instances round alike.  The state's term,
+// the largest by far, is one product to which the increment is added whole: two
+// roundings at its size, as many as the formulas have.  load() issues
 // the mode's global reads, apply() the arithmetic and the stores.
 struct StageF64 {
   struct Mode {
@@ -522,6 +524,10 @@ struct StageF64 {
   __device__ __forceinline__ static double2 mac(double a, double2 x, double2 y) {
     return make_double2(fma(a, x.x, y.x), fma(a, x.y, y.y));
   }
+  // 2 N3 - N1
+  __device__ __forceinline__ static double2 twice(double so2, double2 n3, double2 n1) {
+    return make_double2(fma(so2, n3.x, -n1.x), fma(so2, n3.y, -n1.y));
+  }
   __device__ __forceinline__ void apply(const Mode& md, const double2* nl, double2* un) const {
     const size_t cs = s.cs;
     switch (s.op) {
@@ -551,29 +557,29 @@ struct StageF64 {
         return;
       }
       case ST_ETD_REF_3: {  // solver.rs:318-344
-        const double q = dt * md.c1, q2 = 2.0 * q * so, b23 = md.c3 * so;
+        const double q = dt * md.c1, so2 = 2.0 * so, b23 = md.c3 * so;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           s.acc[c * cs + md.idx] = mac(b23, nl[c], md.b[c]);
-          s.temp[c * cs + md.idx] = mac(q2, nl[c], lin(-q, md.a[c], md.c0, md.u[c]));
+          s.temp[c * cs + md.idx] = lin(q, twice(so2, nl[c], md.a[c]), md.c0, md.u[c]);
         }
         return;
       }
       case ST_ETD_CM_3: {   // c = E2 a + (h/2) phi1(z/2) (2 N3 - N1), a rebuilt from u, N1
-        const double q = 0.5 * dt * md.c1, q2 = 2.0 * q * so, b23 = md.c3 * so;
+        const double q = 0.5 * dt * md.c1, so2 = 2.0 * so, b23 = md.c3 * so;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           s.acc[c * cs + md.idx] = mac(b23, nl[c], md.b[c]);
           const double2 av = lin(q, md.a[c], md.c0, md.u[c]);
-          s.temp[c * cs + md.idx] = mac(q2, nl[c], lin(-q, md.a[c], md.c0, av));
+          s.temp[c * cs + md.idx] = lin(q, twice(so2, nl[c], md.a[c]), md.c0, av);
         }
         return;
       }
       case ST_ETD_4: {      // solver.rs:354-378
-        const double b4 = dt * md.c1 * so;
+        const double b4 = md.c1 * so;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const double2 v = mac(b4, nl[c], lin(dt, md.b[c], md.c0, md.u[c]));
+          const double2 v = lin(dt, mac(b4, nl[c], md.b[c]), md.c0, md.u[c]);
           s.u_out[c * cs + md.idx] = v;
           flag_nonfinite<double>(s, v);
           un[c] = v;
