@@ -72,28 +72,29 @@ VK_FIX_HD fx2 fx_sub(fx2 a, fx2 b) { return fx2{a.x - b.x, a.y - b.y}; }
 template <bool INV> VK_FIX_HD fx2 fx_rot(fx2 a) { return INV ? fx2{-a.y, a.x} : fx2{a.y, -a.x}; }
 VK_FIX_HD fx2 fx_neg(fx2 a) { return fx2{-a.x, -a.y}; }
 
-// Rounding is to nearest even, or compensated to a mean of zero (short twiddles:
-// within an eighth of a unit): a bias that is the same in every line would add
-// up over the N^2 lines of a grid.
+// Rounding has no preferred direction and keeps zeros: shifts round to nearest
+// even, and of the two cross products of an operand a = h 2^32 + l with a factor
+// one is floored and the other rounded up, minus the floor of its negative.
+// Their means cancel, and a zero operand adds nothing.  A constant that
+// returned the floors' mean instead would turn an exact zero into a few units,
+// the same in every line, and these add up over the N^2 lines of a grid.
 // a w / 2^64, or a conj(w) / 2^64 for INV, of an |a| < 2^62 (so that the sum of
-// the four cross terms stays inside a word).  The four floors lose 1/2 each,
-// which r0 = 2 returns; the dropped low x low terms are below half a unit and
-// have mean zero.  Quarter turns have one component of zero, whose products
-// lose nothing, and take r0 = 1; w = 1 takes r0 = 0, and its products are exact
-// where a is a multiple of the factor 2^growth in the table's units (the stage
-// before rounds the outputs that meet it so: all inputs of one butterfly of a
-// line do).  The table holds r0 in the lowest two bits of cl, and no other low
-// word of zero.
+// the four cross terms stays inside a word); the dropped low x low terms are
+// below half a unit, of mean zero.  Which of the two is rounded up differs
+// between the terms of x and of y: the short components of quarter and twelfth
+// turns (low words of 1, fx_stage_twiddle) leave 1/16 or 1/32 of a unit, whose
+// signs so alternate over the turns that one butterfly meets.  The products of
+// w = 1 are exact where a is a multiple of the factor 2^growth in the table's units
+// (the stage before rounds the outputs that meet it so: all inputs of one
+// butterfly of a line do).
 template <bool INV> VK_FIX_HD fx2 fx_twiddle(fx2 a, fxtw w) {
   const fxsplit x = fx_split(a.x), y = fx_split(a.y);
-  const int r0 = w.cl & 3;
-  const int nh = -w.dh, nl = -w.dl;
-  const int ph = INV ? w.dh : nh, pl = INV ? w.dl : nl;   // y's factor in the real part
-  const int qh = INV ? nh : w.dh, ql = INV ? nl : w.dl;   // x's factor in the imaginary part
-  int t = fx_madhi(x.l, w.ch, fx_madhi(x.h, w.cl, r0));
-  t = fx_madhi(y.l, ph, fx_madhi(y.h, pl, t));
-  int s = fx_madhi(y.l, w.ch, fx_madhi(y.h, w.cl, r0));
-  s = fx_madhi(x.l, qh, fx_madhi(x.h, ql, s));
+  const int nc = -w.ch, nh = -w.dh, nl = -w.dl;
+  // y's factor in the real part (p) is minus x's in the imaginary part (q)
+  const int ph = INV ? w.dh : nh, pl = INV ? w.dl : nl;
+  const int qh = INV ? nh : w.dh, ql = INV ? nl : w.dl;
+  const int t = fx_madhi(x.h, w.cl, fx_madhi(y.l, ph, 0)) - fx_madhi(x.l, nc, fx_madhi(y.h, ql, 0));
+  const int s = fx_madhi(y.h, w.cl, fx_madhi(x.l, qh, 0)) - fx_madhi(y.l, nc, fx_madhi(x.h, pl, 0));
   return fx2{fx_wide(x.h, w.ch) + fx_wide(y.h, ph) + (long long)t, fx_wide(y.h, w.ch) + fx_wide(x.h, qh) + (long long)s};
 }
 // v plus what makes a floor to a multiple of 2^B round to nearest even
@@ -145,31 +146,27 @@ inline fxtw fx_make_twiddle(int m, int L, long double c, long double s) {
   fxtw w;
   words(c, w.ch, w.cl);
   words(-s, w.dh, w.dl);
-  if (m % L == 0) {
-    w.cl = w.dl = 0;
-  } else if (4 * (m % L) % L == 0) {   // (-1, 0) or (0, +-1)
-    w.cl = 1;
-    w.dl = 0;
-  } else {
-    w.cl = (w.cl & ~3) | 2;
-    if (w.dl == 0) w.dl = 1;
+  if (4 * (m % L) % L == 0) {   // the zeros of quarter turns exactly
+    if (2 * (m % L) % L == 0) w.dh = w.dl = 0;
+    else w.ch = w.cl = 0;
   }
   return w;
 }
-// the table's twiddle in the units of a stage of growth g
+// the table's twiddle in the units of a stage of growth g.  Short components
+// (other than of w = 1, whose products are exact) get a low word of 1: the term
+// that it adds is -1 for negative operands, which makes the rounding up of the other
+// term one away from zero.
 VK_FIX_HD fxtw fx_stage_twiddle(fxtw w, int g) {
-  const auto shift = [g](int& h, int& l) {
+  const bool one = w.ch > 0 && (w.dh | w.dl) == 0;
+  const auto shift = [g, one](int& h, int& l) {
     const long long v = ((long long)h * 4294967296ll + l) >> (g - 2);
     l = (int)(unsigned)(unsigned long long)v;
     h = (int)((v - (long long)l) >> 32);
     if (l == INT32_MIN) ++l;   // fx_twiddle negates it
+    if (l == 0 && h != 0 && !one) l = 1;
   };
-  const int r0 = w.cl & 3;
-  w.cl &= ~3;
   shift(w.ch, w.cl);
   shift(w.dh, w.dl);
-  w.cl = (w.cl & ~3) | r0;
-  if (r0 == 2 && w.dl == 0) w.dl = 1;
   return w;
 }
 
@@ -189,7 +186,7 @@ template <unsigned long long K, bool NEG> struct FxWords {
 template <unsigned long long K> VK_FIX_HD long long fx_mulc(long long v) {
   using W = FxWords<K, false>;
   const fxsplit s = fx_split(v);
-  return fx_wide(s.h, W::h) + (long long)fx_madhi(s.l, W::h, fx_madhi(s.h, W::l, 1));
+  return fx_wide(s.h, W::h) + (long long)(fx_madhi(s.h, W::l, 0) - fx_madhi(s.l, -W::h, 0));
 }
 // a exp(-+ 2 pi i M / 16) (INV: +)
 template <int M, bool INV> VK_FIX_HD fx2 fx_w16(fx2 a) {
@@ -209,10 +206,8 @@ template <int M, bool INV> VK_FIX_HD fx2 fx_w16(fx2 a) {
     using S = FxWords<FxConst::sn, !pos>;
     using T = FxWords<FxConst::sn, pos>;
     const fxsplit x = fx_split(a.x), y = fx_split(a.y);
-    int t = fx_madhi(x.l, C::h, fx_madhi(x.h, C::l, 2));
-    t = fx_madhi(y.l, S::h, fx_madhi(y.h, S::l, t));
-    int s = fx_madhi(y.l, C::h, fx_madhi(y.h, C::l, 2));
-    s = fx_madhi(x.l, T::h, fx_madhi(x.h, T::l, s));
+    const int t = fx_madhi(x.h, C::l, fx_madhi(y.l, S::h, 0)) - fx_madhi(x.l, -C::h, fx_madhi(y.h, T::l, 0));
+    const int s = fx_madhi(y.h, C::l, fx_madhi(x.l, T::h, 0)) - fx_madhi(y.l, -C::h, fx_madhi(x.h, S::l, 0));
     return fx2{fx_wide(x.h, C::h) + fx_wide(y.h, S::h) + (long long)t + a.x,
                fx_wide(y.h, C::h) + fx_wide(x.h, T::h) + (long long)s + a.y};
   }

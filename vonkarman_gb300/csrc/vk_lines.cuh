@@ -1152,10 +1152,11 @@ template <bool LEFT>   // s >= 0
 __device__ __forceinline__ long long fx_shl(long long v, int s) {   // v 2^s, rounded for s < 0
   return LEFT || s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
 }
-// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split): the
-// floors of the two products' cross terms cancel in the mean
+// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split): of
+// each product's cross terms one is floored and one rounded up, so that the
+// means cancel and a product with a zero factor is zero
 __device__ __forceinline__ long long fx_det(fxsplit a, fxsplit b, fxsplit c, fxsplit d) {
-  const int t = fx_madhi(a.l, b.h, fx_madhi(a.h, b.l, 0)), u = fx_madhi(c.l, d.h, fx_madhi(c.h, d.l, 0));
+  const int t = fx_madhi(a.h, b.l, fx_madhi(c.l, -d.h, 0)), u = fx_madhi(c.h, d.l, fx_madhi(a.l, -b.h, 0));
   return fx_wide(a.h, b.h) - fx_wide(c.h, d.h) + (long long)(t - u);
 }
 // u x omega at one position of a column (parts exchanged), lines at stride ls
