@@ -147,7 +147,8 @@ template <typename R, int GN = 0, int GM = 0> struct OpAdjYInv {
 //   (u_x + i u_y), (u_z + i w_x), (w_y + i w_z), (cb_x + i cb_y), and
 //   (cb_z of column 0 + i cb_z of column 1) shared by a column pair;
 // after the inverse FFT: a_bar = w x cb, o_bar = cb x u; per column three
-// forward lines (ab_x + i ab_y), (ab_z + i ob_x), (ob_y + i ob_z).
+// forward lines (ab_x + i ab_y), (ab_z + i ob_x), (ob_y + i ob_z).  FP64: every line
+// holds one field of a column pair (k_adj_zx).
 // Output fields: ab_x, ab_y, ab_z, ob_x, ob_y, ob_z, each (M, M, H).
 template <typename R> struct A3Args {
   int ncols;
@@ -185,12 +186,12 @@ struct AdjZRowUnpack {
   }
 };
 
-// On the register engine: inverse lines l < 8 CP are the packed pair
+// On the register engine (FP32): inverse lines l < 8 CP are the packed pair
 // t = l / 2CP of column c = l % 2CP; lines 8 CP + pr carry c_bar_z of the two
 // columns of pair pr.  Forward lines l = t * 2CP + c: (ab_x + i ab_y),
 // (ab_z + i ob_x), (ob_y + i ob_z) of column c.
 template <typename R, int M, int CP, int NT>
-__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? fx_min_blocks<M, NT>() : M >= 768 ? 1 : cmax(1, 512 / NT))
+__global__ void __launch_bounds__(NT, M >= 768 ? 1 : cmax(1, 512 / NT))
 k_adj_z(A3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int N = 2 * M / 3;
   constexpr int H = N / 2 + 1;
@@ -198,10 +199,9 @@ k_adj_z(A3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr int NI = 9 * CP, NF = 6 * CP;
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, true>(M)];
-  // L2 prefetch of the nine input ranges of the CTA pf blocks ahead (FP32:
-  // per field 2 CP columns of H complex values, a multiple of 16 bytes at a
-  // 16-byte boundary)
-  if constexpr (sizeof(R) == 4) {
+  // L2 prefetch of the nine input ranges of the CTA pf blocks ahead (per field
+  // 2 CP columns of H complex values, a multiple of 16 bytes at a 16-byte boundary)
+  {
     const int b = (int)blockIdx.x + pf;
     if (pf > 0 && threadIdx.x < 9 && b < (int)gridDim.x && (b + 1) * 2 * CP <= a.ncols)
       prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fsin + (size_t)b * (2 * CP * H), 2 * CP * H * sizeof(C2<R>));
@@ -281,6 +281,71 @@ k_adj_z(A3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
     zunpack<R>(B + (t * 2 * CP + c) * LP, M, k, X, Y);
     a.out[(size_t)(2 * t) * a.fsout + (size_t)col * H + k] = X;
     a.out[(size_t)(2 * t + 1) * a.fsout + (size_t)col * H + k] = Y;
+  }
+}
+
+// The FP64 form: inverse lines l = f CP + pr (field f of the two columns of pair pr),
+// the products in doubles, forward lines the same with the six products.
+template <int M, int CP, int NT>
+__global__ void __launch_bounds__(NT, fx_min_blocks<M, NT>())
+k_adj_zx(A3Args<double> a, const double2* __restrict__ tw) {
+  constexpr int N = 2 * M / 3;
+  constexpr int H = N / 2 + 1;
+  constexpr int LP = zpad_len<double>(M);
+  constexpr int NI = 9 * CP, NF = 6 * CP;
+  using Inv = FxLines<M, true, NT, NI, MapContig<double, M, NI>, true, H, M - H + 1>;
+  using Fwd = FxLines<M, false, NT, NF, MapContig<double, M, NF>, true, 0, 0>;
+  extern __shared__ __align__(16) unsigned char vk_smem[];
+  __shared__ double2 tw_s[twtab_elems<double, true>(M)];
+  __shared__ int part[Fwd::PARTS], line_q[NF];
+  load_twtab<double, M, true, NT>(tw_s, tw);
+  grid_depend();
+  double2* A = reinterpret_cast<double2*>(vk_smem);   // NI lines
+  double2* B = A + NI * LP;                           // NF lines
+  const fxtw* twx = reinterpret_cast<const fxtw*>(tw_s);
+  const int col0 = blockIdx.x * 2 * CP;
+  const auto ld = [&](int l, int p) -> C2x2<double> {
+    const int f = l / CP, c = col0 + 2 * (l - f * CP);
+    const bool lo = p < H;
+    C2x2<double> r{};
+    if (lo || p > M - H) {
+      const double2* src = a.in + (size_t)f * a.fsin + (size_t)c * H + (lo ? p : M - p);
+      if (c < a.ncols) r.a = src[0];
+      if (c + 1 < a.ncols) r.b = src[H];
+    }
+    return r;
+  };
+  Inv::run(
+      reinterpret_cast<fx2*>(A), twx, FxFill<M, H, M - H + 1, decltype(ld), ZPack<double, M>>{ld, ZPack<double, M>{}},
+      [&](int l, int p, double2 v) { A[l * LP + zi<double>(p)] = v; }, 0);
+  __syncthreads();
+  for (int e = threadIdx.x; e < CP * M; e += NT) {
+    const int pr = e / M, zp = zi<double>(e % M);
+    double2 v[9];   // u, omega, c_bar of the two columns
+#pragma unroll
+    for (int f = 0; f < 9; ++f) v[f] = A[(f * CP + pr) * LP + zp];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int j = (i + 1) % 3, k = (i + 2) % 3;
+      const double2 *u = v, *w = v + 3, *c = v + 6;
+      // a_bar = w x cb ; o_bar = cb x u
+      B[(i * CP + pr) * LP + zp] = make_double2(w[j].x * c[k].x - w[k].x * c[j].x, w[j].y * c[k].y - w[k].y * c[j].y);
+      B[((3 + i) * CP + pr) * LP + zp] =
+          make_double2(c[j].x * u[k].x - c[k].x * u[j].x, c[j].y * u[k].y - c[k].y * u[j].y);
+    }
+  }
+  __syncthreads();
+  fx2* z = reinterpret_cast<fx2*>(A);
+  const auto products = [&](int l, int p) { return B[l * LP + zi<double>(p)]; };
+  Fwd::run_integers(z, twx, FxFill<M, 0, 0, decltype(products), PrepNone>{products, PrepNone{}}, part, line_q);
+  for (int e = threadIdx.x; e < NF * H; e += NT) {
+    const int l = e / H, k = e - l * H;
+    const int f = l / CP, c = col0 + 2 * (l - f * CP);
+    double2 X, Y;
+    fx_unpack(z[l * LP + zi<double>(k)], z[l * LP + zi<double>(k == 0 ? 0 : M - k)], line_q[l], X, Y);
+    double2* dst = a.out + (size_t)f * a.fsout + (size_t)c * H + k;
+    if (c < a.ncols) dst[0] = X;
+    if (c + 1 < a.ncols) dst[H] = Y;
   }
 }
 

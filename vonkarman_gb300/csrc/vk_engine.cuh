@@ -309,12 +309,19 @@ inline cudaError_t nla_n(const NlaParams<R>& p, cudaStream_t s) {
     constexpr int CP = zcross_pairs<R, M>();
     constexpr int NT = adj_z_threads<R, M, CP>();
     const size_t smem = (size_t)adj_z_smem_elems<R, M, CP>() * sizeof(C2<R>);
-    constexpr auto kern = k_adj_z<R, M, CP, NT>;
-    e = prepare_kernel<kern>(smem);
-    if (e != cudaSuccess) return e;
     A3Args<R> a{M * M, p.bufB, fsB2, p.bufA, fsA3};
     const int nb = (M * M + 2 * CP - 1) / (2 * CP);
-    e = launch_overlapped(kern, nb, NT, smem, s, true, a, p.twM, zpass_prefetch_distance<R, kern>(NT, smem));
+    if constexpr (sizeof(R) == 8) {
+      constexpr auto kern = k_adj_zx<M, CP, NT>;
+      e = prepare_kernel<kern>(smem);
+      if (e != cudaSuccess) return e;
+      e = launch_overlapped(kern, nb, NT, smem, s, true, a, p.twM);
+    } else {
+      constexpr auto kern = k_adj_z<R, M, CP, NT>;
+      e = prepare_kernel<kern>(smem);
+      if (e != cudaSuccess) return e;
+      e = launch_overlapped(kern, nb, NT, smem, s, true, a, p.twM, zpass_prefetch_distance<R, kern>(NT, smem));
+    }
     if (e != cudaSuccess) return e;
   }
   {

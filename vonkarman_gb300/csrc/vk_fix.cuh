@@ -125,14 +125,15 @@ VK_FIX_HD constexpr int fx_radix1(int L) { return fx_stages(L) == 2 ? L / fx_rad
 VK_FIX_HD constexpr int fx_radix(int L, int s) {
   return s == 0 ? fx_radix0(L) : s == 1 ? fx_radix1(L) : L / fx_radix0(L) / fx_radix1(L);
 }
-// log2 of the factor that the twiddles of a later stage of radix r divide by;
+// log2 of the factor that the twiddles of a later stage (radix up to 8) divide by;
 // their components are held in units of 2^-(64 - growth), which makes
 // fx_twiddle's a w / 2^64 the scaled product
-VK_FIX_HD constexpr int fx_growth(int r) { return r <= 8 ? 3 : r <= 16 ? 4 : 5; }
+constexpr int FX_GROWTH = 3;
+VK_FIX_HD constexpr int fx_growth(int) { return FX_GROWTH; }
 // sum of the growths of a plan's stages: the outputs' exponent above the quantum
 VK_FIX_HD constexpr int fx_total_growth(int L) {
   int g = 0;
-  for (int s = 1; s < fx_stages(L); ++s) g += fx_growth(fx_radix(L, s));
+  for (int s = 1; s < fx_stages(L); ++s) g += fx_radix(L, s) <= 8 ? FX_GROWTH : 64;
   return g;
 }
 // W_L^m = c - i s (cosine and sine of 2 pi m / L) in units of 2^-62 (host)
@@ -322,7 +323,7 @@ template <bool INV> struct FxDft<12, INV> {
 // denormals, far below the quantum of a line of normal range) shift out.
 VK_FIX_HD long long fx_from_double(int hi, int lo, int k) {
   // k - exponent, from the sign-cleared high word (its mantissa bits add less than one)
-  const int r = ((k << 20) + 0xfffff - (hi & 0x7fffffff)) >> 20;
+  const unsigned r = (((unsigned)k << 20) + 0xfffffu - ((unsigned)hi & 0x7fffffffu)) >> 20;
   const unsigned mh = ((((unsigned)hi << 10) | ((unsigned)lo >> 22)) & 0x3fffffffu) | 0x40000000u;
   unsigned long long m = ((unsigned long long)mh << 32) | ((unsigned)lo << 10);
 #ifdef __CUDA_ARCH__

@@ -297,7 +297,7 @@ struct RegStage {
   }
 };
 
-// FP64 lines in fixed point.  The outputs are multiplied by 2^xe.
+// FP64 lines in fixed point.
 //
 // Stage 0: one butterfly per thread.  Its bound of the inputs' magnitudes
 // (fx_bound) is maximised over the line's threads, by shuffles where a line's
@@ -307,17 +307,17 @@ struct RegStage {
 // back into the exchange buffer), so that a CTA needs no more threads than stage
 // 0 keeps busy.
 //
-// Lines whose bound is outside the comfortable range carry a code: all zero
-// (the transform's rounding compensations would leave a few units), tiny and
-// huge (scaled by 2^+-FX_RANGE on the way in and back on the way out) or with a
-// NaN or Inf among the inputs (every output is NaN).
-constexpr int FX_RANGE = 600;
-enum FxCode : int { FX_PLAIN = 0, FX_ZERO = 1, FX_TINY = 2, FX_HUGE = 3, FX_NAN = 4 };
-__device__ __forceinline__ double fx_code_factor(int code) {
-  return code == FX_ZERO ? 0.0
-       : code == FX_TINY ? __hiloint2double((1023 - FX_RANGE) << 20, 0)
-       : code == FX_HUGE ? __hiloint2double((1023 + FX_RANGE) << 20, 0)
-                         : __longlong_as_double(0x7ff8000000000000ll);
+// Contiguous lines carry two real lines, Z = X + i Y: one field at two neighbouring
+// columns, which are of one size as a rule, as they share the exponent.
+
+// The exponent of an output, v 2^q; FX_Q_NAN where an input is a NaN or an
+// infinity: every output of the line is NaN.
+constexpr int FX_Q_NAN = 1 << 24;
+constexpr int FX_K_NAN = 0x7fff;   // the bound of such inputs
+// bounds below FX_K_LOW may come from denormals, which 2^FX_UP makes normal
+constexpr int FX_K_LOW = 80, FX_UP = 200;
+__device__ __forceinline__ int fx_line_q(int k, int growth) {
+  return k == FX_K_NAN ? FX_Q_NAN : fx_quantum(k) + growth;
 }
 // v 2^q, q20 = q << 20 (within the normal range)
 __device__ __forceinline__ double fx_to_double(long long v, int q20) {
@@ -325,39 +325,66 @@ __device__ __forceinline__ double fx_to_double(long long v, int q20) {
   const int h = __double2hiint(d);
   return __hiloint2double(h != 0 ? h + q20 : 0, __double2loint(d));
 }
-
-// State of a line between the stages: output exponent and FxCode.
-struct FxState { int q, code; };
+// Exponents outside [-960, 900] are split: the first factor leaves every |v| >= 1
+// normal, the second (the rest, or a NaN) rounds once.
+__device__ __forceinline__ int fx_near_q(int q) { return min(max(q, -960), 900); }
+__device__ __forceinline__ double fx_rest(int q) {
+  const int rest = q - fx_near_q(q);
+  return q >= FX_Q_NAN / 2 ? __longlong_as_double(0x7ff8000000000000ll)
+                           : __hiloint2double((1023 + min(max(rest, -1000), 1000)) << 20, 0);
+}
+// Integers as doubles, put(r, u 2^q).  Two texts, so that the usual one converts and
+// stores value by value (with the rest's factor as a branch before the stores: N = 256
+// P2 1.21 ms against 1.18, P4 0.56 against 0.53).
+template <int R, class PUT> __device__ __forceinline__ void fx_results(const fx2* u, int q, const PUT& put) {
+  const int n = fx_near_q(q), h = n << 20;
+  if (n == q) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) put(r, make_double2(fx_to_double(u[r].x, h), fx_to_double(u[r].y, h)));
+  } else {
+    long long any = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) any |= u[r].x | u[r].y;
+    const double f = any == 0 && q < FX_Q_NAN / 2 ? 1.0 : fx_rest(q);
+    const bool scale = f != 1.0;   // (lines of zeros pass without the FP64 pipe)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      double2 d = make_double2(fx_to_double(u[r].x, h), fx_to_double(u[r].y, h));
+      if (scale) d = make_double2(d.x * f, d.y * f);
+      put(r, d);
+    }
+  }
+}
+__device__ __forceinline__ int fx_magnitude(double2 v) {
+  return max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff);
+}
+__device__ __forceinline__ long long fx_integer(double v, int k) {
+  return fx_from_double(__double2hiint(v), __double2loint(v), k);
+}
 
 // words that the maximum over a contiguous line's threads takes in shared memory
 template <int L, int NLINES> __host__ __device__ constexpr int fx_contig_parts() {
   return 32 % (L / fx_radix(L, 0)) == 0 ? 1 : L / fx_radix(L, 0) * NLINES / 16;
 }
-template <int L, int NT, int NLINES, class MAP>
-__host__ __device__ constexpr int fx_round_lines() {   // lines per stage-1 round (contiguous lines)
-  return cmin(NT / (L / fx_radix(L, fx_stages(L) - 1)), NLINES);
-}
 
+// SL: the last stage writes back into the exchange.
 template <int L, bool INV, int NT, int NLINES, class MAP, bool SL, int Z0, int Z1>
 struct FxLines {
   static constexpr int ST = fx_stages(L);
   static constexpr int R0 = fx_radix(L, 0), NB0 = L / R0, G0 = NB0 * NLINES;
-  // the last stage: radix, butterflies, growth, and its twiddles' place in the table
+  // the last stage: radix, butterflies, and its twiddles' place in the table
   static constexpr int R1 = fx_radix(L, ST - 1), NB1 = L / R1, G1 = NB1 * NLINES;
-  static constexpr int GR = fx_growth(R1);
   static constexpr int TW1 = twtab_off<double, MAP::CONTIG>(L, ST - 1);
   static constexpr int TG = fx_total_growth(L);
-  // growth of the stage after the first
-  static constexpr int GN = fx_growth(fx_radix(L, 1));
   static constexpr unsigned ZM = zero_mask(NB0, R0, Z0, Z1);
   static constexpr int NW0 = (G0 + 31) / 32;
-  static constexpr int CODE_SHIFT = 24;   // stored line state: exponent + (code << 24)
   static_assert(G0 <= NT, "one first-stage butterfly per thread");
   static_assert(!MAP::CONTIG || 32 % NB0 == 0 || NB0 % 16 == 0, "groups of lanes keep one contiguous line");
-  // words of the part array of front and line_max
+  // words of the part array of line_max
   static constexpr int PARTS = MAP::CONTIG ? fx_contig_parts<L, NLINES>() : NW0 * NLINES;
   static_assert(MAP::CONTIG || (32 % NLINES == 0 && !SL), "interleaved lines tile a warp");
 
+  // maximum over a line's threads
   __device__ __forceinline__ static int line_max(int m, int* part) {
     if constexpr (MAP::CONTIG && 32 % NB0 == 0) {
 #pragma unroll
@@ -385,18 +412,11 @@ struct FxLines {
     return m;
   }
 
-  using State = FxState;
-  __device__ __forceinline__ static int pack_state(int q, int code) { return q + (code << CODE_SHIFT); }
-  __device__ __forceinline__ static State unpack_state(int s) {
-    const int code = (s + (1 << (CODE_SHIFT - 1))) >> CODE_SHIFT;
-    return State{s - (code << CODE_SHIFT), code};
-  }
-
-  // Stage 0 from doubles.  fill(l, j, d): the inputs at positions j + r NB0 of
-  // line l (those of ZM excepted).  The state of the thread's line is returned
-  // (interleaved: valid in every thread; contiguous: also in line_s[l]).
+  // Stage 0 from doubles.  fill(l, j, d): the inputs at positions j + r NB0 of line l
+  // (those of ZM excepted).  Returns the exponent of the thread's line (interleaved:
+  // the line of the thread in all stages; contiguous: also in line_q[l]).
   template <class FILL>
-  __device__ __forceinline__ static State front(fx2* xb, const FILL& fill, int* part, int* line_s, int xe) {
+  __device__ __forceinline__ static int front(fx2* xb, const FILL& fill, int* part, int* line_q) {
     const int g = threadIdx.x;
     const int l0 = MAP::template line<NB0>(g), j0 = MAP::template bfly<NB0>(g);
     const bool act = G0 == NT || g < G0;
@@ -409,73 +429,66 @@ struct FxLines {
       int top = 0;
 #pragma unroll
       for (int r = 0; r < R0; ++r)
-        if (!((ZM >> r) & 1u))
-          top = max(top, max(__double2hiint(d[r].x) & 0x7fffffff, __double2hiint(d[r].y) & 0x7fffffff));
+        if (!((ZM >> r) & 1u)) top = max(top, fx_magnitude(d[r]));
       float sum = 0.f;
 #pragma unroll
       for (int r = 0; r < R0; ++r)
-        if (!((ZM >> r) & 1u))
-          sum += fx_relative(max(__double2hiint(d[r].x) & 0x7fffffff, __double2hiint(d[r].y) & 0x7fffffff), top);
-      k = top == 0 ? 0 : top >= 0x7ff00000 ? 0x7fff : fx_bound(top, sum);
+        if (!((ZM >> r) & 1u)) sum += fx_relative(fx_magnitude(d[r]), top);
+      k = top == 0 ? 0 : top >= 0x7ff00000 ? FX_K_NAN : fx_bound(top, sum);
     }
-    k = line_max(k, part);
-    int code = FX_PLAIN;
-    if (k < 1023 - 900 || k > 1023 + 900) {
-      code = k == 0 ? FX_ZERO : k == 0x7fff ? FX_NAN : k < 1023 ? FX_TINY : FX_HUGE;
-      k = code == FX_TINY ? k + FX_RANGE : code == FX_HUGE ? k - FX_RANGE : 1023;
+    k = max(line_max(k, part), 1);
+    int up = 0;
+    if (k < FX_K_LOW) {   // 2^up makes denormals normal
+      up = FX_UP;
+      k += up;
       if (act) {
-        const double f = code == FX_TINY ? fx_code_factor(FX_HUGE) : code == FX_HUGE ? fx_code_factor(FX_TINY) : 0.0;
+        int any = 0;
 #pragma unroll
-        for (int r = 0; r < R0; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
+        for (int r = 0; r < R0; ++r)
+          if (!((ZM >> r) & 1u)) any |= fx_magnitude(d[r]) | __double2loint(d[r].x) | __double2loint(d[r].y);
+        if (any != 0) {
+          const double f = __hiloint2double((1023 + FX_UP) << 20, 0);
+#pragma unroll
+          for (int r = 0; r < R0; ++r)
+            if (!((ZM >> r) & 1u)) d[r] = make_double2(d[r].x * f, d[r].y * f);
+        }
       }
     }
-    const int q = fx_quantum(k) + TG + xe;
+    const int q = fx_line_q(k, TG) - up;
     if (act) {
       fx2 v[R0];
 #pragma unroll
-      for (int r = 0; r < R0; ++r) {
-        if ((ZM >> r) & 1u) {
-          v[r] = fx2{0, 0};
-        } else {
-          v[r].x = fx_from_double(__double2hiint(d[r].x), __double2loint(d[r].x), k);
-          v[r].y = fx_from_double(__double2hiint(d[r].y), __double2loint(d[r].y), k);
-        }
-      }
-      if (MAP::CONTIG && j0 == 0) line_s[l0] = pack_state(q, code);
-      fx2* dst = xb + MAP::template idx<0>(j0 * R0, l0);
-      first_dft(v, [&](int r, fx2 z) { dst[MAP::template step<1, R0>(j0 * R0, r)] = z; });
+      for (int r = 0; r < R0; ++r)
+        v[r] = (ZM >> r) & 1u ? fx2{0, 0} : fx2{fx_integer(d[r].x, k), fx_integer(d[r].y, k)};
+      if (MAP::CONTIG && j0 == 0) line_q[l0] = q;
+      first_dft(v, xb, l0, j0);
     }
-    return State{q, code};
+    return q;
   }
-  // a first-stage butterfly: put(r, value) into the exchange
-  template <class PUT>
-  __device__ __forceinline__ static void first_dft(fx2* v, const PUT& put) {
+
+  // a first-stage butterfly into the exchange
+  __device__ __forceinline__ static void first_dft(fx2* v, fx2* xb, int l, int j) {
     FxDft<R0, INV>::run(v);
-    sfor<R0>([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      if constexpr (r == 0) v[r] = fx_multiple<GN>(v[r]);
-      put(r, v[r]);
-    });
+    v[0] = fx_multiple<FX_GROWTH>(v[0]);
+    fx2* dst = xb + MAP::template idx<0>(j * R0, l);
+#pragma unroll
+    for (int r = 0; r < R0; ++r) dst[MAP::template step<1, R0>(j * R0, r)] = v[r];
   }
   // twiddles and DFT of a later stage's butterfly: twiddle index k of ns
   template <int RAD, int OFF>
   __device__ __forceinline__ static void later_dft(fx2* u, const fxtw* __restrict__ tw, int k, int ns) {
-    u[0] = fx_shift<fx_growth(RAD)>(u[0]);
+    u[0] = fx_shift<FX_GROWTH>(u[0]);
 #pragma unroll
     for (int r = 1; r < RAD; ++r) u[r] = fx_twiddle<INV>(u[r], tw[OFF + (r - 1) * ns + k]);
     FxDft<RAD, INV>::run(u);
   }
-  __device__ __forceinline__ static void last_dft(fx2* u, const fxtw* __restrict__ tw, int j) {
-    later_dft<R1, TW1>(u, tw, j, NB1);
-  }
-  // The middle stage of a three-stage plan, in place (begins and ends with the
-  // exchange complete).
-  __device__ __forceinline__ static void middle(fx2* xb, const fxtw* __restrict__ tw) {
+  // The middle stage of a three-stage plan on nl lines, in place (begins with the
+  // exchange complete and ends so).
+  __device__ __forceinline__ static void middle(fx2* xb, const fxtw* __restrict__ tw, int nl) {
     constexpr int RM = fx_radix(L, 1), NBM = L / RM, GM = NBM * NLINES;
     static_assert(GM <= NT, "one butterfly per thread");
-    const int g = threadIdx.x;
-    const int l = MAP::template line<NBM>(g), j = MAP::template bfly<NBM>(g);
-    const bool act = GM == NT || g < GM;
+    const int l = MAP::template line<NBM>(threadIdx.x), j = MAP::template bfly<NBM>(threadIdx.x);
+    const bool act = MAP::CONTIG ? l < nl : GM == NT || (int)threadIdx.x < GM;
     fx2 u[RM];
     if (act) {
       __builtin_assume(j >= 0 && j < NBM);
@@ -488,7 +501,7 @@ struct FxLines {
     if (act) {
       const int k = j % R0;
       later_dft<RM, 0>(u, tw, k, R0);
-      u[0] = fx_multiple<GR>(u[0]);
+      u[0] = fx_multiple<FX_GROWTH>(u[0]);
       const int p0 = (j - k) * RM + k;
       fx2* dst = xb + MAP::template idx<0>(p0, l);
 #pragma unroll
@@ -496,119 +509,81 @@ struct FxLines {
     }
     __syncthreads();
   }
-
-  // the same for nl contiguous lines, line l at xs + l ls
-  __device__ __forceinline__ static void middle_rt(fx2* xs, int ls, int nl, const fxtw* __restrict__ tw) {
-    constexpr int RM = fx_radix(L, 1), NBM = L / RM;
-    static_assert(NBM * NLINES <= NT, "one butterfly per thread");
-    const int l = threadIdx.x / NBM, j = threadIdx.x % NBM;
-    __builtin_assume(j >= 0 && j < NBM);
-    const bool act = l < nl;
-    fx2 u[RM];
-    if (act) {
-      const fx2* src = xs + l * ls + zi<double>(j);
-#pragma unroll
-      for (int r = 0; r < RM; ++r) u[r] = src[MAP::template step<NBM, 1>(j, r)];
-    }
-    __syncthreads();
-    if (act) {
-      const int k = j % R0;
-      later_dft<RM, 0>(u, tw, k, R0);
-      u[0] = fx_multiple<GR>(u[0]);
-      const int p0 = (j - k) * RM + k;
-      fx2* dst = xs + l * ls + zi<double>(p0);
-#pragma unroll
-      for (int r = 0; r < RM; ++r) dst[MAP::template step<R0, 1>(p0, r)] = u[r];
-    }
-    __syncthreads();
-  }
-
-  // The last stage, in rounds (whole lines, or butterflies of all lines); the
-  // exchange is complete.  em(u, l, j, state) takes a butterfly's outputs
-  // (positions j + r NB1).
+  // The last stage of nl lines, in rounds (whole lines, or butterflies of all
+  // lines); the exchange is complete.  em(u, l, j) takes a butterfly's outputs
+  // (positions j + r NB1), all threads of whose line have read theirs (SL).
   template <class EM>
-  __device__ __forceinline__ static void back(const fx2* xb, const fxtw* __restrict__ tw, const int* line_s, State st0,
-                                              const EM& em) {
-    constexpr int RL = MAP::CONTIG ? fx_round_lines<L, NT, NLINES, MAP>() : NLINES;
-    constexpr int PER = MAP::CONTIG ? RL * NB1 : NT;                 // butterflies per round
-    constexpr int ROUNDS = MAP::CONTIG ? (NLINES + RL - 1) / RL : (G1 + NT - 1) / NT;
+  __device__ __forceinline__ static void back(const fx2* xb, const fxtw* __restrict__ tw, int nl, const EM& em) {
+    constexpr int RL = MAP::CONTIG ? cmin(NT / NB1, NLINES) : NLINES;   // lines of a round
+    constexpr int PER = MAP::CONTIG ? RL * NB1 : NT;                    // butterflies of a round
     static_assert(RL >= 1, "a round holds a line");
-    const int g = threadIdx.x;
+    const int total = MAP::CONTIG ? nl * NB1 : G1;
 #pragma unroll 1
-    for (int i = 0; i < ROUNDS; ++i) {
-      const int gi = i * PER + g;
-      const int l = MAP::template line<NB1>(gi), j = MAP::template bfly<NB1>(gi);
-      const bool act = (PER == NT || g < PER) && (G1 % PER == 0 || gi < G1);
+    for (int g0 = 0; g0 < total; g0 += PER) {
+      const int g = g0 + (int)threadIdx.x;
+      const int l = MAP::template line<NB1>(g), j = MAP::template bfly<NB1>(g);
+      const bool act = (PER == NT || (int)threadIdx.x < PER) && g < total;
       fx2 u[R1];
-      State st = st0;
       if (act) {
         __builtin_assume(j >= 0 && j < NB1);
         __builtin_assume(l >= 0 && l < NLINES);
-        if (MAP::CONTIG) st = unpack_state(line_s[l]);
         const fx2* src = xb + MAP::template idx<0>(j, l);
 #pragma unroll
         for (int r = 0; r < R1; ++r) u[r] = src[MAP::template step<NB1, 1>(j, r)];
       }
       if constexpr (SL) __syncthreads();
       if (act) {
-        last_dft(u, tw, j);
-        em(u, l, j, st);
-      }
-    }
-  }
-
-  // The last stage of nl contiguous lines, line l at xs + l ls, written back in place
-  // or to lines that no thread reads: em(u, l, j).
-  template <class EM>
-  __device__ __forceinline__ static void back_rt(const fx2* xs, int ls, int nl, const fxtw* __restrict__ tw,
-                                                 const EM& em) {
-    constexpr int RL = fx_round_lines<L, NT, NLINES, MAP>();
-    const int lr = threadIdx.x / NB1, j = threadIdx.x % NB1;
-    __builtin_assume(j >= 0 && j < NB1);
-#pragma unroll 1
-    for (int l0 = 0; l0 < nl; l0 += RL) {
-      const int l = l0 + lr;
-      const bool act = lr < RL && l < nl;
-      fx2 u[R1];
-      if (act) {
-        const fx2* src = xs + l * ls + zi<double>(j);
-#pragma unroll
-        for (int r = 0; r < R1; ++r) u[r] = src[MAP::template step<NB1, 1>(j, r)];
-      }
-      __syncthreads();
-      if (act) {
-        last_dft(u, tw, j);
+        later_dft<R1, TW1>(u, tw, j, NB1);
         em(u, l, j);
       }
     }
   }
 
-  // The whole transform from doubles to doubles: st(l, p, v).
+  // From doubles to doubles, times 2^xe: st(l, p, v).
   template <class FILL, class STF>
   __device__ __forceinline__ static void run(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, const STF& st,
                                              int xe) {
     __shared__ int part[PARTS];
-    __shared__ int line_s[MAP::CONTIG ? NLINES : 1];
-    const State s0 = front(xb, fill, part, line_s, xe);
+    __shared__ int line_q[MAP::CONTIG ? NLINES : 1];
+    const int q0 = front(xb, fill, part, line_q);
     __syncthreads();
-    if constexpr (ST == 3) middle(xb, tw);
-    back(xb, tw, line_s, s0, [&](const fx2* u, int l, int j, State s) {
-      double2 d[R1];
-      const int q20 = s.q << 20;
-#pragma unroll
-      for (int r = 0; r < R1; ++r) d[r] = make_double2(fx_to_double(u[r].x, q20), fx_to_double(u[r].y, q20));
-      if (s.code != FX_PLAIN) {
-        const double f = fx_code_factor(s.code);
-#pragma unroll
-        for (int r = 0; r < R1; ++r) d[r] = make_double2(d[r].x * f, d[r].y * f);
-      }
-#pragma unroll
-      for (int r = 0; r < R1; ++r) st(l, j + r * NB1, d[r]);
+    if constexpr (ST == 3) middle(xb, tw, NLINES);
+    back(xb, tw, NLINES, [&](const fx2* u, int l, int j) {
+      fx_results<R1>(u, (MAP::CONTIG ? line_q[l] : q0) + xe, [&](int r, double2 v) { st(l, j + r * NB1, v); });
     });
+  }
+  // From doubles to integers in the exchange, with the exponents line_q (contiguous
+  // lines): see fx_unpack.
+  template <class FILL>
+  __device__ __forceinline__ static void run_integers(fx2* xb, const fxtw* __restrict__ tw, const FILL& fill, int* part,
+                                                      int* line_q) {
+    static_assert(MAP::CONTIG && SL, "in place");
+    front(xb, fill, part, line_q);
+    __syncthreads();
+    if constexpr (ST == 3) middle(xb, tw, NLINES);
+    back(xb, tw, NLINES, [&](const fx2* u, int l, int j) {
+      fx2* dst = xb + MAP::template idx<0>(j, l);
+#pragma unroll
+      for (int r = 0; r < R1; ++r) dst[MAP::template step<NB1, 1>(j, r)] = u[r];
+    });
+    __syncthreads();
   }
 };
 
-// fill functor of FxLines from ld / pp: all loads of a chunk are issued before
+// Mode k of X and Y from a line of Z: z and its mirror image w, exponent q
+// (X = (z + conj w) / 2, Y = (z - conj w) / 2i).
+__device__ __forceinline__ void fx_unpack(fx2 z, fx2 w, int q, double2& X, double2& Y) {
+  const int n = fx_near_q(--q), h = n << 20;
+  X = make_double2(fx_to_double(z.x + w.x, h), fx_to_double(z.y - w.y, h));
+  Y = make_double2(fx_to_double(z.y + w.y, h), fx_to_double(w.x - z.x, h));
+  if (n != q) {
+    const double f = fx_rest(q);
+    X = make_double2(X.x * f, X.y * f);
+    Y = make_double2(Y.x * f, Y.y * f);
+  }
+}
+
+// fill functor of FxLines::front from ld / pp: all loads of a chunk are issued before
 // any arithmetic on them (chunks of 256 bytes per thread where the raw inputs
 // are wider than one complex value)
 template <int L, int Z0, int Z1, class LD, class PP> struct FxFill {
@@ -632,7 +607,7 @@ template <int L, int Z0, int Z1, class LD, class PP> struct FxFill {
   }
 };
 
-// Transform NLINES lines.  All NT threads must call it; the exchange buffer
+// Transform NLINES lines (FP32).  All NT threads must call it; the exchange buffer
 // xb (MAP::elems() elements) must not be in use by any thread.  Returns with
 // no synchronisation after the last stage.
 // SL: the store functor writes into xb itself (in place), so the last stage
@@ -642,18 +617,20 @@ template <typename R, int L, bool INV, int NT, int NLINES, class MAP = MapInterl
           bool TT = false, int Z0 = 0, int Z1 = 0, class LD, class PP, class ST>
 __device__ __forceinline__ void fft_lines(C2<R>* xb, const C2<R>* __restrict__ tw, const LD& ld, const PP& pp,
                                           const ST& st) {
-  static_assert(rstages<R>(L) > 0, "unsupported FFT length");
-  if constexpr (sizeof(R) == 8) {
-    static_assert(TT, "per-stage tables");
-    FxLines<L, INV, NT, NLINES, MAP, SL, Z0, Z1>::run(reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw),
-                                                      FxFill<L, Z0, Z1, LD, PP>{ld, pp}, st, 0);
-  } else {
-    RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
-  }
+  static_assert(rstages<R>(L) > 0 && sizeof(R) == 4, "unsupported FFT length, or not FP32");
+  RegStage<R, L, INV, NT, NLINES, MAP, 0, 1, SL, TT, Z0, Z1>::run(xb, tw, ld, pp, st);
 }
 // pp for inputs that need no arithmetic after the load
 struct PrepNone {
   template <class T> __device__ __forceinline__ T operator()(int, int, const T& v) const { return v; }
+};
+// pp of a c2r over lines of L points: Z = X + i Y with the Hermitian extension
+template <typename R, int L> struct ZPack {
+  __device__ __forceinline__ C2<R> operator()(int, int p, const C2x2<R>& r) const {
+    const C2<R> X = r.a, Y = r.b;
+    if (p == 0 || 2 * p == L) return cmk<R>(X.x, Y.x);   // c2r drops these imaginary parts
+    return 2 * p < L ? cmk<R>(X.x - Y.y, X.y + Y.x) : cmk<R>(X.x + Y.y, Y.x - X.y);
+  }
 };
 
 // Per-stage twiddle tables in shared memory: the stages read them through the
@@ -757,7 +734,6 @@ k_lines(Op op, const C2<R>* __restrict__ tw, int nlines, int pf) {
     });
     FxLines<L, INV, NT, NLINES, MapInterleaved<R, L, NLINES>, false, Z0, Z1>::run(
         reinterpret_cast<fx2*>(xb), reinterpret_cast<const fxtw*>(tw_s), fill, st, xe);
-    return;
   } else {
   sfor<Op::NKIND>([&](auto kc) {
     constexpr int K = decltype(kc)::value;
@@ -1127,51 +1103,54 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
 }
 
 // ---------------------------------------------------------------------------
-// P3 in the FP64 form: k_p3's lines, with the fields, their cross products and
-// the spectra as integers from the first stage of the inverse to the unpacked
-// modes (doubles in between would cost 12 conversions and FP64 operations per
-// position on the pipe that is scarce).
+// P3 in the FP64 form, with the fields, their cross products and the spectra as
+// integers from the first stage of the inverse to the unpacked modes (doubles in
+// between would cost 12 conversions and FP64 operations per position on the pipe
+// that is scarce).
 //
-// The last inverse stage leaves the fields in place with each line's exponent
-// and, per real field, the OR of the high words' magnitudes.  Those give each
-// column the shifts that bring u to 62 and omega to 61 bits; a product keeps the
-// upper 59 of its 123 bits.  The forward first stage shifts
-// its line right by what its largest butterfly needs (rounded), at most 6 bits.
+// Inverse lines l = f CP + pr: field f (u, omega) of the two columns of pair pr,
+// neighbours that are of one size as a rule.  The last inverse stage leaves the
+// fields in place with each line's exponent and the OR of the high words'
+// magnitudes, which gives the shift that brings the line to 62 bits; a product keeps
+// the upper 60 of its 124 bits.  Every field and every component has its exponent, so
+// that a small component keeps its bits beside a large one.  Forward lines i CP + pr:
+// component i of the two columns; they exchange through the lines 3 CP further on.  The forward first stage shifts its line right by
+// what its largest butterfly needs (rounded), at most 6 bits.
 //
 // The inverse runs as a forward transform of lines with real and imaginary
 // parts exchanged, so that both directions are one text (p3x_second) and one
-// twiddle table.  Lines l = t 2CP + c (t: packed pair, c: column); the
-// forward lines (t, pair) use line t 2CP + 2 pair and exchange through the next
-// one, both of which belong to that pair.
+// twiddle table.
 // ---------------------------------------------------------------------------
-struct FxColumn {       // per column: left shifts (negative: right) of the lines' fields, exponent of the products
-  int s1, s2u, s2w, s3, smin;
-  int e, code;
+struct FxPair {
+  int s[6];      // left shifts of the fields
+  int d[3][2];   // per component: right shifts of the two products
+  int e[3];      // exponents of the components (FX_Q_NAN: a NaN among the fields)
 };
-template <bool LEFT>   // s >= 0
-__device__ __forceinline__ long long fx_shl(long long v, int s) {   // v 2^s, rounded for s < 0
-  return LEFT || s >= 0 ? v << s : ((v >> (s > -63 ? -s - 1 : 62)) + 1) >> 1;
+__device__ __forceinline__ long long fx_rshift(long long v, int d) {   // v 2^-d, rounded
+  return d > 0 ? ((v >> min(d - 1, 62)) + 1) >> 1 : v;
 }
-// a b - c d, upper 64 of 128 bits (a, c below 2^62, b, d below 2^61, split): of
-// each product's cross terms one is floored and one rounded up, so that the
-// means cancel and a product with a zero factor is zero
+// a b, upper 64 of 128 bits (below 2^62 each, split): one cross term is floored and
+// one rounded up, so that the means cancel and a zero factor gives zero
+__device__ __forceinline__ long long fx_mulhi(fxsplit a, fxsplit b) {
+  return fx_wide(a.h, b.h) + (long long)(fx_madhi(a.h, b.l, 0) - fx_madhi(a.l, -b.h, 0));
+}
+// a b - c d, the same
 __device__ __forceinline__ long long fx_det(fxsplit a, fxsplit b, fxsplit c, fxsplit d) {
   const int t = fx_madhi(a.h, b.l, fx_madhi(c.l, -d.h, 0)), u = fx_madhi(c.h, d.l, fx_madhi(a.l, -b.h, 0));
   return fx_wide(a.h, b.h) - fx_wide(c.h, d.h) + (long long)(t - u);
 }
-// u x omega at one position of a column (parts exchanged), lines at stride ls
-template <bool LEFT>
-__device__ __forceinline__ void fx_cross(const fx2* x, int ls, const FxColumn& f, long long* c) {
-  const fx2 z1 = x[0], z2 = x[ls], z3 = x[2 * ls];
-  const fxsplit ux = fx_split(fx_shl<LEFT>(z1.y, f.s1)), uy = fx_split(fx_shl<LEFT>(z1.x, f.s1));
-  const fxsplit uz = fx_split(fx_shl<LEFT>(z2.y, f.s2u)), wx = fx_split(fx_shl<LEFT>(z2.x, f.s2w));
-  const fxsplit wy = fx_split(fx_shl<LEFT>(z3.y, f.s3)), wz = fx_split(fx_shl<LEFT>(z3.x, f.s3));
-  c[0] = fx_det(uy, wz, uz, wy);
-  c[1] = fx_det(uz, wx, ux, wz);
-  c[2] = fx_det(ux, wy, uy, wx);
+// u x omega of a column; d: right shifts of the products (none: aligned)
+__device__ __forceinline__ void fx_cross(const fxsplit* f, bool aligned, const int (*d)[2], long long* c) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    if (aligned) {
+      c[i] = fx_det(f[j], f[3 + k], f[k], f[3 + j]);
+    } else {
+      c[i] = fx_rshift(fx_mulhi(f[j], f[3 + k]), d[i][0]) - fx_rshift(fx_mulhi(f[k], f[3 + j]), d[i][1]);
+    }
+  }
 }
-// bits of a field whose high words' magnitudes OR to m, line exponent q
-__device__ __forceinline__ int fx_field_bits(int q, int m) { return q + 64 - __clz(m); }
 
 template <int M, int CP> __host__ __device__ constexpr int p3x_threads() {
   return rthreads<double, M, 6 * CP, true>();
@@ -1180,50 +1159,85 @@ template <int M, int CP> __host__ __device__ constexpr int p3x_threads() {
 // Dynamic shared memory of k_p3x.
 template <int M, int CP> struct P3X {
   static constexpr int LP = zpad_len<double>(M);
-  static constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
+  static constexpr int NI = 6 * CP, NF = 3 * CP;
   static constexpr int TW = NI * LP;                                 // in units of fx2
   static constexpr int INTS = TW + twtab_elems<double, true>(M);
-  static constexpr int BYTES = INTS * 16 + 3 * NI * 4 + NC * (int)sizeof(FxColumn) + fx_contig_parts<M, NI>() * 4;
+  static constexpr int BYTES = INTS * 16 + 2 * NI * 4 + CP * ((int)sizeof(FxPair) + 4) + fx_contig_parts<M, NI>() * 4;
   __device__ __forceinline__ static fx2* lines() {
     extern __shared__ __align__(16) unsigned char vk_smem[];
     return reinterpret_cast<fx2*>(vk_smem);
   }
   __device__ __forceinline__ static fxtw* twiddles() { return reinterpret_cast<fxtw*>(lines() + TW); }
-  __device__ __forceinline__ static int* line_s() { return reinterpret_cast<int*>(lines() + INTS); }
-  __device__ __forceinline__ static int* field_m() { return line_s() + NI; }
-  __device__ __forceinline__ static FxColumn* cols() { return reinterpret_cast<FxColumn*>(field_m() + 2 * NI); }
-  __device__ __forceinline__ static int* part() { return reinterpret_cast<int*>(cols() + NC); }   // FxLines::PARTS
+  __device__ __forceinline__ static int* line_q() { return reinterpret_cast<int*>(lines() + INTS); }
+  __device__ __forceinline__ static int* field_m() { return line_q() + NI; }
+  __device__ __forceinline__ static int* apart() { return field_m() + NI; }   // a pair's products need shifts
+  __device__ __forceinline__ static FxPair* pairs() { return reinterpret_cast<FxPair*>(apart() + CP); }
+  __device__ __forceinline__ static int* part() { return reinterpret_cast<int*>(pairs() + CP); }   // FxLines::PARTS
 };
-// Stages after the first of nl lines at stride ls, from xs to ds (element
-// offsets), with the fields' magnitudes where they are wanted.
+// Stages after the first of nl lines, from xs to ds (element offsets), with the
+// fields' magnitudes where they are wanted.
 // Inlined twice: as one function it spills (N = 256 3.2 ms against 2.9), as a
 // loop over the directions more so (3.7).
 template <int M, int CP, int NT>
-__device__ __forceinline__ void p3x_second(int xs, int ds, int ls, int nl, bool maxima) {
+__device__ __forceinline__ void p3x_second(int xs, int ds, int nl, bool maxima) {
   using P = P3X<M, CP>;
   using Inv = FxLines<M, false, NT, P::NI, MapContig<double, M, P::NI>, true, 0, 0>;
-  if constexpr (Inv::ST == 3) Inv::middle_rt(P::lines() + xs, ls, nl, P::twiddles());
-  Inv::back_rt(P::lines() + xs, ls, nl, P::twiddles(), [&](const fx2* u, int l, int j) {
-    fx2* dst = P::lines() + ds + l * ls + zi<double>(j);
-    int mx = 0, my = 0;
+  if constexpr (Inv::ST == 3) Inv::middle(P::lines() + xs, P::twiddles(), nl);
+  Inv::back(P::lines() + xs, P::twiddles(), nl, [&](const fx2* u, int l, int j) {
+    fx2* dst = P::lines() + ds + l * P::LP + zi<double>(j);
+    int m = 0;
 #pragma unroll
     for (int r = 0; r < Inv::R1; ++r) {
       const int hx = (int)(u[r].x >> 32), hy = (int)(u[r].y >> 32);
-      mx |= hx ^ (hx >> 31);
-      my |= hy ^ (hy >> 31);
+      m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
       dst[MapContig<double, M, P::NI>::template step<Inv::NB1, 1>(j, r)] = u[r];
     }
-    if (maxima) {   // (parts exchanged)
-      if constexpr (Inv::NB1 % 32 == 0) {   // a warp holds butterflies of one line
-        mx = __reduce_or_sync(0xffffffffu, mx);
-        my = __reduce_or_sync(0xffffffffu, my);
-      }
-      if (Inv::NB1 % 32 != 0 || threadIdx.x % 32 == 0) {
-        atomicOr(P::field_m() + 2 * l, my);
-        atomicOr(P::field_m() + 2 * l + 1, mx);
-      }
+    if (maxima) {
+      if constexpr (Inv::NB1 % 32 == 0) m = __reduce_or_sync(0xffffffffu, m);   // a warp holds butterflies of one line
+      if (Inv::NB1 % 32 != 0 || threadIdx.x % 32 == 0) atomicOr(P::field_m() + l, m);
     }
   });
+}
+
+// The shifts and exponents of a pair: component i (one thread each).
+template <int M, int CP>
+__device__ __forceinline__ void p3x_pair(int pr, int i) {
+  using P = P3X<M, CP>;
+  int s[6], e[6];
+  bool nan = false;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int l = f * CP + pr;
+    const int q = P::line_q()[l];
+    nan = nan || q >= FX_Q_NAN / 2;
+    s[f] = __clz(P::field_m()[l]) - 2;
+    e[f] = q - s[f];
+  }
+  // up to three of the 62 bits bring the components of u, and of omega, to one exponent
+#pragma unroll
+  for (int g = 0; g < 6; g += 3) {
+    const int top = max(max(e[g], e[g + 1]), e[g + 2]);
+#pragma unroll
+    for (int f = g; f < g + 3; ++f) {
+      const int low = top - e[f];
+      if (low <= 3 && low <= s[f]) {
+        s[f] -= low;
+        e[f] = top;
+      }
+    }
+  }
+  const auto pick = [](const int* v, int f) { return f == 0 ? v[0] : f == 1 ? v[1] : v[2]; };
+  const int j = i == 2 ? 0 : i + 1, k = i == 0 ? 2 : i - 1;
+  const int a = pick(e, j) + pick(e + 3, k), b = pick(e, k) + pick(e + 3, j);
+  FxPair& out = P::pairs()[pr];
+  out.d[i][0] = max(b - a, 0);
+  out.d[i][1] = max(a - b, 0);
+  out.e[i] = nan ? FX_Q_NAN : max(a, b) + 64;
+  if (a != b) P::apart()[pr] = 1;
+  if (i == 0) {
+#pragma unroll
+    for (int f = 0; f < 6; ++f) out.s[f] = s[f];
+  }
 }
 
 template <int M, int CP, int NT>
@@ -1232,31 +1246,28 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
   constexpr int N = 2 * M / 3;
   constexpr int H = N / 2 + 1;
   constexpr int LP = zpad_len<double>(M);
-  constexpr int NI = 6 * CP, NF = 3 * CP, NC = 2 * CP;
+  constexpr int NI = 6 * CP, NF = 3 * CP;
   using Inv = FxLines<M, false, NT, NI, MapContig<double, M, NI>, true, H, M - H + 1>;
   using Fwd = FxLines<M, false, NT, NF, MapContig<double, M, NF>, true, 0, 0>;
-  using State = FxState;
   using P = P3X<M, CP>;
+  static_assert(NT >= 3 * CP, "a thread per pair and component");
   fx2* A = P::lines();
-  int* line_s = P::line_s();
-  const int* field_m = P::field_m();
-  FxColumn* cols = P::cols();
+  int* line_q = P::line_q();
   load_twtab<double, M, true, NT>(reinterpret_cast<double2*>(P::twiddles()), reinterpret_cast<const double2*>(tw));
   grid_depend();
-  const int col0 = blockIdx.x * NC;
+  const int col0 = blockIdx.x * 2 * CP;
   const int tid = threadIdx.x;
-  for (int i = tid; i < 2 * NI; i += NT) P::field_m()[i] = 0;
+  for (int i = tid; i < NI + CP; i += NT) P::field_m()[i] = 0;   // apart() too
   {
-    // inverse: packed pairs, positions H .. M - H are the z zero-padding
+    // inverse: positions H .. M - H are the z zero-padding
     const auto ld = [&](int l, int p) -> C2x2<double> {
-      const int t = l / NC;
-      const int col = col0 + l % NC;
+      const int f = l / CP, col = col0 + 2 * (l - f * CP);
       const bool lo = p < H;
       C2x2<double> r{};
-      if (col < a.ncols && (lo || p > M - H)) {
-        const double2* src = a.in + (size_t)col * H + (lo ? p : M - p);
-        r.a = src[(size_t)(2 * t) * a.fsin];
-        r.b = src[(size_t)(2 * t + 1) * a.fsin];
+      if (lo || p > M - H) {
+        const double2* src = a.in + (size_t)f * a.fsin + (size_t)col * H + (lo ? p : M - p);
+        if (col < a.ncols) r.a = src[0];
+        if (col + 1 < a.ncols) r.b = src[H];
       }
       return r;
     };
@@ -1265,63 +1276,33 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
       if (p == 0) return make_double2(r.b.x, r.a.x);
       return p < H ? make_double2(r.a.y + r.b.x, r.a.x - r.b.y) : make_double2(r.b.x - r.a.y, r.a.x + r.b.y);
     };
-    Inv::front(A, FxFill<M, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, P::part(), line_s, 0);
+    Inv::front(A, FxFill<M, H, M - H + 1, decltype(ld), decltype(pp)>{ld, pp}, P::part(), line_q);
   }
   __syncthreads();
-  p3x_second<M, CP, NT>(0, 0, LP, NI, true);
+  p3x_second<M, CP, NT>(0, 0, NI, true);
   __syncthreads();
-  if (tid < NC) {   // the column's shifts
-    int q[3], code[3];
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      const State s = Inv::unpack_state(line_s[t * NC + tid]);
-      code[t] = s.code;
-      q[t] = s.q + (s.code == FX_TINY ? -FX_RANGE : s.code == FX_HUGE ? FX_RANGE : 0);
-    }
-    const int* m1 = field_m + 2 * tid;
-    const int* m2 = m1 + 2 * NC;
-    const int* m3 = m2 + 2 * NC;
-    constexpr int NONE = -(1 << 20);
-    int bu = code[0] == FX_ZERO ? NONE : fx_field_bits(q[0], m1[0] | m1[1]);
-    int bw = code[2] == FX_ZERO ? NONE : fx_field_bits(q[2], m3[0] | m3[1]);
-    if (code[1] != FX_ZERO) {
-      bu = max(bu, fx_field_bits(q[1], m2[0]));
-      bw = max(bw, fx_field_bits(q[1], m2[1]));
-    }
-    FxColumn c;
-    c.s1 = code[0] == FX_ZERO ? -63 : q[0] - (bu - 62);
-    c.s2u = code[1] == FX_ZERO ? -63 : q[1] - (bu - 62);
-    c.s2w = code[1] == FX_ZERO ? -63 : q[1] - (bw - 61);
-    c.s3 = code[2] == FX_ZERO ? -63 : q[2] - (bw - 61);
-    c.code = code[0] == FX_NAN || code[1] == FX_NAN || code[2] == FX_NAN ? FX_NAN
-           : bu == NONE || bw == NONE ? FX_ZERO : FX_PLAIN;
-    c.e = c.code == FX_PLAIN ? (bu - 62) + (bw - 61) + 64 : NONE;
-    c.smin = min(min(c.s1, c.s2u), min(c.s2w, c.s3));
-    cols[tid] = c;
-  }
+  if (tid < 3 * CP) p3x_pair<M, CP>(tid / 3, tid % 3);
   __syncthreads();
   for (int e = tid; e < CP * M; e += NT) {
     const int pr = e / M, p = e % M;
-    const int zp = zi<double>(p);
-    const FxColumn& fa = cols[2 * pr];
-    const FxColumn& fb = cols[2 * pr + 1];
-    fx2* x = A + 2 * pr * LP + zp;   // lines of the pair: t NC LP + column LP
-    const int ez = max(fa.e, fb.e);
-    long long ca[3], cb[3];
-    if (min(fa.smin, fb.smin) >= 0) {   // (the same for a pair's positions: no divergence within a column)
-      fx_cross<true>(x, NC * LP, fa, ca);
-      fx_cross<true>(x + LP, NC * LP, fb, cb);
-    } else {
-      fx_cross<false>(x, NC * LP, fa, ca);
-      fx_cross<false>(x + LP, NC * LP, fb, cb);
+    const FxPair& f = P::pairs()[pr];
+    const bool aligned = P::apart()[pr] == 0;
+    fx2* x = A + pr * LP + zi<double>(p);
+    fxsplit va[6], vb[6];   // the columns (parts exchanged)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const fx2 z = x[i * CP * LP];
+      va[i] = fx_split(z.y << f.s[i]);
+      vb[i] = fx_split(z.x << f.s[i]);
     }
-    x[0] = fx2{ca[0], ca[1]};
-    x[NC * LP] = fx2{fx_shl<false>(ca[2], fa.e - ez), fx_shl<false>(cb[2], fb.e - ez)};
-    x[2 * NC * LP] = fx2{cb[0], cb[1]};
+    long long ca[3], cb[3];
+    fx_cross(va, aligned, f.d, ca);
+    fx_cross(vb, aligned, f.d, cb);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) x[i * CP * LP] = fx2{ca[i], cb[i]};
   }
   __syncthreads();
   {
-    // forward lines l = t CP + pr
     const int l = MapContig<double, M, NF>::template line<Fwd::NB0>(tid);
     const int j = MapContig<double, M, NF>::template bfly<Fwd::NB0>(tid);
     const bool act = tid < Fwd::G0;
@@ -1332,7 +1313,7 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
       __builtin_assume(l >= 0 && l < NF);
 #pragma unroll
       for (int r = 0; r < Fwd::R0; ++r) {
-        v[r] = A[2 * l * LP + zi<double>(j) + MapContig<double, M, NF>::template step<Fwd::NB0, 1>(j, r)];
+        v[r] = A[l * LP + zi<double>(j) + MapContig<double, M, NF>::template step<Fwd::NB0, 1>(j, r)];
         const int hx = (int)(v[r].x >> 32), hy = (int)(v[r].y >> 32);
         sum += max(hx ^ (hx >> 31), hy ^ (hy >> 31)) >> 5;
       }
@@ -1345,69 +1326,33 @@ k_p3x(P3Args<double> a, const fxtw* __restrict__ tw) {
       const long long half = (1ll << sh) >> 1;
 #pragma unroll
       for (int r = 0; r < Fwd::R0; ++r) v[r] = fx2{(v[r].x + half) >> sh, (v[r].y + half) >> sh};
-      fx2* dst = A + (2 * l + 1) * LP + zi<double>(j * Fwd::R0);
-      Fwd::first_dft(v, [&](int r, fx2 z) {
-        dst[MapContig<double, M, NF>::template step<1, Fwd::R0>(j * Fwd::R0, r)] = z;
-      });
-      if (j == 0) {
-        const int t = l / CP, pr = l - t * CP;
-        const FxColumn& ca = cols[2 * pr];
-        const FxColumn& cb = cols[2 * pr + 1];
-        const int e = t == 0 ? ca.e : t == 1 ? max(ca.e, cb.e) : cb.e;
-        int code = t == 0 ? ca.code : t == 2 ? cb.code : ca.code == FX_NAN || cb.code == FX_NAN ? FX_NAN
-                 : ca.code == FX_ZERO && cb.code == FX_ZERO ? FX_ZERO : FX_PLAIN;
-        int q = e + sh + Fwd::TG - 1;   // the modes are halved by the unpacking
-        if (code == FX_PLAIN && (q < -950 || q > 900)) {   // near the ends of the double range, or beyond
-          code = q < -950 - FX_RANGE ? FX_ZERO : q < 0 ? FX_TINY : q <= 900 + FX_RANGE ? FX_HUGE : FX_NAN;
-          q += q < 0 ? FX_RANGE : -FX_RANGE;
-        }
-        line_s[l] = Fwd::pack_state(code == FX_ZERO || code == FX_NAN ? 0 : q, code);
-      }
+      Fwd::first_dft(v, A + NF * LP, l, j);
+      if (j == 0) line_q[l] = P::pairs()[l % CP].e[l / CP] + sh + Fwd::TG;
     }
   }
   __syncthreads();
-  p3x_second<M, CP, NT>(LP, 0, 2 * LP, NF, false);
+  p3x_second<M, CP, NT>(NF * LP, 0, NF, false);
   __syncthreads();
-  for (int e = tid; e < CP * 3 * H; e += NT) {
-    const int k = e % H;
-    const int t = (e / H) % 3;
-    const int pr = e / (3 * H);
-    const State s = Fwd::unpack_state(line_s[t * CP + pr]);
-    const fx2* line = A + 2 * (t * CP + pr) * LP;
-    const fx2 z = line[zi<double>(k)], w = line[zi<double>(k == 0 ? 0 : M - k)];
-    const int q20 = s.q << 20;
-    double2 X = make_double2(fx_to_double(z.x + w.x, q20), fx_to_double(z.y - w.y, q20));
-    double2 Y = make_double2(fx_to_double(z.y + w.y, q20), fx_to_double(w.x - z.x, q20));
-    if (s.code != FX_PLAIN) {
-      const double f = fx_code_factor(s.code);
-      X = make_double2(X.x * f, X.y * f);
-      Y = make_double2(Y.x * f, Y.y * f);
-    }
-    const int ca = col0 + 2 * pr, cb = ca + 1;
-    if (t == 0) {
-      if (ca < a.ncols) {
-        a.out[(size_t)ca * H + k] = X;
-        a.out[a.fsout + (size_t)ca * H + k] = Y;
-      }
-    } else if (t == 1) {
-      if (ca < a.ncols) a.out[2 * a.fsout + (size_t)ca * H + k] = X;
-      if (cb < a.ncols) a.out[2 * a.fsout + (size_t)cb * H + k] = Y;
-    } else {
-      if (cb < a.ncols) {
-        a.out[(size_t)cb * H + k] = X;
-        a.out[a.fsout + (size_t)cb * H + k] = Y;
-      }
-    }
+  for (int e = tid; e < NF * H; e += NT) {
+    const int l = e / H, k = e - l * H;
+    const int i = l / CP, col = col0 + 2 * (l - i * CP);
+    const fx2* line = A + l * LP;
+    double2 X, Y;
+    fx_unpack(line[zi<double>(k)], line[zi<double>(k == 0 ? 0 : M - k)], line_q[l], X, Y);
+    double2* dst = a.out + (size_t)i * a.fsout + (size_t)col * H + k;
+    if (col < a.ncols) dst[0] = X;
+    if (col + 1 < a.ncols) dst[H] = Y;
   }
 }
 
 // ---------------------------------------------------------------------------
 // N-grid z pass on the register engine: c2r of u and/or omega (already x/y
 // inverted and scaled by 1/N^3) packed in pairs, and max |u|^2, max |omega|^2
-// over the N^3 grid (solver.rs:180-218 and :537-567).  Lines per column pair:
+// over the N^3 grid (solver.rs:180-218 and :537-567).  Lines per column pair, FP32:
 // BOTH: l = 6 pr + 3 cc + t, the pair t of column cc; otherwise l = 3 pr + cc
-// (f0 + i f1 of column cc) and 3 pr + 2 (f2 of both columns).  The inverse
-// writes its physical values in place; the maxima follow.
+// (f0 + i f1 of column cc) and 3 pr + 2 (f2 of both columns).  FP64: field f of both
+// columns, l = f CP + pr (k_p3x's lines).  The inverse writes its physical values in
+// place; the maxima follow.
 // ---------------------------------------------------------------------------
 template <typename R, int N, int CP, bool BOTH>
 __host__ __device__ constexpr int nz_threads() {
@@ -1438,35 +1383,46 @@ k_nz_max(NZArgs<R> a, const C2<R>* __restrict__ tw, int pf) {
   grid_depend();
   if (threadIdx.x == 0) redn = 0;
   const int col0 = blockIdx.x * 2 * CP;
-  fft_lines<R, N, true, NT, NL, MapContig<R, N, NL>, true, true>(
-      lines, tw_s,
-      [&](int l, int p) -> C2x2<R> {
-        const int pr = l / LPP, j = l % LPP;
-        int fx, fy, cx, cy;
-        if (BOTH) {
-          const int cc = j / 3, t = j % 3;
-          fx = 2 * t; fy = 2 * t + 1;
-          cx = cy = col0 + 2 * pr + cc;
-        } else if (j < 2) {
-          fx = 0; fy = 1;
-          cx = cy = col0 + 2 * pr + j;
-        } else {
-          fx = fy = 2;
-          cx = col0 + 2 * pr;
-          cy = cx + 1;
-        }
-        const int k = p < H ? p : N - p;
-        C2x2<R> r{};
-        if (cx < a.ncols) r.a = a.in[(size_t)fx * a.fs + (size_t)cx * H + k];
-        if (cy < a.ncols) r.b = a.in[(size_t)fy * a.fs + (size_t)cy * H + k];
-        return r;
-      },
-      [&](int, int p, const C2x2<R>& r) -> C2<R> {   // Z = X + i Y with the Hermitian extension
-        const C2<R> X = r.a, Y = r.b;
-        if (p == 0 || 2 * p == N) return cmk<R>(X.x, Y.x);   // c2r drops these imaginary parts
-        return p < H ? cmk<R>(X.x - Y.y, X.y + Y.x) : cmk<R>(X.x + Y.y, Y.x - X.y);
-      },
-      [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
+  if constexpr (sizeof(R) == 8) {
+    const auto ld = [&](int l, int p) -> C2x2<R> {
+      const int f = l / CP, c = col0 + 2 * (l - f * CP);
+      const C2<R>* src = a.in + (size_t)f * a.fs + (size_t)c * H + (p < H ? p : N - p);
+      C2x2<R> r{};
+      if (c < a.ncols) r.a = src[0];
+      if (c + 1 < a.ncols) r.b = src[H];
+      return r;
+    };
+    FxLines<N, true, NT, NL, MapContig<R, N, NL>, true, 0, 0>::run(
+        reinterpret_cast<fx2*>(lines), reinterpret_cast<const fxtw*>(tw_s),
+        FxFill<N, 0, 0, decltype(ld), ZPack<R, N>>{ld, ZPack<R, N>{}},
+        [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; }, 0);
+  } else {
+    fft_lines<R, N, true, NT, NL, MapContig<R, N, NL>, true, true>(
+        lines, tw_s,
+        [&](int l, int p) -> C2x2<R> {
+          const int pr = l / LPP, j = l % LPP;
+          int fx, fy, cx, cy;
+          if (BOTH) {
+            const int cc = j / 3, t = j % 3;
+            fx = 2 * t; fy = 2 * t + 1;
+            cx = cy = col0 + 2 * pr + cc;
+          } else if (j < 2) {
+            fx = 0; fy = 1;
+            cx = cy = col0 + 2 * pr + j;
+          } else {
+            fx = fy = 2;
+            cx = col0 + 2 * pr;
+            cy = cx + 1;
+          }
+          const int k = p < H ? p : N - p;
+          C2x2<R> r{};
+          if (cx < a.ncols) r.a = a.in[(size_t)fx * a.fs + (size_t)cx * H + k];
+          if (cy < a.ncols) r.b = a.in[(size_t)fy * a.fs + (size_t)cy * H + k];
+          return r;
+        },
+        ZPack<R, N>{},
+        [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
+  }
   __syncthreads();
   // maxima in the working precision (the FP32-bulk form keeps FP64 only for
   // the dt arithmetic that consumes them)
@@ -1477,19 +1433,35 @@ k_nz_max(NZArgs<R> a, const C2<R>* __restrict__ tw, int pf) {
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       if (col0 + 2 * pr + cc >= a.ncols) continue;
-      if (BOTH) {
-        const C2<R>* L0 = lines + (6 * pr + 3 * cc) * LP;
-        const C2<R> A = L0[zi<R>(p)], B = L0[LP + zi<R>(p)], C = L0[2 * LP + zi<R>(p)];
-        const R ux = A.x, uy = A.y, uz = B.x, wx = B.y, wy = C.x, wz = C.y;
+      if constexpr (BOTH) {
+        R ux, uy, uz, wx, wy, wz;
+        if constexpr (sizeof(R) == 8) {
+          const auto at = [&](int f) {
+            const C2<R> v = lines[(f * CP + pr) * LP + zi<R>(p)];
+            return cc == 0 ? v.x : v.y;
+          };
+          ux = at(0); uy = at(1); uz = at(2); wx = at(3); wy = at(4); wz = at(5);
+        } else {
+          const C2<R>* L0 = lines + (6 * pr + 3 * cc) * LP;
+          const C2<R> A = L0[zi<R>(p)], B = L0[LP + zi<R>(p)], C = L0[2 * LP + zi<R>(p)];
+          ux = A.x; uy = A.y; uz = B.x; wx = B.y; wy = C.x; wz = C.y;
+        }
         const R s1 = ux * ux + uy * uy + uz * uz;
         const R s2 = wx * wx + wy * wy + wz * wz;
         bad |= (s1 != s1) | (s2 != s2);
         m1 = fmax(m1, s1);
         m2 = fmax(m2, s2);
       } else {
-        const C2<R> A = lines[(3 * pr + cc) * LP + zi<R>(p)];
-        const C2<R> Z = lines[(3 * pr + 2) * LP + zi<R>(p)];
-        const R fx = A.x, fy = A.y, fz = cc == 0 ? Z.x : Z.y;
+        R fx, fy, fz;
+        if constexpr (sizeof(R) == 8) {
+          const C2<R> A = lines[pr * LP + zi<R>(p)], B = lines[(CP + pr) * LP + zi<R>(p)],
+                      C = lines[(2 * CP + pr) * LP + zi<R>(p)];
+          fx = cc == 0 ? A.x : A.y; fy = cc == 0 ? B.x : B.y; fz = cc == 0 ? C.x : C.y;
+        } else {
+          const C2<R> A = lines[(3 * pr + cc) * LP + zi<R>(p)];
+          const C2<R> Z = lines[(3 * pr + 2) * LP + zi<R>(p)];
+          fx = A.x; fy = A.y; fz = cc == 0 ? Z.x : Z.y;
+        }
         const R s = fx * fx + fy * fy + fz * fz;
         bad |= (s != s);
         m1 = fmax(m1, s);
@@ -1551,14 +1523,31 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_r2c(FZArgs
   grid_depend();
   C2<R>* lines = reinterpret_cast<C2<R>*>(vk_smem);
   const int col0 = blockIdx.x * 2 * CP;
+  const auto ld = [&](int l, int p) -> C2<R> {
+    const int c = col0 + 2 * l;
+    const R* x = a.real + (size_t)c * L + p;
+    return cmk<R>(c < a.ncols ? x[0] : R(0), c + 1 < a.ncols ? x[L] : R(0));
+  };
+  if constexpr (sizeof(R) == 8) {
+    using Fwd = FxLines<L, false, NT, CP, MapContig<R, L, CP>, true, 0, 0>;
+    __shared__ int part[Fwd::PARTS], line_q[CP];
+    fx2* z = reinterpret_cast<fx2*>(lines);
+    Fwd::run_integers(z, reinterpret_cast<const fxtw*>(tw_s),
+                      FxFill<L, 0, 0, decltype(ld), PrepNone>{ld, PrepNone{}}, part, line_q);
+    for (int e = threadIdx.x; e < CP * H; e += NT) {
+      const int l = e / H, k = e - l * H;
+      const int c = col0 + 2 * l;
+      if (c >= a.ncols) break;
+      C2<R> X, Y;
+      fx_unpack(z[l * LP + zi<R>(k)], z[l * LP + zi<R>(k == 0 ? 0 : L - k)], line_q[l], X, Y);
+      C2<R>* dst = a.cplx + (size_t)c * H + k;
+      dst[0] = X;
+      if (c + 1 < a.ncols) dst[H] = Y;
+    }
+    return;
+  } else {
   fft_lines<R, L, false, NT, CP, MapContig<R, L, CP>, true, true>(
-      lines, tw_s,
-      [&](int l, int p) -> C2<R> {
-        const int c = col0 + 2 * l;
-        const R* x = a.real + (size_t)c * L + p;
-        return cmk<R>(c < a.ncols ? x[0] : R(0), c + 1 < a.ncols ? x[L] : R(0));
-      },
-      PrepNone{}, [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
+      lines, tw_s, ld, PrepNone{}, [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
   __syncthreads();
   for (int e = threadIdx.x; e < 2 * CP * H; e += NT) {
     const int col = e / H, k = e % H;
@@ -1566,6 +1555,7 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_r2c(FZArgs
     C2<R> X, Y;
     zunpack<R>(lines + (col / 2) * LP, L, k, X, Y);
     a.cplx[(size_t)(col0 + col) * H + k] = col % 2 == 0 ? X : Y;
+  }
   }
 }
 
@@ -1577,27 +1567,28 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_c2r(FZArgs
   load_twtab<R, L, true, NT>(tw_s, tw);
   grid_depend();
   const int col0 = blockIdx.x * 2 * CP;
-  fft_lines<R, L, true, NT, CP, MapContig<R, L, CP>, false, true>(
-      reinterpret_cast<C2<R>*>(vk_smem), tw_s,
-      [&](int l, int p) -> C2x2<R> {
-        const int c = col0 + 2 * l;
-        const C2<R>* x = a.cplx + (size_t)c * H + (p < H ? p : L - p);
-        C2x2<R> r{};
-        if (c < a.ncols) r.a = x[0];
-        if (c + 1 < a.ncols) r.b = x[H];
-        return r;
-      },
-      [&](int, int p, const C2x2<R>& r) -> C2<R> {   // Z = X + i Y with the Hermitian extension
-        const C2<R> X = r.a, Y = r.b;
-        if (p == 0 || 2 * p == L) return cmk<R>(X.x, Y.x);   // c2r drops these imaginary parts
-        return p < H ? cmk<R>(X.x - Y.y, X.y + Y.x) : cmk<R>(X.x + Y.y, Y.x - X.y);
-      },
-      [&](int l, int p, C2<R> z) {
-        const int c = col0 + 2 * l;
-        R* x = a.real + (size_t)c * L + p;
-        if (c < a.ncols) x[0] = z.x * a.scale;
-        if (c + 1 < a.ncols) x[L] = z.y * a.scale;
-      });
+  const auto ld = [&](int l, int p) -> C2x2<R> {
+    const int c = col0 + 2 * l;
+    const C2<R>* x = a.cplx + (size_t)c * H + (p < H ? p : L - p);
+    C2x2<R> r{};
+    if (c < a.ncols) r.a = x[0];
+    if (c + 1 < a.ncols) r.b = x[H];
+    return r;
+  };
+  const auto st = [&](int l, int p, C2<R> z) {
+    const int c = col0 + 2 * l;
+    R* x = a.real + (size_t)c * L + p;
+    if (c < a.ncols) x[0] = z.x * a.scale;
+    if (c + 1 < a.ncols) x[L] = z.y * a.scale;
+  };
+  if constexpr (sizeof(R) == 8) {
+    FxLines<L, true, NT, CP, MapContig<R, L, CP>, false, 0, 0>::run(
+        reinterpret_cast<fx2*>(vk_smem), reinterpret_cast<const fxtw*>(tw_s),
+        FxFill<L, 0, 0, decltype(ld), ZPack<R, L>>{ld, ZPack<R, L>{}}, st, 0);
+  } else {
+    fft_lines<R, L, true, NT, CP, MapContig<R, L, CP>, false, true>(
+        reinterpret_cast<C2<R>*>(vk_smem), tw_s, ld, ZPack<R, L>{}, st);
+  }
 }
 
 }  // namespace vk
