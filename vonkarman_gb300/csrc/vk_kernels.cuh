@@ -268,6 +268,12 @@ template <typename R>
 __device__ __forceinline__ C2<R> axpby(R a, C2<R> x, R b, C2<R> y) {
   return cmk<R>(a * x.x + b * y.x, a * x.y + b * y.y);
 }
+// e u + b y for a state u, to which the increment b y is small: one rounding at
+// the state's size (the compiler may fuse the other product, which leaves two)
+template <typename R>
+__device__ __forceinline__ C2<R> state_sum(R e, C2<R> u, R b, C2<R> y) {
+  return cmk<R>(fma(e, u.x, b * y.x), fma(e, u.y, b * y.y));
+}
 
 // The final stage of a step raises the context's sticky non-finite flag when
 // it writes a NaN or an infinity (the NaN check of the reference's audit,
@@ -359,7 +365,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           s.n1[c * cs + idx[q]] = nl[q][c];
-          s.temp[c * cs + idx[q]] = axpby<R>(eh[q], u[q][c], qq[q], nl[q][c]);
+          s.temp[c * cs + idx[q]] = state_sum<R>(eh[q], u[q][c], qq[q], nl[q][c]);
         }
       }
       break;
@@ -381,7 +387,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           s.acc[c * cs + idx[q]] = axpby<R>(b1[q], n1[q][c], b23[q], nl[q][c]);
-          s.temp[c * cs + idx[q]] = axpby<R>(eh[q], u[q][c], qq[q], nl[q][c]);
+          s.temp[c * cs + idx[q]] = state_sum<R>(eh[q], u[q][c], qq[q], nl[q][c]);
         }
       }
       break;
@@ -405,7 +411,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
         for (int c = 0; c < 3; ++c) {
           s.acc[c * cs + idx[q]] = cmk<R>(a[q][c].x + b23[q] * nl[q][c].x, a[q][c].y + b23[q] * nl[q][c].y);
           const C2<R> dn = cmk<R>(R(2) * nl[q][c].x - n1[q][c].x, R(2) * nl[q][c].y - n1[q][c].y);
-          s.temp[c * cs + idx[q]] = axpby<R>(ef[q], u[q][c], qq[q], dn);
+          s.temp[c * cs + idx[q]] = state_sum<R>(ef[q], u[q][c], qq[q], dn);
         }
       }
       break;
@@ -425,7 +431,7 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const C2<R> rhs = cmk<R>(a[q][c].x + b4[q] * nl[q][c].x, a[q][c].y + b4[q] * nl[q][c].y);
-          const C2<R> v = axpby<R>(ef[q], u[q][c], (R)dt, rhs);
+          const C2<R> v = state_sum<R>(ef[q], u[q][c], (R)dt, rhs);
           s.u_out[c * cs + idx[q]] = v;
           flag_nonfinite<R>(s, v);
           if constexpr (KEEP) un[q][c] = v;
@@ -451,9 +457,9 @@ __device__ __forceinline__ void stage_apply_n(const StageArgs<R>& s, const size_
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           s.acc[c * cs + idx[q]] = cmk<R>(ac[q][c].x + b23[q] * nl[q][c].x, ac[q][c].y + b23[q] * nl[q][c].y);
-          const C2<R> av = axpby<R>(eh[q], u[q][c], qq[q], n1[q][c]);
+          const C2<R> av = state_sum<R>(eh[q], u[q][c], qq[q], n1[q][c]);
           const C2<R> dn = cmk<R>(R(2) * nl[q][c].x - n1[q][c].x, R(2) * nl[q][c].y - n1[q][c].y);
-          s.temp[c * cs + idx[q]] = axpby<R>(eh[q], av, qq[q], dn);
+          s.temp[c * cs + idx[q]] = state_sum<R>(eh[q], av, qq[q], dn);
         }
       }
       break;
