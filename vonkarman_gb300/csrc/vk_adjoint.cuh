@@ -442,7 +442,7 @@ template <typename R> struct A5Args {
   AdjStageArgs<R> st;
 };
 
-template <typename R> struct A5Lines { static constexpr int value = 8; };
+constexpr int A5_LINES = 8;
 
 // Transposed P5 (FP32) for the six cotangent fields (a_bar, o_bar): x-forward, keep
 // N of M modes, weight, and y = a_bar + i k x o_bar accumulated field by field

@@ -117,8 +117,8 @@ inline int wave_blocks(int nt, size_t smem) {
 }
 
 // L2 prefetch distance of the FP32 column-pair z passes (k_p3, k_nz_max,
-// k_adj_z): one residency wave (0 = off, and for FP64, whose passes the FP64
-// pipe bounds)
+// k_adj_z): one residency wave (0 = off, and for FP64, whose passes wait on
+// instruction issue and barriers)
 template <typename R, auto KERN>
 inline int zpass_prefetch_distance(int nt, size_t smem) {
   return sizeof(R) == 4 && VK_P3F_PREFETCH ? wave_blocks<KERN>(nt, smem) : 0;
@@ -340,7 +340,7 @@ inline cudaError_t nla_n(const NlaParams<R>& p, cudaStream_t s) {
     e = launch_overlapped(k_adj_stage_f64<N>, p5_ctas(N, false), StageGrid<double, N>::NT, 0, s, true, a);
   } else {
     TimerScope ts(p.timer, PASS_A5, s);
-    constexpr int NL = A5Lines<R>::value;
+    constexpr int NL = A5_LINES;
     constexpr int NT = cmin(rthreads<R, M, NL>(), 384);
     const int nlines = N * H;
     const size_t smem = (size_t)(rsmem_elems<R, M, NL>() + 3 * N * NL) * sizeof(C2<R>);

@@ -212,9 +212,9 @@ struct RegStage {
     C2<R> v[Q][RAD];
     if constexpr (S == 0) {
       // raw inputs wider than one complex value are staged in chunks of
-      // 192 (FP32) / 128 (FP64) bytes per thread (registers)
+      // 192 bytes per thread (registers)
       using Raw = decltype(ld(0, 0));
-      constexpr int CH = sizeof(Raw) > sizeof(C2<R>) ? cmin(RAD, (int)((sizeof(R) == 4 ? 192 : 128) / sizeof(Raw))) : RAD;
+      constexpr int CH = sizeof(Raw) > sizeof(C2<R>) ? cmin(RAD, (int)(192 / sizeof(Raw))) : RAD;
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int g = tid + q * NT;
@@ -996,7 +996,7 @@ struct P3RowUnpack {
 // line over whole warps
 template <typename R, int M, int NF, int NT>
 __host__ __device__ constexpr bool z_row_unpack() {
-  if (sizeof(R) != 4 || VK_P3_ROW_UNPACK == 0) return false;
+  if (VK_P3_ROW_UNPACK == 0) return false;
   constexpr int S = rstages<R, true>(M);
   constexpr int RAD = rradix<R, true>(M, S - 1);
   constexpr int NB = M / RAD;
@@ -1013,10 +1013,9 @@ k_p3(P3Args<R> a, const C2<R>* __restrict__ tw, int pf) {
   constexpr bool INPL = p3_inplace<CP>();
   extern __shared__ __align__(16) unsigned char vk_smem[];
   __shared__ C2<R> tw_s[twtab_elems<R, true>(M)];
-  // L2 prefetch of the six input ranges of the CTA pf blocks ahead (FP32:
-  // 2 CP columns of H complex values per field, a multiple of 16 bytes at a
-  // 16-byte boundary)
-  if constexpr (sizeof(R) == 4) {
+  // L2 prefetch of the six input ranges of the CTA pf blocks ahead (2 CP columns
+  // of H complex values per field, a multiple of 16 bytes at a 16-byte boundary)
+  {
     const int b = (int)blockIdx.x + pf;
     if (pf > 0 && threadIdx.x < 6 && b < (int)gridDim.x && (b + 1) * 2 * CP <= a.ncols)
       prefetch_l2_bulk(a.in + (size_t)threadIdx.x * a.fsin + (size_t)b * (2 * CP * H), 2 * CP * H * sizeof(C2<R>));
@@ -1546,16 +1545,16 @@ __global__ void __launch_bounds__(NT, fz_min_blocks<R, L, NT>()) k_fz_r2c(FZArgs
     }
     return;
   } else {
-  fft_lines<R, L, false, NT, CP, MapContig<R, L, CP>, true, true>(
-      lines, tw_s, ld, PrepNone{}, [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
-  __syncthreads();
-  for (int e = threadIdx.x; e < 2 * CP * H; e += NT) {
-    const int col = e / H, k = e % H;
-    if (col0 + col >= a.ncols) break;
-    C2<R> X, Y;
-    zunpack<R>(lines + (col / 2) * LP, L, k, X, Y);
-    a.cplx[(size_t)(col0 + col) * H + k] = col % 2 == 0 ? X : Y;
-  }
+    fft_lines<R, L, false, NT, CP, MapContig<R, L, CP>, true, true>(
+        lines, tw_s, ld, PrepNone{}, [&](int l, int p, C2<R> v) { lines[l * LP + zi<R>(p)] = v; });
+    __syncthreads();
+    for (int e = threadIdx.x; e < 2 * CP * H; e += NT) {
+      const int col = e / H, k = e % H;
+      if (col0 + col >= a.ncols) break;
+      C2<R> X, Y;
+      zunpack<R>(lines + (col / 2) * LP, L, k, X, Y);
+      a.cplx[(size_t)(col0 + col) * H + k] = col % 2 == 0 ? X : Y;
+    }
   }
 }
 
