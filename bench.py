@@ -203,7 +203,7 @@ def step_bytes(n: int, elem: int) -> float:
 # ncu captures (dram__bytes_read.sum + dram__bytes_write.sum): FP64 at N=128,
 # FP32-bulk at N=256, scaled to grid n by the padded columns x modes (M^2 H).
 NCU_TRAFFIC = {
-    ("P3_z_c2r_cross_r2c", "fp64"): (128, 230142720 + 85930752),
+    ("P3_z_c2r_cross_r2c", "fp64"): (128, 230277632 + 85332736),
     ("P3_z_c2r_cross_r2c", "fp32bulk"): (256, 913113600 + 424164352),
 }
 
@@ -650,7 +650,7 @@ def run_ours(args, d: Dist):
                      "peak_source": hbm_src,
                      "algorithmic_bytes_per_launch": dom_bytes, "ms_per_launch": dom_ms,
                      "note": ("HBM fraction of the FP64 form's dominant kernel, whose transforms run in 64-bit fixed point: "
-                              "bound by instruction issue (61 % of the slots in ncu) and latency")
+                              "bound by instruction issue (58 % of the slots in ncu at N=128), barriers and latency")
                      if args.precision == "fp64" else
                      ("FP32-bulk P3 (k_p3f): issue- and latency-bound in ncu at N=256 (53 % of issue slots, "
                       "global-load latency the top stall, 4 CTAs of 96 threads per SM)"

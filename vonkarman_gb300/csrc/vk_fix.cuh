@@ -113,8 +113,9 @@ template <int B> VK_FIX_HD fx2 fx_shift(fx2 a) { return fx2{fx_bump<B>(a.x) >> B
 // the cross product, ms: N = 256 {24, 16} 2.90, {8, 8, 6} 2.65; N = 128 {12, 16}
 // 0.414, {12, 4, 4} 0.375, {6, 8, 4} 0.355.)  Below, two stages: a third one's
 // exchange costs about what it gains (N = 64 {12, 8} 0.055, {3, 8, 4} 0.062;
-// {6, 4, 4} 0.047, but its roundings drift one way).  The first stage has 2^b or
-// 16 c butterflies, so that groups of lanes keep one contiguous line.
+// {6, 4, 4} 0.047, but with the roundings of that time a mean error of its own).
+// The first stage has 2^b or 16 c butterflies, so that groups of lanes keep one
+// contiguous line.
 VK_FIX_HD constexpr int fx_radix0(int L) {
   return L == 8 ? 2 : L == 12 ? 3 : L == 16 ? 4 : L == 24 ? 6 : L == 32 ? 4 : L == 48 ? 6 : L == 64 ? 8 : L == 96 ? 12
        : L == 128 ? 16 : L == 192 ? 6 : L == 256 ? 8 : L == 384 ? 8 : L == 512 ? 8 : L == 768 ? 12 : 0;
